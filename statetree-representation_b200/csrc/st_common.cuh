@@ -128,6 +128,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// one lane of a converged warp, in a form the compiler knows to be a single lane (operands of TMA and tcgen05
+// instructions then go to uniform registers without a loop over the lanes)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(p));
+  return p != 0;
+}
+
 // ------------------------------------------------------------------------------------------------ mbarrier / TMA
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(bar)), "r"(count) : "memory");
@@ -150,13 +158,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (mbar_try(bar, parity)) return true;
   return false;
 }
-// the same with a non-blocking look first, for waiters whose barrier has usually flipped already (the tcgen05 GEMM's
-// warps, which wait twice per k-tile)
-__device__ __forceinline__ bool mbar_wait_look(uint64_t* bar, uint32_t parity) {
+// one non-blocking look: has the phase of this parity completed?
+__device__ __forceinline__ bool mbar_look(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-  return ok ? true : mbar_wait(bar, parity);
+  return ok != 0;
+}
+// the same as mbar_wait with a non-blocking look first, for waiters whose barrier has usually flipped already (the tcgen05 GEMM's
+// warps, which wait twice per k-tile)
+__device__ __forceinline__ bool mbar_wait_look(uint64_t* bar, uint32_t parity) {
+  return mbar_look(bar, parity) ? true : mbar_wait(bar, parity);
 }
 // non-suspending variant: polls with test_wait, so a waiter notices the flip within a few cycles (try_wait may park the
 // thread for a while); for short hand-overs between a few warps

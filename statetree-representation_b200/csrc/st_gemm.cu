@@ -1,24 +1,25 @@
 // Large-batch fused tree-decode + GEMM on the 5th-generation tensor cores (tcgen05 / TMEM) of sm_100a.
 //   Y[B, M] = X[B, N] W[M, N]^T,  W as state-tree records, fp32 accumulation in tensor memory, BF16 output.
 //
-// One CTA computes a 128-row block of W against one tile of NT tokens (NT = 64, 128 or 256) over a contiguous range
-// of 64-column k-tiles.  Warp roles (20 warps):
-//   warps 0-15  decode, in two groups of eight (group g takes every second k-tile): each warp turns one record into
-//               its mma-fragment registers (five integer ops per four weights), patches escapes, and writes the
-//               16 x 64 BF16 sub-tile into the K-major, 128-byte-swizzled A tile with stmatrix; fence.proxy.async
-//               hands the tile to the tensor core
-//   warp 16     record producer: one 3-D tiled TMA load per k-tile brings the eight 1552-byte records of the block's
-//               eight 16-row tiles into a deep ring
-//   warp 17     activation producer: one tiled TMA load of X[tok0 .. tok0 + NT, 64 cols] with the 128-byte swizzle
-//   warps 18-19 MMA issuers: one elected thread each issues four tcgen05.mma (128 x NT x 16, kind::f16) per k-tile of
-//               its decode group, A and B read from shared memory through descriptors, D in its own TMEM
-//               accumulator; tcgen05.commit releases the stage
-// Epilogue: the decode warps read the accumulators with tcgen05.ld, add the two issuers' tiles in a fixed order and
-// park the fp32 tile in shared memory; the CTAs that split a k range form a thread-block cluster and add their tiles
-// through distributed shared memory in rank order (deterministic), then store BF16.
+// One CTA computes a 128-row block of W against one tile of NT tokens over a contiguous range of 64-column k-tiles.
+// Warp roles:
+//   8 DG decode warps, in DG groups of eight (group g takes the k-tile pairs g, g + DG, ...): each warp turns the two
+//              records of its 16 rows into mma-fragment registers (five integer ops per four weights), patches escapes,
+//              and writes each 16 x 64 BF16 sub-tile into TENSOR MEMORY with one tcgen05.st.16x128b.x8: a record is stored in mma.m16n8k16
+//              A-fragment order, which is that instruction's register layout, so the A operand never touches shared
+//              memory (no stmatrix, no proxy fence, no operand read by the tensor core)
+//   record producer: one 3-D tiled TMA load per pair of k-tiles brings the sixteen 1552-byte records of the block's eight
+//              16-row tiles into a ring
+//   activation producer: tiled TMA loads of X[tok0 .. tok0 + NT, 64 cols] with the 128-byte swizzle
+//   MMA issuer: one elected thread issues four tcgen05.mma (128 x NT x 16, kind::f16; two halves beyond 256 tokens) per
+//              k-tile, A from tensor memory, B from shared memory, D in tensor memory; tcgen05.commit frees the stage
+// Epilogue: a CTA that owns its whole k range stores BF16 straight from tcgen05.ld registers; the CTAs that split a k
+// range form a thread-block cluster, park their fp32 tiles in shared memory and add them through distributed shared
+// memory in rank order (deterministic), then store BF16.
 // The grouped (mixture-of-experts) variant runs the same pipeline per (block of NT routed pairs, 128-row block): the
 // block's expert selects the weight tensor map and escape tables, the activation tile comes from rows gathered in
-// block order, and the result rows are scattered back to their pair indices.
+// block order, the MMA width and the activation loads cover only the pairs the block really holds, and the result rows
+// are scattered back to their pair indices.
 // Every mbarrier wait is bounded; a wait that runs out sets the device status word and the CTA leaves after
 // releasing its tensor memory.
 #include <cuda.h>
@@ -35,8 +36,9 @@
 namespace {
 using namespace st;
 
-constexpr int A_TILE = 128 * 128;            // 128 rows x 64 bf16, one swizzle atom wide
-constexpr int NDEC = 8;                      // decode warps = records per k-tile
+constexpr int NDEC = 8;                      // decode warps of a group = records per k-tile
+constexpr int A_COLS = 32;                   // tensor-memory columns of a decoded weight tile: 128 rows x 64 BF16
+constexpr int PAIR = 2;                      // k-tiles per decode step
 
 constexpr int MAXL = 4;                       // matrices in one list launch
 
@@ -47,8 +49,7 @@ struct GemmArgs {
   const CUtensorMap* maps; const long long* eop; const long long* elp;
   const int* sorted; const int* bexp; const int* npost; int E;
   long long M, N;
-  int B, NG, NT, KS, RB, TT, stages, rstages, nmma, bar_off;
-  uint32_t idesc;
+  int B, NG, NT, KS, RB, TT, astages, xstages, rstages, bar_off, tmem_cols, rb0;
   // list of matrices that share the activations (q / k / v, gate / up as separate trees): member of each row block
   int nlist; int rbend[MAXL];                 // first row block after each member in the concatenation
   const int* leo[MAXL]; const uint32_t* lel[MAXL]; uint16_t* lY[MAXL]; float* lYf[MAXL]; long long lM[MAXL];
@@ -77,11 +78,22 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-               :: "r"(d_tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+// D[128 x n] (+)= A B^T with A (128 rows x 16 BF16: eight 32-bit columns) in tensor memory, B in shared memory
+__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+               :: "r"(d_tmem), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[32]) {
+// a decoded record (16 rows x 64 BF16 as four mma A fragments) -> 16 lanes x 32 columns of tensor memory.  16x128b: lane
+// (g, t) holds column t of rows g (even registers) and g + 8 (odd), each register pair four columns further: exactly
+// (A[s][0], A[s][1]) = k 16 s + 2t, (A[s][2], A[s][3]) = k 16 s + 8 + 2t
+__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const uint32_t (&A)[4][4]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               :: "r"(taddr), "r"(A[0][0]), "r"(A[0][1]), "r"(A[0][2]), "r"(A[0][3]), "r"(A[1][0]), "r"(A[1][1]),
+                  "r"(A[1][2]), "r"(A[1][3]), "r"(A[2][0]), "r"(A[2][1]), "r"(A[2][2]), "r"(A[2][3]), "r"(A[3][0]),
+                  "r"(A[3][1]), "r"(A[3][2]), "r"(A[3][3]) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
@@ -94,47 +106,72 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-// Two decode groups of eight warps (group g takes the k-tiles g, g + 2, ...), a record producer, an activation
-// producer and two MMA issuer warps: one CTA per SM.
-constexpr int DG = 2;
-constexpr int NDW = DG * NDEC;                                              // decode warps
-constexpr int W_RAW = NDW, W_X = NDW + 1, W_MMA = NDW + 2;                  // role warps
-constexpr int THREADS = (NDW + 2 + DG) * 32;
 #define GW mbar_wait_look
-__device__ __forceinline__ bool wait_decode(uint64_t* bar, uint32_t parity) { return GW(bar, parity); }
-constexpr int RAW_SLOT = NDEC * REC;         // 12416 B: the eight records of one k-tile
+constexpr int RAW_SLOT = NDEC * PAIR * REC;  // 24832 B: the sixteen records of a pair of k-tiles
+constexpr int XBOX_GROUPED = 32;             // rows per activation load of the grouped variant
+template <int DG> constexpr int gemm_threads() { return (DG * NDEC + 3) * 32; }
 
-// Two rings.  The RAW ring (R slots of eight records) faces HBM: its depth sets the bytes in flight.  The TILE ring
-// (S stages of decoded weight tile + activation tile) covers the decode -> MMA hand-over and the L2 latency of the
-// activation loads; one mbarrier per stage counts both operands so the MMA thread waits once and commits once.
+// instruction descriptor: D fp32, A and B bf16, both K-major, N = n, M = 128
+__host__ __device__ constexpr uint32_t mma_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+
+// Three rings.  The RAW ring (R slots of sixteen records) faces HBM: its depth sets the bytes in flight.  The A ring (SA
+// slots of two decoded weight tiles in tensor memory) covers the decode -> MMA hand-over, the X ring (SX activation tiles
+// of one k-tile in shared memory) the L2 latency of the activation loads.
+//
+// Why pairs: a decode warp's time per step is ~250 cycles of decoding per record and ~700 cycles of barrier looks, slot
+// hand-overs and escape bookkeeping per step, whatever the step holds (cycle counters around each part, 6144 x 4096): one
+// record per step cost 1000 cycles, i.e. 63 per record and SM with sixteen warps.
+//
+// DG = 1 (token tiles up to 128): eight decode warps, at most half of an SM's shared memory, registers and tensor memory,
+// so two CTAs share an SM: one CTA's start-up, drain and epilogue run under the other's main loop, and the next launch's
+// CTAs become resident (and start streaming weights) as soon as any CTA of this launch leaves.
+// DG = 2 (up to 320 tokens): one CTA per SM, sixteen decode warps; a whole batch of up to 320 rows decodes every record once.
+//
+// Measured, the four projections of a layer (6144, 4096, 24576 x 4096 and 4096 x 12288) in a graph, us per layer: 64 rows
+// 108 -> 85, 300 rows 251 -> 153 (was: A through shared memory by stmatrix, one record per step, 64 / 128 / 256-token
+// tiles, an issuer under a lane test).  What bounds it now: up to ~128 tokens HBM plus ~5 us per launch of start-up, drain
+// and the split's epilogue; beyond, the shared-memory port (records in and out, activation tile in and out:
+// 3.1 KB + 32 B x tokens per record at 128 B per cycle; 800 cycles per k-tile at 304 tokens against 608 of MMAs).
+//
+// *Slot parity.*  An mbarrier tells only its current phase from the previous one, so a waiter must never be two phases
+// away.  With two decode groups that alternate pairs every A slot and record slot has to belong to one group (whose own
+// program order guarantees that): both counts are even when DG = 2.
+//
 // The KS CTAs that split the k range of one (row block, token tile) form a thread-block cluster (blockIdx.x % KS is
 // the rank).  After its main loop every CTA parks its fp32 accumulator tile in its own shared memory; after a cluster
 // barrier CTA j adds the KS tiles for its share of the token columns through distributed shared memory, in rank
 // order (bit-identical from run to run), and stores BF16.  No partial sums travel through global memory.
-template <bool GROUPED>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int DG, bool GROUPED>
+__global__ void __launch_bounds__(gemm_threads<DG>(), DG == 1 ? 2 : 1)
 gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ WMaps wmaps) {
-  constexpr int NMMA = DG;                                     // issuer warps; a.nmma of them work
+  constexpr int NDW = DG * NDEC;                                              // decode warps
+  constexpr int W_RAW = NDW, W_X = NDW + 1, W_MMA = NDW + 2;                  // role warps
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int NT = a.NT, S = a.stages, R = a.rstages;
+  __shared__ int s_used[(gemm_threads<DG>() + 31) / 32];
+  uint8_t* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);   // (stays a shared-memory pointer to the compiler)
+  const int NT = a.NT, SA = a.astages, SX = a.xstages, R = a.rstages;
   const int XT = NT * 128;                       // bytes of an activation tile
-  const int STAGE = A_TILE + XT;                 // tile stage: decoded weight tile + activation tile
-  uint8_t* rawring = smem + (size_t)S * STAGE;                       // [R] record slots (deep: covers HBM latency)
-  // one barrier per tile stage collects both operands: 8 decode-warp arrivals + the activation tile's TMA bytes
-  uint64_t* ready = reinterpret_cast<uint64_t*>(smem + a.bar_off);   // [S] both operands of the stage are in place
-  uint64_t* empty = ready + S;                                       // [S] MMAs that read the stage have completed
-  uint64_t* rfull = empty + S;                                       // [R] records landed
+  uint8_t* rawring = smem + (size_t)SX * XT;                         // [R] record slots
+  uint64_t* aready = reinterpret_cast<uint64_t*>(smem + a.bar_off);  // [SA] the slot's weight tiles are in tensor memory
+  uint64_t* aempty = aready + SA;                                    // [SA] the MMAs that read the slot have completed
+  uint64_t* xfull = aempty + SA;                                     // [SX] activation tile landed
+  uint64_t* xempty = xfull + SX;                                     // [SX] the MMAs that read it have completed
+  uint64_t* rfull = xempty + SX;                                     // [R] records landed
   uint64_t* rempty = rfull + R;                                      // [R] records copied to registers
   uint64_t* accbar = rempty + R;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accbar + 1);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // unit of this CTA
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0);   // (a warp-uniform value to the compiler)
+  // unit of this CTA.  Dense: the token tiles of a row block run next to each other (its records then come from HBM once
+  // and from L2 for the other tiles); grouped: the row blocks of a pair block do (they share the gathered activations)
   const int ks = blockIdx.x % a.KS, rt = blockIdx.x / a.KS;
-  const int rb = rt % a.RB, tt = rt / a.RB;
-  const int k0 = (int)((long long)a.NG * ks / a.KS), k1 = (int)((long long)a.NG * (ks + 1) / a.KS);
-  const int nk = k1 - k0;
+  const int rb = GROUPED ? rt % a.RB : a.rb0 + rt / a.TT, tt = GROUPED ? rt / a.RB : rt % a.TT;
+  // whole pairs of k-tiles; an odd last tile is paired with one beyond the matrix, which both tensor maps fill with zeros
+  const int pairs = (a.NG + PAIR - 1) / PAIR;
+  const int p0 = (int)((long long)pairs * ks / a.KS), np = (int)((long long)pairs * (ks + 1) / a.KS) - p0;
+  const int k0 = p0 * PAIR;
   const int tok0 = tt * NT;
   // the matrix this CTA multiplies by: the one of the call, or (grouped) the expert of pair block tt
   const int* eo = a.eo;
@@ -144,6 +181,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   uint16_t* Yp = a.Y;
   float* Yfp = a.Yf;
   long long Mp = a.M;
+  int ncol = GROUPED ? NT : min(NT, a.B - tok0);                 // token columns that exist
   if (!GROUPED && a.nlist > 0) {                                 // a list: the member this row block belongs to
     int m = 0;
     while (m + 1 < a.nlist && rb >= a.rbend[m]) ++m;
@@ -159,228 +197,273 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
     eo = reinterpret_cast<const int*>(a.eop[expert]);
     el = reinterpret_cast<const uint32_t*>(a.elp[expert]);
     wm = a.maps + expert;
+    // pairs in the block: one past the last entry that is not padding
+    int used = 0;
+    if (tid < NT) {
+      const int p = a.sorted[tok0 + tid];
+      used = (p >= 0 && p < a.B) ? tid + 1 : 0;
+    }
+    used = __reduce_max_sync(FULL, used);
+    if (lane == 0) s_used[warp] = used;
+    __syncthreads();
+    ncol = 0;
+    for (int w = 0; w * 32 < NT; ++w) ncol = max(ncol, s_used[w]);
+    if (ncol == 0) return;
   }
+  const int nmma = GROUPED ? (ncol + 15) & ~15 : NT;             // token columns the MMAs cover
 
   if (tid == 0) {
-    for (int s = 0; s < S; ++s) { mbar_init(ready + s, NDEC + 1); mbar_init(empty + s, 1); }
+    for (int s = 0; s < SA; ++s) { mbar_init(aready + s, NDEC); mbar_init(aempty + s, 1); }
+    for (int s = 0; s < SX; ++s) { mbar_init(xfull + s, 1); mbar_init(xempty + s, 1); }
     for (int r = 0; r < R; ++r) { mbar_init(rfull + r, 1); mbar_init(rempty + r, NDEC); }
-    mbar_init(accbar, NMMA);                                       // every issuer warp arrives, working or not
+    mbar_init(accbar, 1);
     fence_barrier_init();
   }
   if (warp == W_MMA) {
-    tmem_alloc(tmem_slot, (uint32_t)(a.nmma * NT));              // 64 .. 256 columns: one accumulator per working issuer
+    tmem_alloc(tmem_slot, (uint32_t)a.tmem_cols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem_a = tmem + (uint32_t)((NT + 31) & ~31);    // the weight tiles' columns follow the accumulator
   pdl_launch_dependents();
 
   if (warp == W_RAW) {
-    // ---------------------------------------------------------------- record producer: one tiled TMA load per k-tile
-    // fetches the eight records (row tiles rb * 8 .. + 7 of column group k0 + i) through a 3-D view of the tree
-    // [row tile][column group][194 x u64]; eight separate 1552-byte bulk copies per k-tile would cost far more issue time
-    if (lane == 0) {
-      for (int i = 0, r = 0, k = 0; i < nk; ++i, r = (r + 1 == R ? 0 : r + 1), k += (r == 0)) {
-        if (k > 0 && !GW(rempty + r, (uint32_t)(k - 1) & 1u)) { atomicExch(a.status, ERR_WAIT_EMPTY); break; }
+    // ---------------------------------------------------------------- record producer: one tiled TMA load per pair of
+    // k-tiles fetches sixteen records (row tiles rb * 8 .. + 7, column groups k0 + 2 i and + 1) through a 3-D view of the
+    // tree [row tile][column group][194 x u64]; separate bulk copies would cost far more issue time
+    for (int i = 0, r = 0, k = 0; i < np; ++i, r = (r + 1 == R ? 0 : r + 1), k += (r == 0)) {
+      if (k > 0 && !GW(rempty + r, (uint32_t)(k - 1) & 1u)) { if (lane == 0) atomicExch(a.status, ERR_WAIT_EMPTY); break; }
+      if (elect_one()) {
         mbar_expect_tx(rfull + r, (uint32_t)RAW_SLOT);
-        tma_load_3d(rawring + (size_t)r * RAW_SLOT, wm, 0, k0 + i, lrb * 8, rfull + r);
+        tma_load_3d(rawring + (size_t)r * RAW_SLOT, wm, 0, k0 + PAIR * i, lrb * 8, rfull + r);
       }
+      __syncwarp();
     }
   } else if (warp == W_X) {
     // ---------------------------------------------------------------- activation producer.  The activations are the
     // only input an earlier kernel of the stream may still be writing: with programmatic dependent launch the CTA
     // starts (and its record producer streams weights) under the tail of that kernel, and this thread is the one that
     // waits for it.  Everything that touches the output is downstream of the first activation tile.
-    if (lane == 0) {
-      pdl_wait();
-      for (int i = 0, s = 0, k = 0; i < nk; ++i, s = (s + 1 == S ? 0 : s + 1), k += (s == 0)) {
-        if (k > 0 && !GW(empty + s, (uint32_t)(k - 1) & 1u)) { atomicExch(a.status, ERR_WAIT_EMPTY); break; }
-        mbar_expect_tx(ready + s, (uint32_t)XT);
-        tma_load_2d(smem + (size_t)s * STAGE + A_TILE, &xmap, (k0 + i) * 64, tok0, ready + s);
+    pdl_wait();
+    const int box = GROUPED ? XBOX_GROUPED : (NT > 256 ? NT / 2 : NT);       // rows per load
+    const int nbox = GROUPED ? (nmma + XBOX_GROUPED - 1) / XBOX_GROUPED : (NT > 256 ? 2 : 1);
+    for (int i = 0, s = 0, k = 0; i < np * PAIR; ++i, s = (s + 1 == SX ? 0 : s + 1), k += (s == 0)) {
+      if (k > 0 && !GW(xempty + s, (uint32_t)(k - 1) & 1u)) { if (lane == 0) atomicExch(a.status, ERR_WAIT_EMPTY); break; }
+      if (elect_one()) {
+        mbar_expect_tx(xfull + s, (uint32_t)(nbox * box * 128));
+        for (int b = 0; b < nbox; ++b)
+          tma_load_2d(smem + (size_t)s * XT + (size_t)b * box * 128, &xmap, (k0 + i) * 64, tok0 + b * box, xfull + s);
       }
+      __syncwarp();
     }
-  } else if (warp >= W_MMA) {
-    // ---------------------------------------------------------------- MMA issuers.  The serial cost of one thread
-    // per k-tile (its barrier wait, four tcgen05.mma and the commit) is of the order of a k-tile's share of the decode
-    // time, so one issuer would hold the pipeline back.  Two issuers alternate k-tiles, each into its own accumulator (the epilogue adds the two in a
-    // fixed order), so the serial cost per k-tile halves and the result does not depend on which issuer ran first.
-    // This needs an even number of tile stages and record slots: then every stage and slot belongs to one decode group
-    // and one issuer, which use it in their own program order.  (A waiter may be at most one phase ahead of an mbarrier:
-    // with shared stages an issuer could ask for use k of a stage whose use k - 1, the other issuer's, has not
-    // completed, and the parity test would pass on use k - 2.)  With three stages (256-token tiles) one issuer works.
-    const int m = warp - W_MMA;
-    if (lane == 0 && m >= a.nmma) mbar_arrive(accbar);
-    if (lane == 0 && m < a.nmma) {
-      const uint32_t acc = tmem + (uint32_t)(m * NT);
-      int s = m % S, k = m / S;
-      for (int i = m; i < nk; i += a.nmma) {
-        if (!GW(ready + s, (uint32_t)k & 1u)) {
-          atomicExch(a.status, ERR_WAIT_MMA);
-          break;
-        }
-        tc_fence_after();
-        const uint32_t sa = smem_addr(smem + (size_t)s * STAGE);
-        const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + A_TILE);
+  } else if (warp == W_MMA) {
+    // ---------------------------------------------------------------- MMA issuer.  The whole warp waits; one elected
+    // lane issues.  The loop must stay warp-uniform: tensor-core and TMA instructions take their operands from uniform
+    // registers, and under a lane test (`if (lane == 0)`) the compiler has to serialise over the lanes around each one
+    // (measured: ~1000 cycles for the four MMAs and the commit of a k-tile instead of < 200).
+    // beyond 256 tokens one MMA cannot cover the tile: two, of (up to 16 tokens) different width
+    const int half = NT > 256 ? ((NT / 2 + 15) & ~15) : 0;
+    const uint32_t idesc = mma_idesc(half ? half : nmma), idesc2 = mma_idesc(half ? NT - half : 16);
+    int xs = 0, xk = 0;
+    bool ok = true;
+    for (int i = 0, s = 0, k = 0; ok && i < np; ++i, s = (s + 1 == SA ? 0 : s + 1), k += (s == 0)) {
+      ok = GW(aready + s, (uint32_t)k & 1u);
+      tc_fence_after();
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tc_mma(acc, da + 2 * j, db + 2 * j, a.idesc, (i >= a.nmma || j) ? 1u : 0u);
-        tc_commit(empty + s);
-        s += a.nmma; while (s >= S) { s -= S; ++k; }
+      for (int h = 0; h < PAIR; ++h) {
+        ok = ok && GW(xfull + xs, (uint32_t)xk & 1u);
+        if (!ok) break;
+        const uint64_t db = smem_desc_sw128(smem_addr(smem + (size_t)xs * XT));
+        const uint32_t ta = tmem_a + (uint32_t)((s * PAIR + h) * A_COLS);
+        if (elect_one()) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            tc_mma(tmem, ta + 8 * j, db + 2 * j, idesc, (i || h || j) ? 1u : 0u);
+            if (half)
+              tc_mma(tmem + (uint32_t)half, ta + 8 * j, db + 2 * j + (uint64_t)(half * 8), idesc2, (i || h || j) ? 1u : 0u);
+          }
+          tc_commit(xempty + xs);
+          if (h == PAIR - 1) tc_commit(aempty + s);
+        }
+        __syncwarp();
+        if (++xs == SX) { xs = 0; ++xk; }
       }
-      tc_commit(accbar);                                          // arrives when every MMA of this issuer has completed
     }
+    if (!ok && lane == 0) atomicExch(a.status, ERR_WAIT_MMA);
+    if (elect_one()) tc_commit(accbar);                           // arrives when every MMA has completed
+    __syncwarp();
   } else {
     // ---------------------------------------------------------------- decode warps: group g = warp / 8 takes the
-    // k-tiles i = g, g + DG, ...; warp r of a group decodes record r (rows 16 r .. 16 r + 15 of the block)
-    const int grp = warp / NDEC, rec = warp % NDEC;
-    const size_t rbase = (size_t)(lrb * 8 + rec) * a.NG + k0;
-    // Escape entries are fetched one k-tile ahead: the list offsets of this warp's records come 32 k-tiles at a time
-    // (lane l holds the offsets of k-tile eo_base + l) and the first 32 entries of the next record are requested before
-    // this record is decoded, so no global-load latency sits between the records landing and the tile being handed
-    // to the tensor core (one record in six has an escape; eight warps must all arrive before the MMA can start)
+    // pairs i = g, g + DG, ...  A warp reaches only the 32 tensor-memory lanes of its quadrant (warp % 4), i.e. the two
+    // 16-row tiles 2 (warp % 4) and 2 (warp % 4) + 1: warps w and w + 4 of a group take one each.
+    const int grp = warp / NDEC, w8 = warp % NDEC, rec = 2 * (w8 & 3) + (w8 >> 2);
+    const uint32_t my_a = tmem_a + ((uint32_t)(rec * 16) << 16);
+    const uint8_t* const my_raw = rawring + rec * (PAIR * REC);
+    const int* const my_eo = eo + (size_t)(lrb * 8 + rec) * a.NG + k0;
+    const int last = a.NG - k0;                                    // records of this row tile from k0 on
+    // The two records of a pair are neighbours in memory order, so their escapes are one run of the list.  It is fetched
+    // one pair ahead: the list offsets come 32 pairs at a time (lane l holds those of pair eo_base + l) and the first 32
+    // entries of the next pair are requested before this pair is decoded, so no global-load latency sits between the
+    // records landing and the tiles being handed to the tensor core
     int eo_base = 0, eo_lo = 0, eo_hi = 0;
-    unsigned emask = 0u;                                           // bit l: k-tile eo_base + l of this warp has escapes
+    unsigned emask = 0u;                                           // bit l: pair eo_base + l of this warp has escapes
     auto load_offsets = [&](int first) {
       eo_base = first;
-      const int j = first + lane;
-      eo_lo = j < nk ? __ldg(eo + rbase + j) : 0;
-      eo_hi = j < nk ? __ldg(eo + rbase + j + 1) : 0;
+      const int j = (first + lane) * PAIR;
+      eo_lo = j < last ? __ldg(my_eo + j) : 0;
+      eo_hi = j < last ? __ldg(my_eo + min(j + PAIR, last)) : 0;
       emask = __ballot_sync(FULL, eo_hi > eo_lo);
     };
     int lo = 0, hi = 0;
     uint32_t ent = 0u;
-    if (grp < nk) {
-      load_offsets(grp);
-      if (emask & 1u) {
-        lo = __shfl_sync(FULL, eo_lo, 0);
-        hi = __shfl_sync(FULL, eo_hi, 0);
+    auto fetch_escapes = [&](int i) {                              // (lo, hi, ent) of pair i
+      lo = hi = 0;
+      if (i >= np) return;
+      if (i - eo_base >= 32) load_offsets(i);
+      const int off = i - eo_base;
+      if ((emask >> off) & 1u) {                                  // most pairs have none: one bit test
+        lo = __shfl_sync(FULL, eo_lo, off);
+        hi = __shfl_sync(FULL, eo_hi, off);
         if (lane < hi - lo) ent = __ldg(el + lo + lane);
       }
-    }
-    int s = grp % S, k = grp / S, r = grp % R, rk = grp / R;          // tile stage / use count, record slot / use count
-    for (int i = grp; i < nk; i += DG) {
-      int nlo = 0, nhi = 0;
-      uint32_t nent = 0u;
-      if (i + DG < nk) {
-        if (i + DG - eo_base >= 32) load_offsets(i + DG);
-        const int off = i + DG - eo_base;
-        if ((emask >> off) & 1u) {                                // five records in six have none: one bit test
-          nlo = __shfl_sync(FULL, eo_lo, off);
-          nhi = __shfl_sync(FULL, eo_hi, off);
-          if (lane < nhi - nlo) nent = __ldg(el + nlo + lane);
-        }
-      }
-      if (!wait_decode(rfull + r, (uint32_t)rk & 1u)) {
+    };
+    load_offsets(grp);
+    fetch_escapes(grp);
+    int s = grp % SA, r = grp % R;                                 // A slot, record slot
+    uint32_t sph = (uint32_t)(grp / SA) & 1u, rph = (uint32_t)(grp / R) & 1u;
+    bool first = grp < SA;                                         // the slot has not been used yet: nothing to wait for
+    for (int i = grp; i < np; i += DG) {
+      if (!mbar_wait(rfull + r, rph)) {
         if (lane == 0) atomicExch(a.status, ERR_WAIT_FULL);
         break;
       }
-      const RecRegs rr = load_rec_shared(rawring + (size_t)r * RAW_SLOT + rec * REC, lane);
+      RecRegs rr[PAIR];
+#pragma unroll
+      for (int h = 0; h < PAIR; ++h) rr[h] = load_rec_shared(my_raw + r * RAW_SLOT + h * REC, lane);
+      const int clo = lo, chi = hi;
+      const uint32_t cent = ent;
+      fetch_escapes(i + DG);
       __syncwarp();
       if (lane == 0) mbar_arrive(rempty + r);                     // the slot can be refilled while we decode
-      uint32_t A[4][4];
-      decode_frag(rr, A);
-      {
-        const int n = min(32, hi - lo);
-        for (int e = 0; e < n; ++e) patch_entry(A, __shfl_sync(FULL, ent, e), lane);
+      r += DG; if (r >= R) { r -= R; rph ^= 1u; }
+      bool ok = true;
+#pragma unroll
+      for (int h = 0; h < PAIR; ++h) {
+        uint32_t A[4][4];
+        decode_frag(rr[h], A);
+        if (clo < chi) {                                          // entries of record h: bits 10..12 = column group % 8
+          const uint32_t want = (uint32_t)(k0 + i * PAIR + h) & 7u;
+          for (int base = clo; base < chi; base += 32) {
+            const uint32_t mine = base == clo ? cent : (lane < chi - base ? __ldg(el + base + lane) : 0u);
+            unsigned m = __ballot_sync(FULL, lane < chi - base && ((mine >> 10) & 7u) == want);
+            while (m) {
+              const int src = __ffs(m) - 1;
+              m &= m - 1;
+              patch_entry(A, __shfl_sync(FULL, mine, src), lane);
+            }
+          }
+        }
+        if (h == 0) {
+          if (!first) ok = mbar_wait(aempty + s, sph ^ 1u);        // the MMAs of the slot's last use are done
+          __syncwarp();
+          if (!ok) break;
+          tc_fence_after();
+        }
+        tmem_st_frag(my_a + (uint32_t)((s * PAIR + h) * A_COLS), A);
       }
-      for (int base = lo + 32; base < hi; base += 32) {          // a crowded record: the rest of its list
-        const int n = min(32, hi - base);
-        const uint32_t mine = (lane < n) ? __ldg(el + base + lane) : 0u;
-        for (int e = 0; e < n; ++e) patch_entry(A, __shfl_sync(FULL, mine, e), lane);
-      }
-      lo = nlo; hi = nhi; ent = nent;
-      if (k > 0 && !wait_decode(empty + s, (uint32_t)(k - 1) & 1u)) {   // the MMAs of the stage's last use are done
+      if (!ok) {
         if (lane == 0) atomicExch(a.status, ERR_WAIT_EMPTY);
         break;
       }
-      uint8_t* st = smem + (size_t)s * STAGE;
-      // lane l addresses row (l & 7) of matrix (l >> 3): matrices = (rows 0-7 | 8-15) x (16-byte chunk 2q | 2q+1)
-      const int mrow = rec * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
-      const uint32_t rowaddr = smem_addr(st) + mrow * 128;
-      const int chalf = lane >> 4;
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        stmatrix_x4(rowaddr + (uint32_t)(((2 * q + chalf) ^ (mrow & 7)) << 4), A[q][0], A[q][1], A[q][2], A[q][3]);
-      fence_proxy_async();
+      tmem_wait_st();
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ready + s);
-      s += DG; while (s >= S) { s -= S; ++k; }
-      r += DG; while (r >= R) { r -= R; ++rk; }
+      if (lane == 0) mbar_arrive(aready + s);
+      s += DG; if (s >= SA) { s -= SA; sph ^= 1u; first = false; }
     }
-    // ---------------------------------------------------------------- epilogue 1: accumulator -> own shared memory
+    // ---------------------------------------------------------------- epilogue 1: accumulator -> registers
+    __syncwarp();
     const bool acc_ok = GW(accbar, 0u);
     if (!acc_ok && lane == 0) atomicExch(a.status, ERR_WAIT_ACC);
+    __syncwarp();
     tc_fence_after();
-    float* stg = reinterpret_cast<float*>(smem);                 // [NT][128] fp32, over the (now idle) ring
     const int q4 = warp & 3, cg = warp >> 2;                     // TMEM lane quadrant, column share of the warp
-    const int cper = NT / (NDW / 4);
-    const bool two = a.nmma > 1 && nk > 1;                       // the second issuer had a k-tile
-    for (int c0 = cg * cper; c0 < (cg + 1) * cper; c0 += 16) {
-      uint32_t v[32], w[32];                                     // (the x16 load fills the first sixteen)
-      const uint32_t t0 = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)c0;
-      tmem_ld16(t0, v);
-      if (two) {
-        tmem_ld16(t0 + (uint32_t)NT, w);
+    float* stg = reinterpret_cast<float*>(smem);                 // [NT][128] fp32, over the (now idle) rings
+    for (int c0 = cg * 16; c0 < nmma; c0 += (NDW / 4) * 16) {
+      uint32_t v[16];
+      tmem_ld16(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)c0, v);
+      if (!GROUPED && a.KS > 1) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+        for (int j = 0; j < 16; ++j) stg[(size_t)(c0 + j) * 128 + q4 * 32 + lane] = __uint_as_float(v[j]);
+      } else {
+        // whole k range: this lane holds row q4 * 32 + lane of 16 token columns.  Lanes pair up (even: column j, odd:
+        // column j + 1, two rows each) so that a store instruction writes 4 bytes per lane, 64 bytes per column
+        const long long m0 = (long long)lrb * 128 + q4 * 32 + (lane & ~1);
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          const uint32_t give = (lane & 1) ? v[j] : v[j + 1], keep = (lane & 1) ? v[j + 1] : v[j];
+          const uint32_t got = __shfl_xor_sync(FULL, give, 1);
+          const float x0 = __uint_as_float((lane & 1) ? got : keep), x1 = __uint_as_float((lane & 1) ? keep : got);
+          const int c = c0 + j + (lane & 1);
+          if (c < ncol && acc_ok) {
+            long long row = tok0 + c;
+            if (GROUPED) row = a.sorted[tok0 + c];                 // result rows go back to their pair index
+            if (!GROUPED || (row >= 0 && row < a.B)) {
+              *reinterpret_cast<uint32_t*>(Yp + (size_t)row * Mp + m0) = pack_bf16(x0, x1);
+              if (Yfp) *reinterpret_cast<float2*>(Yfp + (size_t)row * Mp + m0) = make_float2(x0, x1);
+            }
+          }
+        }
       }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) stg[(size_t)(c0 + j) * 128 + q4 * 32 + lane] = __uint_as_float(v[j]);
     }
   }
   tc_fence_before();
   __syncwarp();
-  cluster_sync_all();                                            // every CTA of the cluster has parked its tile
-  if (warp < NDW) {
-    // ---------------------------------------------------------------- epilogue 2: add the KS tiles, rank order
-    const int ncol = GROUPED ? NT : min(NT, a.B - tok0);        // grouped: padding pairs are filtered per column
-    const int c_lo = (int)((long long)NT * ks / a.KS), c_hi = (int)((long long)NT * (ks + 1) / a.KS);
-    const uint32_t mine = smem_addr(smem);
-    const int c_end = min(c_hi, ncol);
-    // two columns per pass, every partial tile's float4 requested before the first add: distributed-shared-memory
-    // reads have a long latency, so the loads of a pass must all be in flight together
-    for (int c = c_lo + warp; c < c_end; c += 2 * NDW) {
-      const int c2 = c + NDW;
-      float4 v0[8], v1[8];
+  if (GROUPED || a.KS == 1) {
+    __syncthreads();
+  } else {
+    cluster_sync_all();                                          // every CTA of the cluster has parked its tile
+    if (warp < NDW) {
+      // -------------------------------------------------------------- epilogue 2: add the KS tiles, rank order
+      const int c_lo = (int)((long long)ncol * ks / a.KS), c_end = (int)((long long)ncol * (ks + 1) / a.KS);
+      const uint32_t mine = smem_addr(smem);
+      // CPP columns per pass, every partial tile's float4 requested before the first add: distributed-shared-memory
+      // reads have a long latency, so the loads of a pass must all be in flight together
+      constexpr int CPP = DG;                                    // (DG = 1 has 80 registers per thread, DG = 2 twice the columns)
+      for (int c = c_lo + warp; c < c_end; c += CPP * NDW) {
+        float4 v[CPP][8];
 #pragma unroll
-      for (int p = 0; p < 8; ++p) {
-        if (p < a.KS) {
-          v0[p] = ld_cluster_f4(map_to_cta(mine + (uint32_t)((c * 128 + 4 * lane) * 4), (uint32_t)p));
-          if (c2 < c_end) v1[p] = ld_cluster_f4(map_to_cta(mine + (uint32_t)((c2 * 128 + 4 * lane) * 4), (uint32_t)p));
-        }
-      }
+        for (int h = 0; h < CPP; ++h)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int cc = h ? c2 : c;
-        if (cc >= c_end) break;
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int p = 0; p < 8; ++p)
+            if (p < a.KS && c + h * NDW < c_end)
+              v[h][p] = ld_cluster_f4(map_to_cta(mine + (uint32_t)(((c + h * NDW) * 128 + 4 * lane) * 4), (uint32_t)p));
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
-          if (p < a.KS) {
-            const float4 v = h ? v1[p] : v0[p];
-            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-          }
+        for (int h = 0; h < CPP; ++h) {
+          const int cc = c + h * NDW;
+          if (cc >= c_end) break;
+          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int p = 0; p < 8; ++p)
+            if (p < a.KS) { sum.x += v[h][p].x; sum.y += v[h][p].y; sum.z += v[h][p].z; sum.w += v[h][p].w; }
+          const size_t o = (size_t)(tok0 + cc) * Mp + lrb * 128 + 4 * lane;
+          uint2 packed;
+          packed.x = pack_bf16(sum.x, sum.y);
+          packed.y = pack_bf16(sum.z, sum.w);
+          *reinterpret_cast<uint2*>(Yp + o) = packed;
+          if (Yfp) *reinterpret_cast<float4*>(Yfp + o) = sum;
         }
-        long long row = tok0 + cc;
-        if (GROUPED) {                                            // result rows go back to their pair index
-          row = a.sorted[tok0 + cc];
-          if (row < 0 || row >= a.B) continue;
-        }
-        const size_t o = (size_t)row * Mp + lrb * 128 + 4 * lane;
-        uint2 packed;
-        packed.x = pack_bf16(sum.x, sum.y);
-        packed.y = pack_bf16(sum.z, sum.w);
-        *reinterpret_cast<uint2*>(Yp + o) = packed;
-        if (Yfp) *reinterpret_cast<float4*>(Yfp + o) = sum;
       }
     }
+    __syncwarp();
+    cluster_sync_all();                                          // nobody leaves while a peer still reads its tile
   }
-  __syncwarp();
-  cluster_sync_all();                                            // nobody leaves while a peer still reads its tile
   if (warp == W_MMA) {
     __syncwarp();
-    tmem_dealloc(tmem, (uint32_t)(a.nmma * NT));
+    tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
   }
 }
 
@@ -402,36 +485,42 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-struct GemmPlan { int NT, TT, RB, KS, stages, rstages, nmma, bar_off; size_t smem; };
+struct GemmPlan {
+  int RB1, KS1;                                                  // the first RB1 row blocks go out in a launch of their own, split KS1 ways
+  int NT, TT, RB, KS, DG, astages, xstages, rstages, bar_off, tmem_cols;
+  size_t smem;
+};
 
-template <bool GROUPED>
+template <int DG, bool GROUPED>
 int gemm_attr() {                                                // once per device: opt in to the large dynamic shared memory
   static bool set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !set[dev]) {
-    if (int e = st::cuda_fail(cudaFuncSetAttribute(gemm_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   220 * 1024), "st_gemm: shared memory attribute"))
+    if (int e = st::cuda_fail(cudaFuncSetAttribute(gemm_kernel<DG, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   DG == 1 ? 113 * 1024 : 220 * 1024), "st_gemm: shared memory attribute"))
       return e;
     set[dev] = true;
   }
   return 0;
 }
 
-// CTAs that can be resident at once when launched as clusters of ks (one CTA per SM): a cluster lives inside one GPC,
-// so sizes that do not divide a GPC's SM count strand SMs (clusters of 3 fit 44 times, not 49: a 48-cluster grid then
-// runs as two waves).  Asked from the driver once per (device, cluster size, token tile).
-long long resident_ctas(int ks, int NT, size_t smem, int sms) {
-  static int cache[64][9][3] = {};
+// CTAs that can be resident at once when launched as clusters of ks: a cluster lives inside one GPC, so sizes that do not
+// divide a GPC's SM count strand SMs (one CTA per SM: clusters of 3 fit 45 times, not 49).  Asked from the driver once per
+// (device, cluster size, kernel).  The driver's answer assumes one CTA per SM for every kernel that allocates tensor
+// memory; the DG = 1 kernel takes half of an SM's, and two do share an SM (start times of 296 such CTAs: all at once).
+template <int DG>
+long long resident_ctas(int ks, size_t smem, int sms) {
+  static int cache[64][9] = {};
+  const int per_sm = DG == 1 ? 2 : 1;
   int dev = 0;
   cudaGetDevice(&dev);
-  const int ti = NT <= 64 ? 0 : (NT <= 128 ? 1 : 2);
-  if (ks == 1 || dev < 0 || dev >= 64) return sms;
-  if (cache[dev][ks][ti] == 0) {
+  if (ks == 1 || dev < 0 || dev >= 64) return (long long)sms * per_sm;
+  if (cache[dev][ks] == 0) {
     int n = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(ks * sms));
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(gemm_threads<DG>());
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -440,75 +529,105 @@ long long resident_ctas(int ks, int NT, size_t smem, int sms) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (gemm_attr<false>() != 0 || cudaOccupancyMaxActiveClusters(&n, gemm_kernel<false>, &cfg) != cudaSuccess || n <= 0) {
+    if (gemm_attr<DG, false>() != 0 || cudaOccupancyMaxActiveClusters(&n, gemm_kernel<DG, false>, &cfg) != cudaSuccess || n <= 0) {
       (void)cudaGetLastError();
       n = sms / ks;                                              // no answer (no device): assume perfect packing
     }
-    cache[dev][ks][ti] = n;
+    cache[dev][ks] = n;
   }
-  return (long long)cache[dev][ks][ti] * ks;
+  return (long long)cache[dev][ks] * ks * per_sm;
 }
 
-// rings and issuers for a token tile of NT
+// rings for a token tile of NT
 void gemm_rings(GemmPlan& p) {
-  const size_t stage = A_TILE + (size_t)p.NT * 128;
+  const size_t xt = (size_t)p.NT * 128;
   const size_t stg = (size_t)p.NT * 128 * 4;                      // the parked accumulator tile reuses the rings
-  // tile stages (decoded weight tile + activation tile): enough to cover the L2 latency of the activation loads; the
-  // rest of the shared memory goes to the record ring, which covers the HBM latency
-  p.stages = p.NT >= 256 ? 3 : 4;
-  p.rstages = (int)((212 * 1024 - p.stages * stage) / RAW_SLOT);
-  if (p.rstages > 12) p.rstages = 12;
-  // The two decode groups alternate k-tiles.  A decode warp waits for the fill of a record slot by the parity of that
-  // slot's use count, and an mbarrier tells only the current phase from the previous one, so a waiter must never be
-  // two fills ahead.  With an even slot count every slot belongs to one group, whose own program order guarantees
-  // that; with an odd count the groups share slots, and a group that runs ahead while a bulk copy of the other
-  // group's k-tile is still in flight passes its wait on the stale phase, reads old records and releases the slot a
-  // second time.  So: always an even number of record slots.  (Tile stages may be odd: their waits are on the
-  // previous use of a stage.)
-  p.rstages &= ~1;
-  // two MMA issuers need every tile stage owned by one decode group as well: an even count of stages
-  p.nmma = (p.stages % 2 == 0 && p.rstages >= 4) ? 2 : 1;
-  size_t ring = (size_t)p.stages * stage + (size_t)p.rstages * RAW_SLOT;
-  ring = (ring + 15) & ~(size_t)15;
+  const size_t slack = 1024 /* alignment */ + 512 /* barriers */;
+  const int acc = (p.NT + 31) & ~31;
+  p.DG = p.NT <= 128 ? 1 : 2;
+  p.tmem_cols = p.DG == 1 ? 256 : 512;
+  const size_t budget = (p.DG == 1 ? 112 : 216) * 1024 - slack;
+  p.astages = (p.tmem_cols - acc) / (PAIR * A_COLS);
+  if (p.astages > 4) p.astages = 4;
+  if (p.DG == 2) p.astages &= ~1;                                 // slot parity: see the kernel
+  // activation tiles: enough to cover the L2 latency (four if they fit beside two record slots); the rest of the shared
+  // memory goes to the record ring, which covers the HBM latency
+  p.xstages = 4;
+  while (p.xstages > 2 && p.xstages * xt + 2 * RAW_SLOT > budget) --p.xstages;
+  p.rstages = (int)((budget - p.xstages * xt) / RAW_SLOT);
+  if (p.rstages > 6) p.rstages = 6;
+  if (p.DG == 2) p.rstages &= ~1;
+  p.xstages = (int)((budget - (size_t)p.rstages * RAW_SLOT) / xt);
+  if (p.xstages > 6) p.xstages = 6;
+  size_t ring = p.xstages * xt + (size_t)p.rstages * RAW_SLOT;
   if (ring < stg) ring = stg;
+  ring = (ring + 15) & ~(size_t)15;
   p.bar_off = (int)ring;
-  p.smem = ring + 1024 /* alignment slack */ + 512 /* barriers */;
+  p.smem = ring + slack;
 }
+
+constexpr int NT_MAX = 320;                                      // 320 accumulator columns + 4 weight tiles of 32 fill TMEM
 
 GemmPlan gemm_plan(long long M, long long N, long long B) {
   GemmPlan p;
-  p.NT = B <= 64 ? 64 : (B <= 128 ? 128 : 256);
-  p.TT = (int)((B + p.NT - 1) / p.NT);
+  // the fewest token tiles (every tile decodes the records again), of equal width
+  p.TT = (int)((B + NT_MAX - 1) / NT_MAX);
+  const int per = (int)((B + p.TT - 1) / p.TT);
+  p.NT = (per + 15) & ~15;                                        // MMA widths: multiples of 16
   p.RB = (int)(M / 128);
   const int NG = (int)(N / 64), sms = st::sm_count();
-  const long long units = (long long)p.RB * p.TT;
   gemm_rings(p);
-  // Split of the k range = cluster size (<= 8).  A CTA's time is its k-tiles plus a fixed part (start-up, pipeline fill,
-  // epilogue; the epilogue grows with the tiles to add through distributed shared memory); a grid larger than the
-  // CTAs that are resident at once runs in waves, each paying all of it again.  Take the split with the least
-  // estimated time (the constants are in units of one k-tile of a 64-token tile).
-  int best = 1;
-  double best_t = 1e30;
-  const int ksmax = NG / 4 < 1 ? 1 : (NG / 4 > 8 ? 8 : NG / 4);
-  const double tile = p.NT >= 256 ? 1.4 : (p.NT >= 128 ? 1.08 : 1.0);
-  for (int ks = 1; ks <= ksmax; ++ks) {
-    const long long ctas = units * ks;
-    const long long slots = resident_ctas(ks, p.NT, p.smem, sms);
-    if (slots <= 0) continue;
-    const long long waves = (ctas + slots - 1) / slots;
-    const double t = (double)waves * ((double)((NG + ks - 1) / ks) * tile + 14.0 + 0.8 * ks * p.NT / 64.0);
-    if (t < best_t - 1e-9) { best_t = t; best = ks; }
+  // Split of the k range = cluster size (<= 8): the least estimated time in us, fitted to launches of the four projection
+  // shapes of a 4096 / 12288 model in a graph (32 to 192 row blocks, 16 to 304 tokens, splits 1 to 8; within 10 %):
+  //   start-up + drain, the epilogue (grows with the tiles to add through distributed shared memory), and per pair of
+  //   k-tiles a time that grows with the CTAs that stream at once (two per SM) or with the token tile (one per SM).
+  // A grid larger than the CTAs that are resident at once runs in waves.
+  const int pairs = (NG + PAIR - 1) / PAIR, ksmax = pairs / 4 < 1 ? 1 : (pairs / 4 > 8 ? 8 : pairs / 4);
+  auto estimate = [&](int rows, int ks) {
+    const double ctas = (double)rows * p.TT * ks;
+    const double slots = (double)(p.DG == 1 ? resident_ctas<1>(ks, p.smem, sms) : resident_ctas<2>(ks, p.smem, sms));
+    if (slots <= 0) return 1e30;
+    const double waves = ctas <= slots ? 1.0 : (double)(long long)((ctas + slots - 1) / slots);
+    const double per_cta = (double)((pairs + ks - 1) / ks);
+    if (p.DG == 1) {
+      const double load = ctas < slots ? ctas : slots;
+      return waves * (per_cta * (0.45 + 0.0024 * load) * (1.0 + 0.0015 * (p.NT - 16)) + 3.0 + 0.3 * ks * p.NT / 64.0);
+    }
+    const double pair = 0.785 * p.NT / 304.0 > 0.5 ? 0.785 * p.NT / 304.0 : 0.5;
+    return waves * (per_cta * pair + 4.0 + 0.45 * ks * p.NT / 64.0);
+  };
+  auto best_split = [&](int rows, double& t) {
+    int best = 1;
+    t = 1e30;
+    for (int ks = 1; ks <= ksmax; ++ks) {
+      const double e = estimate(rows, ks);
+      if (e < t - 1e-9) { t = e; best = ks; }
+    }
+    return best;
+  };
+  double whole;
+  p.KS = best_split(p.RB, whole);
+  p.RB1 = 0;
+  p.KS1 = 1;
+  // One CTA per SM: a last wave that is nearly empty costs as much as a full one (192 row blocks at 300 tokens: 148 + 44).
+  // Then the full waves go out unsplit and the rest of the row blocks in a second launch with a split of its own.
+  if (p.DG == 2 && p.RB * p.TT > sms) {
+    const int rows1 = (int)((long long)p.RB * p.TT / sms * sms / p.TT);
+    double rest;
+    if (rows1 > 0 && rows1 < p.RB) {
+      const int ks2 = best_split(p.RB - rows1, rest);
+      if (estimate(rows1, 1) + rest + 1.0 < whole) { p.RB1 = rows1; p.KS1 = 1; p.KS = ks2; }
+    }
   }
-  p.KS = best;
   return p;
 }
 
-template <bool GROUPED>
+template <int DG, bool GROUPED>
 int gemm_launch(const GemmPlan& p, const GemmArgs& a, const CUtensorMap& xmap, const WMaps& wmaps, cudaStream_t stream) {
-  if (int e = gemm_attr<GROUPED>()) return e;
+  if (int e = gemm_attr<DG, GROUPED>()) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.RB * p.TT * p.KS));
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(gemm_threads<DG>());
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -520,16 +639,39 @@ int gemm_launch(const GemmPlan& p, const GemmArgs& a, const CUtensorMap& xmap, c
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = st::pdl_enabled() ? 2 : 1;
-  return st::cuda_fail(cudaLaunchKernelEx(&cfg, gemm_kernel<GROUPED>, a, xmap, wmaps), GROUPED ? "st_moe_group_gemm launch" : "st_gemm launch");
+  return st::cuda_fail(cudaLaunchKernelEx(&cfg, gemm_kernel<DG, GROUPED>, a, xmap, wmaps),
+                       GROUPED ? "st_moe_group_gemm launch" : "st_gemm launch");
+}
+void plan_args(GemmArgs& a, const GemmPlan& p) {
+  a.NT = p.NT; a.KS = p.KS; a.RB = p.RB; a.TT = p.TT;
+  a.astages = p.astages; a.xstages = p.xstages; a.rstages = p.rstages; a.bar_off = p.bar_off; a.tmem_cols = p.tmem_cols;
 }
 
-// activations [rows, N] BF16 as 64-column x NT-row boxes with the 128-byte swizzle
-int make_xmap(CUtensorMap* map, const void* X, long long rows, long long N, int NT, const char* who) {
+int dense_launch(const GemmPlan& plan, GemmArgs& a, const CUtensorMap& xmap, const WMaps& wmaps, cudaStream_t stream) {
+  GemmPlan p = plan;
+  auto go = [&] {
+    plan_args(a, p);
+    return p.DG == 1 ? gemm_launch<1, false>(p, a, xmap, wmaps, stream) : gemm_launch<2, false>(p, a, xmap, wmaps, stream);
+  };
+  a.rb0 = 0;
+  if (plan.RB1 > 0) {
+    p.RB = plan.RB1;
+    p.KS = plan.KS1;
+    if (int e = go()) return e;
+    p.RB = plan.RB - plan.RB1;
+    p.KS = plan.KS;
+    a.rb0 = plan.RB1;
+  }
+  return go();
+}
+
+// activations [rows, N] BF16 as boxes of 64 columns x `box_rows` rows with the 128-byte swizzle
+int make_xmap(CUtensorMap* map, const void* X, long long rows, long long N, int box_rows, const char* who) {
   EncodeTiledFn enc = encode_fn();
   ST_REQUIRE(enc != nullptr, "%s: cuTensorMapEncodeTiled is not available from the driver", who);
   const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)N * 2};
-  const cuuint32_t box[2] = {64u, (cuuint32_t)NT};
+  const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1u, 1u};
   const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -538,13 +680,13 @@ int make_xmap(CUtensorMap* map, const void* X, long long rows, long long N, int 
   return 0;
 }
 
-// a tree [M/16][N/64][1552 B] as 194 x u64 rows, boxes of eight row tiles of one column group
+// a tree [M/16][N/64][1552 B] as 194 x u64 rows, boxes of eight row tiles of two column groups
 int make_wmap(CUtensorMap* map, const void* tree, long long M, long long N, const char* who) {
   EncodeTiledFn enc = encode_fn();
   ST_REQUIRE(enc != nullptr, "%s: cuTensorMapEncodeTiled is not available from the driver", who);
   const cuuint64_t wd[3] = {194u, (cuuint64_t)(N / 64), (cuuint64_t)(M / 16)};
   const cuuint64_t wst[2] = {(cuuint64_t)REC, (cuuint64_t)(N / 64) * REC};
-  const cuuint32_t wbox[3] = {194u, 1u, 8u};
+  const cuuint32_t wbox[3] = {194u, (cuuint32_t)PAIR, 8u};
   const cuuint32_t we[3] = {1u, 1u, 1u};
   const CUresult wr = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void*>(tree), wd, wst, wbox, we,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -553,8 +695,6 @@ int make_wmap(CUtensorMap* map, const void* tree, long long M, long long N, cons
   return 0;
 }
 
-// instruction descriptor: D fp32, A and B bf16, both K-major, N = NT, M = 128
-uint32_t mma_idesc(int NT) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24); }
 }  // namespace
 
 extern "C" int64_t st_gemm_workspace_bytes(int64_t M, int64_t N, int64_t B) {
@@ -575,16 +715,15 @@ extern "C" int st_gemm(const void* tree, const int32_t* eo, const uint32_t* el, 
   CUtensorMap xmap;
   WMaps wmaps;
   memset(&wmaps, 0, sizeof(wmaps));
-  if (int e = make_xmap(&xmap, X, B, N, p.NT, "st_gemm")) return e;
+  if (int e = make_xmap(&xmap, X, B, N, p.NT > 256 ? p.NT / 2 : p.NT, "st_gemm")) return e;
   if (int e = make_wmap(&wmaps.m[0], tree, M, N, "st_gemm")) return e;
   GemmArgs a = {};
   a.tree = (const uint8_t*)tree; a.eo = eo; a.el = el; a.Y = (uint16_t*)Y; a.Yf = Yf32;
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "st_gemm: no device status word");
-  a.M = M; a.N = N; a.B = (int)B; a.NG = (int)(N / 64); a.NT = p.NT; a.KS = p.KS; a.RB = p.RB; a.TT = p.TT;
-  a.stages = p.stages; a.rstages = p.rstages; a.nmma = p.nmma; a.bar_off = p.bar_off;
-  a.idesc = mma_idesc(p.NT);
-  return gemm_launch<false>(p, a, xmap, wmaps, (cudaStream_t)stream);
+  a.M = M; a.N = N; a.B = (int)B; a.NG = (int)(N / 64);
+  plan_args(a, p);
+  return dense_launch(p, a, xmap, wmaps, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------------------------- list of matrices
@@ -614,14 +753,13 @@ extern "C" int st_gemm_list(int64_t n, const void* const* trees, const int32_t* 
   const GemmPlan p = gemm_plan(total, N, B);
   ST_REQUIRE((long long)p.RB * p.TT * p.KS < (1ll << 31), "%s: grid too large", who);
   CUtensorMap xmap;
-  if (int e = make_xmap(&xmap, X, B, N, p.NT, who)) return e;
+  if (int e = make_xmap(&xmap, X, B, N, p.NT > 256 ? p.NT / 2 : p.NT, who)) return e;
   a.eo = eo[0]; a.el = el[0]; a.Y = (uint16_t*)Y[0];
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "%s: no device status word", who);
-  a.M = total; a.N = N; a.B = (int)B; a.NG = (int)(N / 64); a.NT = p.NT; a.KS = p.KS; a.RB = p.RB; a.TT = p.TT;
-  a.stages = p.stages; a.rstages = p.rstages; a.nmma = p.nmma; a.bar_off = p.bar_off;
-  a.idesc = mma_idesc(p.NT);
-  return gemm_launch<false>(p, a, xmap, wmaps, (cudaStream_t)stream);
+  a.M = total; a.N = N; a.B = (int)B; a.NG = (int)(N / 64);
+  plan_args(a, p);
+  return dense_launch(p, a, xmap, wmaps, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------------------------- grouped (MoE)
@@ -661,7 +799,7 @@ extern "C" int st_moe_group_gemm(const void* maps, const int64_t* eop, const int
   ST_REQUIRE((long long)p.RB * p.TT < (1ll << 31), "st_moe_group_gemm: grid too large");
   CUtensorMap xmap;
   WMaps unused;
-  if (int e = make_xmap(&xmap, Xg, nblk * bs, N, p.NT, "st_moe_group_gemm")) return e;
+  if (int e = make_xmap(&xmap, Xg, nblk * bs, N, XBOX_GROUPED, "st_moe_group_gemm")) return e;
   memset(&unused, 0, sizeof(unused));
   GemmArgs a = {};
   a.Y = (uint16_t*)Y; a.Yf = Yf32;
@@ -669,8 +807,7 @@ extern "C" int st_moe_group_gemm(const void* maps, const int64_t* eop, const int
   a.sorted = sorted; a.bexp = bexp; a.npost = npost; a.E = (int)E;
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "st_moe_group_gemm: no device status word");
-  a.M = M; a.N = N; a.B = (int)S; a.NG = (int)(N / 64); a.NT = p.NT; a.KS = 1; a.RB = p.RB; a.TT = p.TT;
-  a.stages = p.stages; a.rstages = p.rstages; a.nmma = p.nmma; a.bar_off = p.bar_off;
-  a.idesc = mma_idesc(p.NT);
-  return gemm_launch<true>(p, a, xmap, unused, (cudaStream_t)stream);
+  a.M = M; a.N = N; a.B = (int)S; a.NG = (int)(N / 64);
+  plan_args(a, p);
+  return gemm_launch<1, true>(p, a, xmap, unused, (cudaStream_t)stream);
 }

@@ -102,6 +102,20 @@ def test_gemm_matches_fp64(M, N, regime, monkeypatch):
     _status_ok()
 
 
+@pytest.mark.parametrize("M,N,regime", [(384, 2048, "mixed"), (128, 320, "heavy")])
+def test_gemm_token_tile_edges(M, N, regime, monkeypatch):
+    """batches at the edges of the token tiling: one MMA step (16), the widest tile of the two-CTAs-per-SM form (128), the
+    first of the one-CTA form, one MMA / two halves (256 / 257), the widest tile (320) and the first split into two"""
+    import statetree_b200.linear as L
+    monkeypatch.setattr(L, "PREFILL_MIN", 0)
+    monkeypatch.setattr(L, "GEMV_MAX", 0)
+    tl, _ = layer_from_oracle(G.weights(M, N, 3 * M + N, regime))
+    W = G.weights(M, N, 3 * M + N, regime)
+    for B in (1, 15, 16, 17, 112, 113, 128, 129, 144, 256, 257, 288, 320, 321, 641):
+        _check_linear(tl, W, B, B, "gemm")
+    _status_ok()
+
+
 @pytest.mark.parametrize("Ms,N,regime", [((256, 64, 64), 1024, "mixed"), ((512, 128), 512, "heavy"),
                                          ((16, 16, 16, 16), 64, "mixed"), ((1024, 256, 256), 4096, "llm"),
                                          ((768, 768), 2048, "each")])
