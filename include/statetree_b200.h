@@ -46,6 +46,19 @@ int st_dec(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, i
 int st_rows(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, int64_t N, const int64_t* ids,
             int64_t n, void* out, void* stream);
 
+/* BF16 matrix W [M, N] -> state tree (statetree/format.py:43-83 does this with PyTorch operations), in two passes with the
+ * caller's prefix sums between them:
+ *   st_encode        the records; rowcnt uint8 [M, N/64] = escapes of each row's 64 values; reccnt int32 [M/16 * N/64 + 1] =
+ *                    0, then the escapes of each record (its inclusive prefix sum is eo)
+ *   st_encode_lists  given eo and roff int32 [M, N/64] (inclusive prefix sum of rowcnt, row-major): el and eb as above and the
+ *                    format's lists rows / cols int32, bits int16 in (row, col) order; n = eo[last] entries each
+ * st_dec_check decodes the tree and adds to *bad (int32, zeroed by the caller) for every record that differs from W. */
+int st_encode(const void* W, int64_t M, int64_t N, void* tree, uint8_t* rowcnt, int32_t* reccnt, void* stream);
+int st_encode_lists(const void* W, int64_t M, int64_t N, const uint8_t* rowcnt, const int32_t* roff, const int32_t* eo,
+                    uint32_t* el, uint32_t* eb, int32_t* rows, int32_t* cols, int16_t* bits, void* stream);
+int st_dec_check(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, int64_t N, const void* W, int32_t* bad,
+                 void* stream);
+
 /* Small-batch fused decode + GEMV, 1 <= B <= 32.  Replaces the reference's mv / mvs / mvh / mvc / mvt entry points
  * (statetree/csrc/kernels.cu:243-254, 370-400, 548-599, 771-808; statetree/csrc/hop.cu:993-1019).
  * ws: workspace of st_gemv_workspace_bytes() bytes whose 32-bit words all hold 0xFFFFFFFF on entry and are left so

@@ -76,6 +76,8 @@ def encode(W, chunk_rows=4096):
     assert W.dim() == 2 and W.dtype == torch.bfloat16, "encode expects a 2-D bf16 matrix"
     M, N = W.shape
     assert M % 16 == 0 and N % 64 == 0, f"shape {tuple(W.shape)}: rows must be a multiple of 16, cols of 64"
+    if W.is_cuda and M > 0 and N > 0:
+        return encode_with_tables(W)[0]
     chunk_rows = max(16, chunk_rows // 16 * 16)
     tree = torch.empty(M // 16, N // 64, RECORD_BYTES, dtype=torch.uint8, device=W.device)
     rows, cols, bits = [], [], []
@@ -87,6 +89,17 @@ def encode(W, chunk_rows=4096):
         cols.append(ec.to(torch.int32))
         bits.append(eb)
     return dict(tree=tree, esc_rows=torch.cat(rows), esc_cols=torch.cat(cols), esc_bits=torch.cat(bits))
+
+
+@torch.no_grad()
+def encode_with_tables(W):
+    """encode() of a matrix on a GPU by the kernels of the library, with the side tables escape_tables() would build:
+    (the dict encode() returns, (eo, el, eb))"""
+    from .ops import ext
+    if W.data_ptr() % 16 or not W.is_contiguous():
+        W = W.clone(memory_format=torch.contiguous_format)
+    tree, rows, cols, bits, tables = ext().encode(W)
+    return dict(tree=tree, esc_rows=rows, esc_cols=cols, esc_bits=bits), tables
 
 
 @torch.no_grad()

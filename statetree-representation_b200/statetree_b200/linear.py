@@ -232,17 +232,26 @@ class TreeLinear(nn.Module):
             escapes = F.escape_count(W)
             if escapes > max_escape_fraction * W.numel():
                 raise EscapeHeavy(f"{escapes / W.numel():.2%} of the weights escape")
-        enc = F.encode(W)
         out_features, in_features = W.shape
+        on_gpu = W.is_cuda and W.dim() == 2 and W.numel() > 0 and out_features % 16 == 0 and in_features % 64 == 0
+        enc, tables = F.encode_with_tables(W) if on_gpu else (F.encode(W), None)
         layer = cls(in_features, out_features, bias=bias is not None, device="meta", n_esc=int(enc["esc_rows"].numel()))
         layer._buffers.update({name: enc[name] for name in _BUFFERS})
         if bias is not None:
             layer._buffers["bias"] = bias.detach().to(device=W.device, dtype=torch.bfloat16).clone()
         layer._reset_runtime()
         if verify:
-            back = layer.dequantize() if layer.tree.is_cuda else F.decode_reference(*(layer._buffers[n] for n in _BUFFERS))
-            if not torch.equal(back.view(torch.int16), W.view(torch.int16)):
+            if on_gpu:
+                same = ext().dec_check(enc["tree"], tables[0], tables[1],
+                                       W if W.data_ptr() % 16 == 0 and W.is_contiguous() else W.clone(memory_format=torch.contiguous_format))
+            else:
+                back = F.decode_reference(*(layer._buffers[n] for n in _BUFFERS))
+                same = torch.equal(back.view(torch.int16), W.view(torch.int16))
+            if not same:
                 raise RuntimeError("TreeLinear: the tree does not decode to the weights it was built from")
+        if on_gpu:                                      # (see tables(): complete before any later kernel may start)
+            torch.cuda.current_stream(W.device).synchronize()
+            layer._tables = tables
         return layer
 
     def _load_from_state_dict(self, state_dict, prefix, local_metadata, strict, missing_keys, unexpected_keys,

@@ -23,6 +23,9 @@ _SIGNATURES = {
     "st_device_status": (_int, []),
     "st_dec": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp]),
     "st_rows": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _i64, _vp, _vp]),
+    "st_encode": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
+    "st_encode_lists": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "st_dec_check": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
     "st_gemv_workspace_bytes": (_i64, [_i64, _i64, _i64]),
     "st_gemv": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp]),
     "st_gemv_static": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
@@ -132,6 +135,38 @@ class _Weights:
         M, N = W.shape
         with _ctx(T):
             _check(lib().st_dec(_ptr(T), _ptr(EO), _ptr(EL), M, N, _ptr(W), _stream(T)))
+
+    @staticmethod
+    def encode(W):
+        """W [M, N] BF16 on a GPU -> (tree, rows, cols, bits, (eo, el, eb)): the format's parts and the kernels' side tables"""
+        M, N = W.shape
+        dev, nrec = W.device, (M // 16) * (N // 64)
+        tree = torch.empty(M // 16, N // 64, 1552, dtype=torch.uint8, device=dev)
+        rowcnt = torch.empty(M * (N // 64), dtype=torch.uint8, device=dev)
+        reccnt = torch.empty(nrec + 1, dtype=torch.int32, device=dev)
+        with _ctx(W):
+            _check(lib().st_encode(_ptr(W), M, N, _ptr(tree), _ptr(rowcnt), _ptr(reccnt), _stream(W)))
+            eo = reccnt.cumsum(0, dtype=torch.int32)
+            roff = rowcnt.cumsum(0, dtype=torch.int32)
+            n = int(eo[-1])                              # (synchronises: the lists' length depends on the data)
+            rows, cols = (torch.empty(n, dtype=torch.int32, device=dev) for _ in range(2))
+            bits = torch.empty(n, dtype=torch.int16, device=dev)
+            el = torch.empty(n, dtype=torch.int32, device=dev) if n else torch.zeros(1, dtype=torch.int32, device=dev)
+            eb = torch.empty((M // 16) * ((N // 64 + 7) // 8), 16, dtype=torch.int32, device=dev)
+            spare = el                                   # (no escapes: empty tensors have no address; nothing is written)
+            _check(lib().st_encode_lists(_ptr(W), M, N, _ptr(rowcnt), _ptr(roff), _ptr(eo), _ptr(el), _ptr(eb),
+                                         _ptr(rows if n else spare), _ptr(cols if n else spare), _ptr(bits if n else spare),
+                                         _stream(W)))
+        return tree, rows, cols, bits, (eo, el, eb)
+
+    @staticmethod
+    def dec_check(T, EO, EL, W):
+        """does the tree decode to W [M, N] BF16 exactly (synchronises)"""
+        M, N = W.shape
+        bad = torch.zeros(1, dtype=torch.int32, device=W.device)
+        with _ctx(T):
+            _check(lib().st_dec_check(_ptr(T), _ptr(EO), _ptr(EL), M, N, _ptr(W), _ptr(bad), _stream(T)))
+            return int(bad) == 0
 
     @staticmethod
     def rows(T, EO, EL, ids, out):

@@ -420,3 +420,37 @@ def test_layer_prepare_then_graph_capture():
         torch.cuda.synchronize()
         assert torch.equal(y, tl(x)), B
     _status_ok()
+
+
+@pytest.mark.parametrize("M,N,regime", [(16, 64, "mixed"), (48, 576, "heavy"), (256, 512, "each"), (512, 1088, "mixed"),
+                                        (1024, 4096, "llm"), (32, 128, "zero"), (64, 1024, "special")])
+def test_encode_kernels_equal_the_torch_formulation(M, N, regime):
+    """records, lists in (row, col) order and the three side tables, byte for byte against format's torch code (the CPU
+    path); tiles whose last unit is short, matrices without escapes, rows of zeros, infinities and NaN, unaligned and
+    strided inputs; the check kernel tells a changed value"""
+    from statetree_b200 import TreeLinear, format as F, ops
+    if regime == "zero":
+        W = torch.zeros(M, N, dtype=torch.bfloat16)
+    elif regime == "special":
+        W = torch.randint(-32768, 32768, (M, N), dtype=torch.int16, generator=torch.Generator().manual_seed(3)).view(torch.bfloat16)
+    else:
+        W = bits_to_torch(G.weights(M, N, M + 2 * N, regime), "cpu")
+    want = F.encode(W)
+    tabs = F.escape_tables(M, N, want["esc_rows"], want["esc_cols"], want["esc_bits"])
+    big = torch.zeros(M, N + 3, dtype=torch.bfloat16, device=DEV)
+    big[:, 3:] = W.to(DEV)
+    for src in (W.to(DEV), big[:, 3:]):
+        got, gtabs = F.encode_with_tables(src)
+        for k in want:
+            assert got[k].dtype == want[k].dtype and torch.equal(got[k].cpu(), want[k]), (k, regime)
+        for a, b, name in zip(gtabs, tabs, ("eo", "el", "eb")):
+            assert a.dtype == b.dtype and torch.equal(a.cpu(), b), (name, regime)
+    eo, el, _ = gtabs
+    Wd = W.to(DEV)
+    assert ops.ext().dec_check(got["tree"], eo, el, Wd)
+    bits = Wd.view(torch.int16)
+    bits[M - 1, N - 1] ^= 1
+    assert not ops.ext().dec_check(got["tree"], eo, el, Wd)
+    bits[M - 1, N - 1] ^= 1
+    layer = TreeLinear.from_weight(Wd)
+    assert torch.equal(layer.dequantize().view(torch.int16), bits)
