@@ -425,12 +425,9 @@ __device__ __forceinline__ void put_exact(uint32_t (&R)[4][4], uint32_t entry, i
   }
 }
 
-// one 1600-byte unit in shared memory -> the lane's fragment registers, escapes (in-record slots, then the pool chain)
-// applied
-__device__ __forceinline__ void unit_to_frag(const uint8_t* unit, const uint32_t* pool, int pool_blocks, int lane,
-                                             uint32_t (&R)[4][4]) {
-  decode_frag(load_rec_shared(unit, lane), R);
-  const uint32_t head = *reinterpret_cast<const uint32_t*>(unit + REC);
+// exact values of a unit's escapes (in-record slots, then the pool chain) put into its decoded fragments
+__device__ __forceinline__ void unit_escapes(const uint8_t* unit, uint32_t head, const uint32_t* pool, int pool_blocks,
+                                             int lane, uint32_t (&R)[4][4]) {
   if ((head & 31u) == 0u) return;
   const uint32_t* slot = reinterpret_cast<const uint32_t*>(unit + REC + 4);
   const int used = min((int)(head & 15u), NSLOT);
@@ -445,6 +442,18 @@ __device__ __forceinline__ void unit_to_frag(const uint8_t* unit, const uint32_t
     }
   }
 }
+// the two units (dims 0..63, 64..127) of a page's keys or values in shared memory -> the lane's fragment registers.  Both
+// are decoded before the first escape is looked at: two independent chains instead of one
+__device__ __forceinline__ void units_to_frag(const uint8_t* unit, const uint32_t* pool, int pool_blocks, int lane,
+                                              uint32_t (&R)[2][4][4]) {
+  const uint32_t h0 = *reinterpret_cast<const uint32_t*>(unit + REC), h1 = *reinterpret_cast<const uint32_t*>(unit + RKV + REC);
+  const RecRegs r0 = load_rec_shared(unit, lane), r1 = load_rec_shared(unit + RKV, lane);
+  decode_frag(r0, R[0]);
+  decode_frag(r1, R[1]);
+  if (((h0 | h1) & 31u) == 0u) return;
+  unit_escapes(unit, h0, pool, pool_blocks, lane, R[0]);
+  unit_escapes(unit + RKV, h1, pool, pool_blocks, lane, R[1]);
+}
 
 __device__ __forceinline__ float max_over_rows(float v) {        // lanes that differ in g (bits 2..4) hold other tokens
   v = fmaxf(v, __shfl_xor_sync(FULL, v, 4));
@@ -458,16 +467,34 @@ __device__ __forceinline__ float sum_over_rows(float v) {
 }
 
 template <int NW, int STG>
-__global__ void __launch_bounds__(NW * 32) kv_attn_kernel(const AttnLaunch a) {
+__global__ void __launch_bounds__(NW * 32, 16 / NW) kv_attn_kernel(const AttnLaunch a) {
   extern __shared__ __align__(128) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)NW * STG * PAGE_BYTES);      // [NW][STG]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int G = a.group, Hq = a.kv_heads * G;
   const int split = blockIdx.x % a.splits, bh = blockIdx.x / a.splits;
   const int kvh = bh % a.kv_heads, seq = bh / a.kv_heads;
-  pdl_wait();                               // queries, lengths and this step's pages come from earlier kernels
+  uint8_t* ring = smem + (size_t)warp * STG * PAGE_BYTES;
+  uint64_t* bar = bars + warp * STG;
+  if (lane == 0) {
+    for (int s = 0; s < STG; ++s) mbar_init(bar + s, 1);
+    fence_barrier_init();
+  }
+  const uint64_t stream_policy = policy_evict_first();
   pdl_launch_dependents();
+  pdl_wait();                               // queries, lengths and this step's pages come from earlier kernels
 
+  // ---- Q^T as the B operand: lane (g, t) holds head g, dims 16 ks + 2t, +1 and 16 ks + 8 + 2t, +1 (requested first: the
+  // loads run beside the chain length -> block table -> page)
+  uint32_t qf[8][2];
+  {
+    const uint16_t* qrow = a.q + (size_t)seq * a.q_stride + (size_t)(kvh * G + (g < G ? g : 0)) * HD;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      qf[ks][0] = *reinterpret_cast<const uint32_t*>(qrow + 16 * ks + 2 * t);
+      qf[ks][1] = *reinterpret_cast<const uint32_t*>(qrow + 16 * ks + 8 + 2 * t);
+    }
+  }
   // ---- this warp's pages
   const int len = a.seq_len[seq], start = a.seq_start ? a.seq_start[seq] : 0;
   const int first_page = start / PAGE;
@@ -477,36 +504,28 @@ __global__ void __launch_bounds__(NW * 32) kv_attn_kernel(const AttnLaunch a) {
   const int my_first = lo_page + warp;
   const int my_count = hi_page > my_first ? (hi_page - my_first + NW - 1) / NW : 0;
 
-  uint8_t* ring = smem + (size_t)warp * STG * PAGE_BYTES;
-  uint64_t* bar = bars + warp * STG;
-  if (lane == 0) {
-    for (int s = 0; s < STG; ++s) mbar_init(bar + s, 1);
-    fence_barrier_init();
-  }
   __syncwarp();
-  const uint64_t stream_policy = policy_evict_first();
-  auto fetch = [&](int i) {                        // lane 0: this warp's i-th page -> stage i % STG
-    long long blk = a.table[(size_t)seq * a.table_stride + my_first + i * NW];
+  // Block-table entries of this warp's pages come 32 at a time, one per lane, so that no table lookup (a trip to L2) sits
+  // in front of a page's copy: lane l holds the entry of page (i & ~31) + l
+  const int* const my_table = a.table + (size_t)seq * a.table_stride + my_first;
+  int entries = 0;
+  auto fetch = [&](int i) {                        // this warp's i-th page -> stage i % STG (called by the whole warp, i in order)
+    if ((i & 31) == 0) entries = i + lane < my_count ? __ldg(my_table + (i + lane) * NW) : 0;
+    long long blk = __shfl_sync(FULL, entries, i & 31);
     blk = blk < 0 ? 0 : (blk >= a.n_pages ? a.n_pages - 1 : blk);
     const int s = i % STG;
-    mbar_expect_tx(bar + s, PAGE_BYTES);
-    bulk_g2s(ring + (size_t)s * PAGE_BYTES, a.pages + ((size_t)blk * a.kv_heads + kvh) * PAGE_BYTES, PAGE_BYTES, bar + s,
-             stream_policy);
-  };
-  if (lane == 0)
-    for (int i = 0; i < min(my_count, STG); ++i) fetch(i);
-
-  // ---- Q^T as the B operand: lane (g, t) holds head g, dims 16 ks + 2t, +1 and 16 ks + 8 + 2t, +1
-  uint32_t qf[8][2];
-  {
-    const uint16_t* qrow = a.q + (size_t)seq * a.q_stride + (size_t)(kvh * G + (g < G ? g : 0)) * HD;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      const uint32_t v0 = *reinterpret_cast<const uint32_t*>(qrow + 16 * ks + 2 * t);
-      const uint32_t v1 = *reinterpret_cast<const uint32_t*>(qrow + 16 * ks + 8 + 2 * t);
-      qf[ks][0] = g < G ? v0 : 0u;
-      qf[ks][1] = g < G ? v1 : 0u;
+    if (elect_one()) {
+      mbar_expect_tx(bar + s, PAGE_BYTES);
+      bulk_g2s(ring + (size_t)s * PAGE_BYTES, a.pages + ((size_t)blk * a.kv_heads + kvh) * PAGE_BYTES, PAGE_BYTES, bar + s,
+               stream_policy);
     }
+  };
+  for (int i = 0; i < min(my_count, STG); ++i) fetch(i);
+
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {                 // columns beyond the group's heads are zero
+    qf[ks][0] = g < G ? qf[ks][0] : 0u;
+    qf[ks][1] = g < G ? qf[ks][1] : 0u;
   }
   // ---- running state.  This lane's score columns are heads 2t and 2t + 1; heads beyond G never take part: their
   // scores are masked to -inf and their reference maximum stays 0, so their probabilities are exactly 0
@@ -529,12 +548,17 @@ __global__ void __launch_bounds__(NW * 32) kv_attn_kernel(const AttnLaunch a) {
     const uint8_t* pg = ring + (size_t)s * PAGE_BYTES;
     // ---- S^T = K Q^T
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
+    {
+      uint32_t R[2][4][4];
+      float sd[4] = {0.f, 0.f, 0.f, 0.f};          // a second accumulator halves the chain of dependent MMAs
+      units_to_frag(pg, a.pool, a.pool_blocks, lane, R);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t R[4][4];
-      unit_to_frag(pg + half * RKV, a.pool, a.pool_blocks, lane, R);
+      for (int ks = 0; ks < 4; ++ks) {
+        mma_bf16(sc, R[0][ks], qf[ks][0], qf[ks][1]);
+        mma_bf16(sd, R[1][ks], qf[4 + ks][0], qf[4 + ks][1]);
+      }
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) mma_bf16(sc, R[ks], qf[half * 4 + ks][0], qf[half * 4 + ks][1]);
+      for (int q = 0; q < 4; ++q) sc[q] += sd[q];
     }
     // this lane: tokens g and g + 8 of the page; valid tokens of the sequence are [start, len)
     const int tok = page * PAGE + g;
@@ -566,21 +590,22 @@ __global__ void __launch_bounds__(NW * 32) kv_attn_kernel(const AttnLaunch a) {
     const uint32_t rb0 = movmatrix_t(pack_bf16(p00 - r_lo.x, p01 - r_lo.y));
     const uint32_t rb1 = movmatrix_t(pack_bf16(p10 - r_hi.x, p11 - r_hi.y));
     // ---- O^T += V^T P^T
+    {
+      uint32_t R[2][4][4];
+      units_to_frag(pg + 2 * RKV, a.pool, a.pool_blocks, lane, R);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t R[4][4];
-      unit_to_frag(pg + (2 + half) * RKV, a.pool, a.pool_blocks, lane, R);
+      for (int half = 0; half < 2; ++half)
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        // 8 x 8 blocks of the record (tokens x dims) transposed: rows become dims, the k index becomes tokens
-        const uint32_t a0 = movmatrix_t(R[ks][0]), a1 = movmatrix_t(R[ks][2]);
-        const uint32_t a2 = movmatrix_t(R[ks][1]), a3 = movmatrix_t(R[ks][3]);
-        mma_bf16_r(acc[half * 4 + ks], a0, a1, a2, a3, pb0, pb1);
-        mma_bf16_r(acc[half * 4 + ks], a0, a1, a2, a3, rb0, rb1);
-      }
+        for (int ks = 0; ks < 4; ++ks) {
+          // 8 x 8 blocks of the record (tokens x dims) transposed: rows become dims, the k index becomes tokens
+          const uint32_t a0 = movmatrix_t(R[half][ks][0]), a1 = movmatrix_t(R[half][ks][2]);
+          const uint32_t a2 = movmatrix_t(R[half][ks][1]), a3 = movmatrix_t(R[half][ks][3]);
+          mma_bf16_r(acc[half * 4 + ks], a0, a1, a2, a3, pb0, pb1);
+          mma_bf16_r(acc[half * 4 + ks], a0, a1, a2, a3, rb0, rb1);
+        }
     }
     __syncwarp();                                  // every lane has read this stage
-    if (lane == 0 && i + STG < my_count) {
+    if (i + STG < my_count) {
       fence_proxy_async();
       fetch(i + STG);
     }
@@ -631,29 +656,54 @@ __global__ void __launch_bounds__(NW * 32) kv_attn_kernel(const AttnLaunch a) {
   }
 }
 
-// One warp per (sequence, query head): weighs the split partials by exp2(m_j - max m) and normalises.
-__global__ void __launch_bounds__(128) kv_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                       uint16_t* __restrict__ out, long long out_stride, int Hq,
-                                                       int splits, long long rows) {
+// One CTA of four warps per (sequence, query head): weighs the split partials by exp2(m_j - max m) and normalises.  Latency
+// bounds it (a few KB per row), so nothing is loaded inside a dependent loop: lane j of every warp takes (m, l) of split j,
+// and warp w has the partials of its splits w, w + 4, ... (eight at a time) in flight together.  32 rows x 32 splits:
+// 2 us behind the attention kernel; one warp per row walking the splits one after the other took 9 us.
+constexpr int MERGE_WARPS = 4;
+__global__ void __launch_bounds__(MERGE_WARPS * 32) kv_merge_kernel(const float* __restrict__ part_o,
+                                                                    const float* __restrict__ part_ml,
+                                                                    uint16_t* __restrict__ out, long long out_stride, int Hq,
+                                                                    int splits) {
+  __shared__ float4 s_num[MERGE_WARPS][32];
   pdl_wait();
   pdl_launch_dependents();
-  const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const float* ml = part_ml + (size_t)row * splits * 2;
+  const long long row = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* ml = part_ml + row * splits * 2;
+  const float4* po = reinterpret_cast<const float4*>(part_o) + row * splits * (HD / 4) + lane;
   float top = -INFINITY;
   for (int j = lane; j < splits; j += 32) top = fmaxf(top, ml[2 * j]);
 #pragma unroll
   for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
   float den = 0.f;
   float4 num = make_float4(0.f, 0.f, 0.f, 0.f);    // this lane's four dims
-  for (int j = 0; j < splits; ++j) {
-    const float mj = ml[2 * j];
-    if (mj == -INFINITY) continue;                  // a split without tokens
-    const float f = exp2f(mj - top);
-    den += f * ml[2 * j + 1];
-    const float4 o = *reinterpret_cast<const float4*>(part_o + ((size_t)row * splits + j) * HD + 4 * lane);
-    num.x += f * o.x; num.y += f * o.y; num.z += f * o.z; num.w += f * o.w;
+  for (int c = 0; c < splits; c += 32) {
+    float m = -INFINITY, l = 0.f;
+    if (c + lane < splits) { m = ml[2 * (c + lane)]; l = ml[2 * (c + lane) + 1]; }
+    const float f = m == -INFINITY ? 0.f : exp2f(m - top);           // (a split without tokens weighs nothing)
+    den += f * l;
+    float4 o[32 / MERGE_WARPS];
+#pragma unroll
+    for (int k = 0; k < 32 / MERGE_WARPS; ++k) {
+      const int j = c + warp + MERGE_WARPS * k;
+      o[k] = j < splits ? po[(size_t)j * (HD / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < 32 / MERGE_WARPS; ++k) {
+      const float fj = __shfl_sync(FULL, f, warp + MERGE_WARPS * k);
+      num.x += fj * o[k].x; num.y += fj * o[k].y; num.z += fj * o[k].z; num.w += fj * o[k].w;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) den += __shfl_xor_sync(FULL, den, o);
+  s_num[warp][lane] = num;
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int w = 1; w < MERGE_WARPS; ++w) {           // the warps in order: one fixed summation order
+    const float4 o = s_num[w][lane];
+    num.x += o.x; num.y += o.y; num.z += o.z; num.w += o.w;
   }
   const float inv = den > 0.f ? 1.f / den : 0.f;
   uint2 packed;
@@ -770,12 +820,15 @@ extern "C" int st_kv_attn(const void* q, int64_t qs, int64_t B, int64_t Hq, cons
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "st_kv_attn: no device status word");
   cudaStream_t st_ = (cudaStream_t)stream;
-  // four warps with two pages in flight each (51 KB): several CTAs share an SM and hide each other's latencies
-  if (int e = attn_launch<4, 2>(a, (int)B, st_)) return e;
-  if (S > 1) {
-    const long long rows = B * Hq;
-    return st::launch("st_kv_attn merge launch", kv_merge_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, st_,
-                      (const float*)wo, (const float*)wml, (uint16_t*)out, (long long)os, (int)Hq, (int)S, rows);
-  }
+  // Warps per CTA (two pages in flight each).  An SM holds sixteen warps' rings: four CTAs of four warps, or two of eight.
+  // A grid of at most two CTAs per SM leaves half of that idle with four warps, so its CTAs get eight (us per call with 4 / 8
+  // warps, 8 KV heads: 1 x 1K 7.8 / 7.0, 1 x 4K 11.6 / 10.1, 1 x 16K 20.0 / 18.0; sixteen: 7.5, 9.9, 22.3).  Larger grids keep
+  // four: more CTAs hide each other's latencies (4 x 4K 17.0 / 19.4, 16 x 4K 26.0 / 31.1; only long ragged batches, 32 x 4K
+  // 75 / 68, would gain, but the lengths are not known here).
+  const int e = B * Hkv * S <= 2ll * st::sm_count() ? attn_launch<8, 2>(a, (int)B, st_) : attn_launch<4, 2>(a, (int)B, st_);
+  if (e) return e;
+  if (S > 1)
+    return st::launch("st_kv_attn merge launch", kv_merge_kernel, dim3((unsigned)(B * Hq)), dim3(MERGE_WARPS * 32), 0, st_,
+                      (const float*)wo, (const float*)wml, (uint16_t*)out, (long long)os, (int)Hq, (int)S);
   return 0;
 }

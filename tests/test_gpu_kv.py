@@ -379,3 +379,40 @@ def test_vllm_page_backend_data_path():
             assert torch.equal(got.view(torch.int16), Ks[b].view(torch.int16)), (rnd, b)
     assert used[0] > 0 and used[-1] < 1.7 * used[0], used                      # recycled chains, no leak
     assert sh.usage()[2] is False
+
+
+@pytest.mark.parametrize("B,heads,splits", [(1, 2, 1), (1, 8, 2), (2, 2, 5), (3, 14, 31), (1, 16, 32), (2, 4, 33), (1, 2, 64),
+                                            (1, 6, 70), (40, 8, 4), (80, 2, 2)])
+def test_attention_split_counts_and_both_cta_sizes(B, heads, splits):
+    """merge of 1 to 70 split partials (below, at and beyond the 32 of one pass; splits without tokens among them), grids of
+    up to two CTAs per SM (eight warps each) and above it (four warps), an empty sequence, sequences that start late"""
+    from statetree_b200.kvcache import PageStore
+    kvh, ctx = 2, 1500 if B < 10 else 200
+    pages = -(-ctx // 16)
+    g = torch.Generator(DEV).manual_seed(splits)
+    K = torch.randn(B * pages * 16, kvh, D, device=DEV, generator=g).to(torch.bfloat16)
+    V = torch.randn(B * pages * 16, kvh, D, device=DEV, generator=g).to(torch.bfloat16)
+    K[:, :, 7] *= 512                                                           # escapes in most records
+    store = PageStore(B * pages, kvh, DEV, pool_blocks=1 << 14)
+    store.append(K, V, torch.arange(B * pages * 16, device=DEV))
+    store.check()
+    table = torch.randperm(B * pages, device=DEV, generator=g).to(torch.int32).view(B, pages)
+    lens = torch.randint(1, ctx + 1, (B,), device=DEV, generator=g).to(torch.int32)
+    lens[0] = ctx
+    starts = (lens.float() * 0.3).to(torch.int32) * (torch.arange(B, device=DEV) % 2)
+    if B > 1:
+        lens[1] = starts[1] = 0                                                 # no tokens at all: zeros
+    q = torch.randn(B, heads, D, device=DEV, generator=g).to(torch.bfloat16) / 16
+    out = store.attention(q, table, lens, 1.0 / math.sqrt(D), splits, starts.to(torch.int32))
+    for b in range(B):
+        n0, n1 = int(starts[b]), int(lens[b])
+        if n1 == 0:
+            assert int((out[b] != 0).sum()) == 0
+            continue
+        k, v = (t.view(-1, 16, kvh, D)[table[b].long()].reshape(-1, kvh, D)[n0:n1].double() for t in (K, V))
+        s = torch.einsum("hgd,nhd->hgn", q[b].double().view(kvh, -1, D), k) / math.sqrt(D)
+        ref = torch.einsum("hgn,nhd->hgd", torch.softmax(s, -1), v).reshape(heads, D)
+        # BF16 result: half an ulp (2^-9 of a value at most) everywhere, fp32 sums below that
+        assert float((out[b].double() - ref).norm() / ref.norm()) < 2.0 ** -9 * 1.1, b
+    from statetree_b200 import ops
+    assert ops.device_status() == 0
