@@ -154,6 +154,7 @@ int st_moe_align(const void* ids, int ids64, int64_t S, int64_t E, int64_t used_
  *                       expert tree into maps_dev; trees_host is a HOST array of E device addresses.  Once per
  *                       expert set, outside graph capture.
  *   st_moe_gather       Xg[i, :] = X[sorted[i] / xdiv, :] for the used entries of sorted (rows = nblk * bs)
+ *   st_moe_silu_gather  Xg[i, :] = silu(gate) * up of row sorted[i] of gu [S, 2 I] = [gate | up], rounded as st_silu_mul
  *   st_moe_group_gemm   one CTA per (block of bs pairs, 128 rows of M): Y[sorted[i], :] = W[bexp[block]] Xg[i, :];
  *                       rows of padding entries and of blocks with a negative expert are not written; eop / elp as
  *                       for st_moe_gemv; M % 128 == 0, bs = 64 or 128.  Yf32 optional as for st_gemv. */
@@ -161,6 +162,8 @@ int64_t st_moe_tensor_map_bytes(void);
 int st_moe_tensor_maps(const int64_t* trees_host, int64_t E, int64_t M, int64_t N, void* maps_dev, void* stream);
 int st_moe_gather(const void* X, const int32_t* sorted, const int32_t* npost, int64_t rows, int64_t S, int64_t xdiv,
                   int64_t N, void* Xg, void* stream);
+int st_moe_silu_gather(const void* gu, const int32_t* sorted, const int32_t* npost, int64_t rows, int64_t S, int64_t I,
+                       void* Xg, void* stream);
 int st_moe_group_gemm(const void* maps, const int64_t* eop, const int64_t* elp, int64_t E, const void* Xg,
                       const int32_t* sorted, const int32_t* bexp, const int32_t* npost, int64_t nblk, int64_t bs,
                       void* Y, float* Yf32, int64_t S, int64_t M, int64_t N, void* stream);

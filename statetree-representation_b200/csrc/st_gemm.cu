@@ -149,7 +149,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   constexpr int NDW = DG * NDEC;                                              // decode warps
   constexpr int W_RAW = NDW, W_X = NDW + 1, W_MMA = NDW + 2;                  // role warps
   extern __shared__ uint8_t smem_raw[];
-  __shared__ int s_used[(gemm_threads<DG>() + 31) / 32];
+  __shared__ int s_used[4], s_row[128];          // grouped: pairs per 32 entries of the block, result row of each entry
   uint8_t* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);   // (stays a shared-memory pointer to the compiler)
   const int NT = a.NT, SA = a.astages, SX = a.xstages, R = a.rstages;
   const int XT = NT * 128;                       // bytes of an activation tile
@@ -191,26 +191,23 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   }
   if (GROUPED) {
     pdl_wait();                                                  // the block table comes from an earlier kernel
-    if (tok0 >= a.npost[0]) return;                              // beyond the blocks the routing filled
-    const int expert = a.bexp[tt];
+    // (the three lookups are requested together: a chain of them would be most of a short CTA's start-up)
+    const int npost = a.npost[0], expert = a.bexp[tt];
+    int p = -1;
+    if (tid < NT) p = a.sorted[tok0 + tid];
+    if (tok0 >= npost) return;                                   // beyond the blocks the routing filled
     if (expert < 0 || expert >= a.E) return;                     // another rank's expert
     eo = reinterpret_cast<const int*>(a.eop[expert]);
     el = reinterpret_cast<const uint32_t*>(a.elp[expert]);
     wm = a.maps + expert;
-    // pairs in the block: one past the last entry that is not padding
-    int used = 0;
+    if (tid == 0) asm volatile("prefetch.tensormap [%0];" :: "l"(wm) : "memory");
     if (tid < NT) {
-      const int p = a.sorted[tok0 + tid];
-      used = (p >= 0 && p < a.B) ? tid + 1 : 0;
+      const bool pair = p >= 0 && p < a.B;
+      s_row[tid] = pair ? p : -1;
+      const int used = __reduce_max_sync(FULL, pair ? tid + 1 : 0);
+      if (lane == 0) s_used[warp] = used;
     }
-    used = __reduce_max_sync(FULL, used);
-    if (lane == 0) s_used[warp] = used;
-    __syncthreads();
-    ncol = 0;
-    for (int w = 0; w * 32 < NT; ++w) ncol = max(ncol, s_used[w]);
-    if (ncol == 0) return;
   }
-  const int nmma = GROUPED ? (ncol + 15) & ~15 : NT;             // token columns the MMAs cover
 
   if (tid == 0) {
     for (int s = 0; s < SA; ++s) { mbar_init(aready + s, NDEC); mbar_init(aempty + s, 1); }
@@ -226,6 +223,11 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (GROUPED) {                                                 // pairs in the block: one past the last that is not padding
+    ncol = 0;
+    for (int w = 0; w * 32 < NT; ++w) ncol = max(ncol, s_used[w]);
+  }
+  const int nmma = GROUPED ? (max(ncol, 1) + 15) & ~15 : NT;     // token columns the MMAs cover
   const uint32_t tmem = *tmem_slot;
   const uint32_t tmem_a = tmem + (uint32_t)((NT + 31) & ~31);    // the weight tiles' columns follow the accumulator
   pdl_launch_dependents();
@@ -410,8 +412,8 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
           const int c = c0 + j + (lane & 1);
           if (c < ncol && acc_ok) {
             long long row = tok0 + c;
-            if (GROUPED) row = a.sorted[tok0 + c];                 // result rows go back to their pair index
-            if (!GROUPED || (row >= 0 && row < a.B)) {
+            if (GROUPED) row = s_row[c];                           // result rows go back to their pair index
+            if (!GROUPED || row >= 0) {
               *reinterpret_cast<uint32_t*>(Yp + (size_t)row * Mp + m0) = pack_bf16(x0, x1);
               if (Yfp) *reinterpret_cast<float2*>(Yfp + (size_t)row * Mp + m0) = make_float2(x0, x1);
             }

@@ -12,9 +12,12 @@ from .linear import TreeLinear, _state
 from .ops import ext
 
 SLOT_MAX = 32                       # (token, expert) pairs up to which the ungrouped kernel runs
-GEMM_PAIRS_PER_EXPERT = 8           # average pairs per expert from which the grouped tcgen05 GEMM takes over: the
+GEMM_PAIRS_PER_EXPERT = 0.5         # average pairs per expert from which the grouped tcgen05 GEMM takes over: the
 #                                     grouped GEMV re-reads an expert's records for every 8 of its pairs, the GEMM
-#                                     reads them once per 64 (128 from 64 pairs per expert on)
+#                                     reads them once per 64 or 128.  Block of 128 experts of 2048 x 768, us with the GEMV /
+#                                     the GEMM: 48 pairs 84 / 89, 64 pairs 106 / 104, 96 pairs 131 / 123, 1024 pairs 362 / 208
+GEMM_WIDE_PAIRS_PER_EXPERT = 48     # average from which its blocks hold 128 pairs (us with 64 / 128: 32 pairs per expert
+#                                     237 / 247, 62 per expert 317 / 294): an expert then rarely needs a second block
 
 
 def _aligned(x):
@@ -135,6 +138,18 @@ def moe_group_gemm(tables, maps, x, aligned, bs, S, M, xdiv, zero=False, yf32=No
     xg = torch.empty(sorted_ids.numel(), x.shape[1], dtype=torch.bfloat16, device=x.device)
     E.moe_gather(x, sorted_ids, npost, S, xdiv, xg)
     E.gtt(maps, tables[1], tables[3], xg, sorted_ids, bexp, npost, bs, y, yf32)
+    return y
+
+
+def _group_gemm_of_gated(tables, maps, gu, aligned, bs, S, M):
+    """moe_group_gemm of silu_mul(gu) (one row per pair): the gate writes its rows in block order, so neither the
+    activations in pair order nor a gather of them is needed"""
+    sorted_ids, bexp, npost = aligned
+    E = ext()
+    y = torch.empty(S, M, dtype=torch.bfloat16, device=gu.device)
+    xg = torch.empty(sorted_ids.numel(), gu.shape[1] // 2, dtype=torch.bfloat16, device=gu.device)
+    E.moe_silu_gather(gu, sorted_ids, npost, S, xg)
+    E.gtt(maps, tables[1], tables[3], xg, sorted_ids, bexp, npost, bs, y, None)
     return y
 
 
@@ -384,6 +399,8 @@ class TreeExperts(nn.Module):
     def tensor_maps(self):
         """weight tensor maps of the grouped tcgen05 GEMM, or None when the shapes do not fit it (rows % 128)"""
         if self._maps is None:
+            if torch.cuda.is_current_stream_capturing():        # (they are copied from the host: not inside a capture)
+                return None
             if (2 * self.inter) % 128 or self.hidden % 128:
                 self._maps = False
             else:
@@ -445,11 +462,11 @@ class TreeExperts(nn.Module):
             gu = moe_gemv(t13, x, ids, 2 * self.inter, K)
             y = moe_gemv(t2, silu_mul(gu), ids, self.hidden, 1)
         elif S >= GEMM_PAIRS_PER_EXPERT * self.num_experts and self.tensor_maps() is not None:
-            bs = 128 if S >= 64 * self.num_experts else 64
+            bs = 128 if S >= GEMM_WIDE_PAIRS_PER_EXPERT * self.num_experts else 64
             m13, m2 = self.tensor_maps()
             al = moe_align(ids, self.num_experts, bs)
             gu = moe_group_gemm(t13, m13, x, al, bs, S, 2 * self.inter, K)
-            y = moe_group_gemm(t2, m2, silu_mul(gu), al, bs, S, self.hidden, 1)
+            y = _group_gemm_of_gated(t2, m2, gu, al, bs, S, self.hidden)
         else:
             al = moe_align(ids, self.num_experts, 8)
             gu = moe_group_gemv(t13, x, al, S, 2 * self.inter, K)

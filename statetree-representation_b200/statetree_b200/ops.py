@@ -61,6 +61,7 @@ _SIGNATURES = {
     "st_moe_tensor_maps": (_int, [_vp, _i64, _i64, _i64, _vp, _vp]),
     "st_moe_gather": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp]),
     "st_moe_group_gemm": (_int, [_vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _vp]),
+    "st_moe_silu_gather": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
     "st_comm_bytes": (_i64, []),
     "st_comm_set_timeout_ms": (_int, [_i64]),
     "st_comm_alloc": (_int, [ctypes.POINTER(ctypes.c_void_p)]),
@@ -331,6 +332,12 @@ class _Weights:
         with _ctx(X):
             _check(lib().st_moe_gather(_ptr(X), _ptr(sorted_ids), _ptr(npost), Xg.shape[0], S, xdiv, X.shape[1], _ptr(Xg),
                                        _stream(X)))
+
+    @staticmethod
+    def moe_silu_gather(gu, sorted_ids, npost, S, Xg):
+        with _ctx(gu):
+            _check(lib().st_moe_silu_gather(_ptr(gu), _ptr(sorted_ids), _ptr(npost), Xg.shape[0], S, Xg.shape[1], _ptr(Xg),
+                                            _stream(gu)))
 
     @staticmethod
     def gtt(maps, EOP, ELP, Xg, sorted_ids, bexp, npost, bs, Y, Yf32=None):

@@ -306,3 +306,23 @@ def test_tree_experts_replaces_a_transformers_experts_module():
             a = torch.nn.functional.silu(g) * u
             want[t] += w[t, j] * (a.float() @ Wd[e].float() + bd[e].float()).to(torch.bfloat16).float()
     assert (got - want).abs().max().item() <= 0.03 * want.abs().max().item() + 1e-3
+
+
+@pytest.mark.parametrize("S,I,bs", [(1, 8, 64), (37, 776, 64), (600, 768, 128), (65, 64, 128)])
+def test_silu_gather_equals_gate_then_gather(S, I, bs):
+    """the gate written in block order against silu_mul followed by an index: widths that do not fill a warp's step, blocks
+    with padding (left as they were), rows beyond the used blocks"""
+    from statetree_b200.experts import moe_align, silu_mul
+    from statetree_b200.ops import ext
+    E = 5
+    g = torch.Generator(DEV).manual_seed(S)
+    gu = torch.randn(S, 2 * I, device=DEV, generator=g).to(torch.bfloat16)
+    gu[0, 0], gu[0, I] = float("inf"), 2.0
+    sorted_ids, _, npost = moe_align(torch.randint(0, E, (S,), device=DEV, generator=g), E, bs)
+    xg = torch.full((sorted_ids.numel(), I), 7.0, dtype=torch.bfloat16, device=DEV)
+    ext().moe_silu_gather(gu, sorted_ids, npost, S, xg)
+    act = silu_mul(gu)
+    valid = (sorted_ids < S) & (torch.arange(sorted_ids.numel(), device=DEV) < npost)
+    want = torch.full_like(xg, 7.0)
+    want[valid] = act[sorted_ids[valid].long()]
+    assert torch.equal(xg.view(torch.int16), want.view(torch.int16))
