@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) silu_mul_vec_kernel(const uint4* __restri
 }
 // silu_mul of the pair each used entry of sorted names, written in block order: Xg[i, :] = silu(gate) * up of gu[sorted[i]]
 // (the activation rows of the second grouped product; no act array and no gather of it in between).  One warp per row,
-// 16-byte vectors.  8000 pairs of 768 in 24 576 bytes of gu each: silu_mul 13 us + gather 5 us before, BBB us.
+// 16-byte vectors.  8000 pairs of 768 in 24 576 bytes of gu each: silu_mul 13 us + gather 5 us before, 10 us.
 __global__ void __launch_bounds__(256) moe_silu_gather_kernel(const uint4* __restrict__ gu, const int* __restrict__ sorted,
                                                               const int* __restrict__ npost, int S, int I8, long long rows,
                                                               uint4* __restrict__ Xg) {
@@ -94,53 +94,52 @@ __global__ void __launch_bounds__(256) moe_silu_gather_kernel(const uint4* __res
 // expert, every expert's run padded to a multiple of bs with the value S; bexp[b] = expert of block b; npost = entries
 // in use.  One CTA does the whole job in shared memory.  Expert ids outside [0, E) count as E - 1 / 0 (clamped).
 //
-// Warp w owns the w-th of 32 contiguous chunks of the pairs.  Pass 1: each warp counts its chunk's pairs per expert, 32 at
-// a time (__match_any_sync finds the lanes of equal expert; the first of them adds their number to the warp's own
-// counter, no atomics).  A prefix sum over (expert, warp) turns the counts into each warp's first slot per expert.  Pass 2:
-// the same walk places every pair at its expert's next slot, so the original order survives without a sort.
-// 8000 pairs, 128 experts: 106 us when every warp scanned all pairs once per expert it owned, AAA us now (latency: two
-// walks of eight steps and the scan).
+// Warp w of W owns the w-th of W contiguous chunks of the pairs.  Pass 1: each warp counts its chunk's pairs per expert in a
+// counter array of its own.  A prefix sum over (expert, warp) turns the counts into each warp's first slot per expert.
+// Pass 2: the chunk again, 32 pairs a step; every lane sets its bit in the warp's mask of its expert, so the lanes of equal
+// expert see one another and each takes its place among them: the original order survives without a sort.
+// 8000 pairs, 128 experts: 106 us when every warp scanned all pairs once per expert it owned, 10 us now (__match_any_sync
+// in place of the masks: 20 us).
 constexpr int ALIGN_MAX_E = 1024;
-constexpr int ALIGN_WARPS = 32;
+__host__ __device__ constexpr int align_warps(int E) { return E <= 512 ? 32 : 16; }      // counters + masks: 8 W E <= 128 KB
 template <bool IDS64>
 __global__ void __launch_bounds__(1024) moe_align_kernel(const void* __restrict__ ids_, int S, int E, int used_bins,
                                                          int nblk, int bs, int* __restrict__ sorted,
                                                          int* __restrict__ bexp, int* __restrict__ npost) {
-  extern __shared__ int s_count[];                                   // [warp][E]: counts, then next slot inside the expert
+  extern __shared__ int s_count[];                                   // [W][E]: counts, then next slot inside the expert
   __shared__ int end_[ALIGN_MAX_E], begin_[ALIGN_MAX_E], wsum[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int W = align_warps(E);
+  unsigned* const s_mask = reinterpret_cast<unsigned*>(s_count + W * E);   // [W][E]: lanes of the current step per expert
   int* const mine = s_count + warp * E;
-  for (int e = lane; e < E; e += 32) mine[e] = 0;
+  unsigned* const mask = s_mask + warp * E;
+  for (int i = tid; i < 2 * W * E; i += 1024) s_count[i] = 0;
   st::pdl_launch_dependents();
   st::pdl_wait();
   auto id_of = [&](int i) {
     long long v = IDS64 ? reinterpret_cast<const long long*>(ids_)[i] : (long long)reinterpret_cast<const int*>(ids_)[i];
     return (int)(v < 0 ? 0 : (v >= E ? E - 1 : v));
   };
-  const int chunk = ((S + ALIGN_WARPS - 1) / ALIGN_WARPS + 31) & ~31;
-  const int lo = min(S, warp * chunk), hi = min(S, lo + chunk);
-  // visits the chunk 32 pairs a step, in order: f(pair index, its expert or -1, lanes of the same expert).  The ids of
-  // four steps are requested together.
+  const int chunk = ((S + W - 1) / W + 31) & ~31;
+  const int lo = min(S, warp * chunk), hi = warp < W ? min(S, lo + chunk) : lo;
+  // visits the chunk 32 pairs a step, in order: f(pair index, its expert or -1).  The ids of four steps are requested together.
   auto walk = [&](auto f) {
     for (int base = lo; base < hi; base += 128) {
       int e[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) e[u] = base + 32 * u + lane < hi ? id_of(base + 32 * u + lane) : -1;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        f(base + 32 * u + lane, e[u], __match_any_sync(st::FULL, e[u]));
-        __syncwarp();
-      }
+      for (int u = 0; u < 4; ++u) f(base + 32 * u + lane, e[u]);
     }
   };
-  __syncwarp();
-  walk([&](int, int e, unsigned same) { if (e >= 0 && lane == __ffs(same) - 1) mine[e] += __popc(same); });
+  __syncthreads();
+  walk([&](int, int e) { if (e >= 0) atomicAdd(mine + e, 1); });
   for (int i = tid; i < nblk * bs; i += 1024) sorted[i] = S;         // padding value; the pairs go over it in pass 2
   __syncthreads();
   // totals per expert (thread e < E) and every warp's first slot inside the expert
   int total = 0;
   if (tid < E)
-    for (int w = 0; w < ALIGN_WARPS; ++w) {
+    for (int w = 0; w < W; ++w) {
       const int n = s_count[w * E + tid];
       s_count[w * E + tid] = total;
       total += n;
@@ -170,15 +169,22 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const void* __restrict_
     begin_[tid] = end_[tid] - room;
   }
   __syncthreads();
-  walk([&](int i, int e, unsigned same) {
-    const int rank = __popc(same & ((1u << lane) - 1u));
+  walk([&](int i, int e) {
+    if (e >= 0) atomicOr(mask + e, 1u << lane);
+    __syncwarp();
+    unsigned same = 0u;
     int at = 0;
     if (e >= 0) {
+      same = mask[e];
       at = mine[e];
-      sorted[begin_[e] + at + rank] = i;
+      sorted[begin_[e] + at + __popc(same & ((1u << lane) - 1u))] = i;
     }
     __syncwarp();
-    if (e >= 0 && rank == 0) mine[e] = at + __popc(same);
+    if (e >= 0 && (same & ((1u << lane) - 1u)) == 0u) {              // the first of them moves the expert on
+      mine[e] = at + __popc(same);
+      mask[e] = 0u;
+    }
+    __syncwarp();
   });
   // expert of every block: first expert whose end lies beyond the block's first slot (clamped for the unused tail)
   for (int b = tid; b < nblk; b += 1024) {
@@ -219,14 +225,14 @@ extern "C" int st_moe_align(const void* ids, int ids64, int64_t S, int64_t E, in
              "st_moe_align: nblk must cover S / bs + min(S, E) blocks");
   ST_REQUIRE(used_bins >= 1 && used_bins <= E, "st_moe_align: used_bins must be in [1, E]");
   ST_REQUIRE(ids && sorted && bexp && npost, "st_moe_align: null pointer");
-  const size_t smem = (size_t)ALIGN_WARPS * E * sizeof(int);
-  static bool set[64] = {};                                      // once per device: beyond 384 experts it takes over 48 KB
+  const size_t smem = (size_t)2 * align_warps((int)E) * E * sizeof(int);
+  static bool set[64] = {};                                      // once per device: beyond 192 experts it takes over 48 KB
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !set[dev]) {
     for (auto k : {moe_align_kernel<true>, moe_align_kernel<false>})
       if (int e = st::cuda_fail(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     ALIGN_WARPS * ALIGN_MAX_E * (int)sizeof(int)), "st_moe_align: shared memory attribute"))
+                                                     128 * 1024), "st_moe_align: shared memory attribute"))
         return e;
     set[dev] = true;
   }
