@@ -71,6 +71,7 @@ struct GemvArgs {
   int E, xdiv;
   int NG, CPT, T;                         // column groups, units per tile, tiles per problem
   long long U;                            // units over all problems
+  int uq, ur;                             // CTA b's range starts at unit b * uq + min(b, ur) (U = C * uq + ur)
   int nprob, maxcover, stages, fill, stage_bytes, nxrows, xwhole, xw_stride, xw_bytes;
   int act;                                // dense mode: rows are gate / up tiles in turn, the reducer stores silu(gate) * up
   ListTab lt;
@@ -135,7 +136,12 @@ __device__ __forceinline__ long long out_row(const GemvArgs& a, int p, int n) {
   return (n < 8 && s >= 0 && s < a.B) ? s : -1;
 }
 
-__device__ __forceinline__ int cta_of_unit(long long u, long long U, int C) { return (int)(((u + 1) * C - 1) / U); }
+// the first ur CTAs take uq + 1 units each, the others uq
+__device__ __forceinline__ int first_unit(const GemvArgs& a, int cta) { return cta * a.uq + min(cta, a.ur); }
+__device__ __forceinline__ int cta_of_unit(const GemvArgs& a, int u) {
+  const int big = a.ur * (a.uq + 1);
+  return u < big ? u / (a.uq + 1) : a.ur + (u - big) / a.uq;
+}
 
 // Walks a CTA's units without divisions: problem p, tile, unit c inside the tile.  The CTA's range [u0, u1) is
 // visited as two segments: first the units of the trailing tile it shares with the next CTA, then the rest.  Both
@@ -162,7 +168,7 @@ struct UnitCursor {
     u = ub; end = ue;
     if (u >= end) return;
     const int upp = a.T * a.CPT;
-    p = u / upp;
+    p = one_matrix(MODE) ? 0 : u / upp;
     const int ul = u - p * upp;
     tile = ul / a.CPT; c = ul - tile * a.CPT;
     enter(a);
@@ -213,6 +219,7 @@ struct UnitCursor {
 template <int NT, int MODE>
 __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(const GemvArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ const uint16_t* s_xrow[8];                        // MODE_SLOT / MODE_GROUP: activation rows of the current problem
   constexpr int NB = 8 * NT;                                   // activation columns of the mma
   constexpr int EL = 16 * NB;                                  // outputs of one tile
   constexpr int NRED = NT == 1 ? 4 : 2;                        // tile results in flight between consumers and reducer
@@ -229,20 +236,24 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
   int* fin_tile = reinterpret_cast<int*>(xbar + 1);                         // MODE_AR: [FIN_CAP] delivered tiles
   uint16_t* fin_mask = reinterpret_cast<uint16_t*>(fin_tile + FIN_CAP);     // MODE_AR: [FIN_CAP][32] values per lane
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0);   // (a warp-uniform value to the compiler)
   const int C = gridDim.x;
-  int u0 = (int)((long long)blockIdx.x * a.U / C), u1 = (int)((long long)(blockIdx.x + 1) * a.U / C);
+  int u0 = first_unit(a, blockIdx.x), u1 = first_unit(a, blockIdx.x + 1);
 
-  if (tid < S) {                                               // one thread per ring stage sets its barriers up
-    mbar_init(full + tid, 1);
-    mbar_init(empty + tid, CW);
+  if (warp == CW) {                                            // one lane per barrier
+    if (lane < S) {
+      mbar_init(full + lane, 1);
+      mbar_init(empty + lane, CW);
+    } else if (lane >= 16 && lane < 16 + NRED) {
+      mbar_init(done + lane - 16, CW);
+      mbar_init(freeb + lane - 16, 1);
+    } else if (lane == 31) {
+      mbar_init(xbar, 1);
+    }
     fence_barrier_init();
-  } else if (tid == 32) {
-    for (int b = 0; b < NRED; ++b) { mbar_init(done + b, CW); mbar_init(freeb + b, 1); }
-    mbar_init(xbar, 1);
-    fence_barrier_init();
+  } else if (tid >= 64 && tid < 64 + XROW / 16) {
+    reinterpret_cast<uint4*>(zrow)[tid - 64] = make_uint4(0, 0, 0, 0);
   }
-  if (tid >= 64 && tid < 64 + XROW / 16) reinterpret_cast<uint4*>(zrow)[tid - 64] = make_uint4(0, 0, 0, 0);
   __syncthreads();
   pdl_launch_dependents();                 // the next kernel in the stream may start its own weight prefetch
   if (MODE == MODE_SLOT || MODE == MODE_GROUP) pdl_wait();   // expert ids / slot tables come from earlier kernels
@@ -260,61 +271,63 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
   cur.init(a, u0, u1);
 
   if (warp == CW) {
-    // ------------------------------------------------------------------ producer warp.  Lane 0 moves the records,
-    // lane 1 the escape block, lane n activation row n.  Weights never depend on the previous kernel, so the first
-    // ring fill is issued before griddepcontrol.wait; activations (and everything the reducer touches) after it.
+    // ------------------------------------------------------------------ producer warp: per unit the records, the escape
+    // block and the activation slices, all issued by one elected lane of the converged warp.  (A copy takes its operands
+    // from uniform registers; issued by different lanes, or under a lane test, each costs ~500 cycles of serialising over the
+    // lanes, which made the first ring fill 1.5 to 4 us long and the eight activation rows of a stage slower to ask for than
+    // to use: 4096 x 12288 at 8 rows 20.8 us, now DOWN8.)  Weights never depend on the previous kernel, so the first ring fill
+    // is issued before griddepcontrol.wait; activations (and everything the reducer touches) after it.
     const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
     int lastp = -1;
-    const uint16_t* xrow = nullptr;                           // this lane's activation row of the current problem
-    unsigned nx = 0;
+    unsigned rows = one_matrix(MODE) && !a.xwhole ? (NX >= 32 ? FULL : (1u << NX) - 1u) : 0u;   // rows staged with every unit
     auto row_of = [&](const UnitCursor<MODE>& k) {
-      if (k.p != lastp) {
-        lastp = k.p;
-        const long long r = lane < NX ? out_row<MODE>(a, k.p, lane) : -1;
-        xrow = r < 0 ? nullptr : a.X + (one_matrix(MODE) ? r : r / a.xdiv) * a.N;
-        nx = a.xwhole ? 0u : __popc(__ballot_sync(FULL, xrow != nullptr));
-      }
+      if (one_matrix(MODE) || k.p == lastp) return;
+      lastp = k.p;
+      const long long r = lane < NX ? out_row<MODE>(a, k.p, lane) : -1;
+      if (lane < NX) s_xrow[lane] = r < 0 ? nullptr : a.X + r / a.xdiv * a.N;
+      rows = __ballot_sync(FULL, r >= 0);
+      __syncwarp();
     };
     auto weights = [&](const UnitCursor<MODE>& k, int s) {
-      const int nrec = k.nrec(a);
+      const uint32_t nrec = (uint32_t)k.nrec(a);
       uint8_t* st = ring + (size_t)s * STAGE;
-      if (lane == 0) {
-        mbar_expect_tx(full + s, (uint32_t)(nrec * REC + SIDE_BYTES) + nx * (uint32_t)(nrec * 128));
-        bulk_g2s(st, k.tree() + ((size_t)k.ltile() * a.NG + (size_t)k.c * CW) * REC, (uint32_t)(nrec * REC), full + s, pol_w);
+      if (elect_one()) {
+        mbar_expect_tx(full + s, nrec * REC + SIDE_BYTES + (uint32_t)__popc(rows) * (nrec * 128));
+        bulk_g2s(st, k.tree() + ((size_t)k.ltile() * a.NG + (size_t)k.c * CW) * REC, nrec * REC, full + s, pol_w);
+        bulk_g2s(st + UNIT_BYTES, k.eb() + ((size_t)k.ltile() * a.CPT + k.c) * 16, SIDE_BYTES, full + s, pol_w);
       }
       __syncwarp();
-      if (lane == 1)
-        bulk_g2s(st + UNIT_BYTES, k.eb() + ((size_t)k.ltile() * a.CPT + k.c) * 16, SIDE_BYTES, full + s, pol_w);
     };
     auto acts = [&](const UnitCursor<MODE>& k, int s) {
-      if (!a.xwhole && xrow != nullptr)
-        bulk_g2s(ring + (size_t)s * STAGE + UNIT_BYTES + SIDE_BYTES + lane * XROW, xrow + (size_t)k.c * CW * 64,
-                 (uint32_t)(k.nrec(a) * 128), full + s, pol_x);
-    };
-    UnitCursor<MODE> mine = cur;                               // lane i looks at unit i of this CTA
-    for (int i = 0; i < lane && mine.valid(); ++i) mine.next(a);
-    // first ring fill: weights, then wait for the previous kernel, then the activations
-    UnitCursor<MODE> pre = cur;
-    int filled = 0;
-    if (one_matrix(MODE)) {                                    // lane i fills stage i
-      const bool on = lane < a.fill && mine.valid();
-      if (on) {
-        const int nrec = mine.nrec(a);
-        uint8_t* st = ring + (size_t)lane * STAGE;
-        mbar_expect_tx(full + lane, (uint32_t)(nrec * REC + SIDE_BYTES) + (a.xwhole ? 0u : (uint32_t)(NX * nrec * 128)));
-        bulk_g2s(st, mine.tree() + ((size_t)mine.ltile() * a.NG + (size_t)mine.c * CW) * REC, (uint32_t)(nrec * REC),
-                 full + lane, pol_w);
-        bulk_g2s(st + UNIT_BYTES, mine.eb() + ((size_t)mine.ltile() * a.CPT + mine.c) * 16, SIDE_BYTES, full + lane, pol_w);
+      const uint32_t bytes = (uint32_t)(k.nrec(a) * 128);
+      uint8_t* dst = ring + (size_t)s * STAGE + UNIT_BYTES + SIDE_BYTES;
+      const size_t at = (size_t)k.c * CW * 64;
+      if (elect_one()) {
+        if (one_matrix(MODE)) {
+          if (!a.xwhole) {
+            const uint16_t* src = a.X + at;
+            for (int n = 0; n < NX; ++n, src += a.N, dst += XROW) bulk_g2s(dst, src, bytes, full + s, pol_x);
+          }
+        } else {
+          for (unsigned m = rows; m; m &= m - 1) {
+            const int n = __ffs(m) - 1;
+            bulk_g2s(dst + n * XROW, s_xrow[n] + at, bytes, full + s, pol_x);
+          }
+        }
       }
-      filled = __popc(__ballot_sync(FULL, on));
-    } else {
-      for (; pre.valid() && filled < a.fill; pre.next(a), ++filled) { row_of(pre); weights(pre, filled); }
-    }
+      __syncwarp();
+    };
+    UnitCursor<MODE> pre = cur;                                // first ring fill
+    int filled = 0;
+    for (; pre.valid() && filled < a.fill; pre.next(a), ++filled) { row_of(pre); weights(pre, filled); }
     pdl_wait();
     if (a.xwhole && MODE != MODE_NORM) {                       // every activation row once, whole
-      if (lane == 0) mbar_expect_tx(xbar, (uint32_t)(NX * a.N * 2));
+      if (elect_one()) {
+        mbar_expect_tx(xbar, (uint32_t)(NX * a.N * 2));
+        for (int n = 0; n < NX; ++n)
+          bulk_g2s(xw + (size_t)n * a.xw_stride, a.X + (size_t)n * a.N, (uint32_t)(a.N * 2), xbar, pol_x);
+      }
       __syncwarp();
-      if (lane < NX) bulk_g2s(xw + (size_t)lane * a.xw_stride, a.X + (size_t)lane * a.N, (uint32_t)(a.N * 2), xbar, pol_x);
     }
     lastp = -1;
     int s = 0;
@@ -465,7 +478,7 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
       mask = 0;
       if (!owned) {
         const long long tg = (long long)cur.p * a.T + cur.tile;
-        const int cfirst = cta_of_unit(tbase, a.U, C), clast = cta_of_unit(tbase + a.CPT - 1, a.U, C);
+        const int cfirst = cta_of_unit(a, tbase), clast = cta_of_unit(a, tbase + a.CPT - 1);
         const int last_level = clast - cfirst;                  // parts - 1
         const int part = blockIdx.x - cfirst;
         uint32_t* slots = reinterpret_cast<uint32_t*>(a.ws) + (size_t)tg * a.maxcover * EL;
@@ -834,7 +847,7 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
 template <int NT, int MODE>
 int launch(GemvArgs& a, int nprob, int nx, long long ws_bytes, cudaStream_t stream, const char* who) {
   const Plan p = make_plan<NT>(a.M, a.N, nprob, nx, one_matrix(MODE), a.act != 0, MODE == MODE_AR);
-  a.NG = p.NG; a.CPT = p.CPT; a.T = p.T; a.U = p.U; a.nprob = nprob; a.maxcover = p.maxcover; a.stages = p.stages; a.fill = p.fill;
+  a.NG = p.NG; a.CPT = p.CPT; a.T = p.T; a.U = p.U; a.uq = (int)(p.U / p.C); a.ur = (int)(p.U % p.C); a.nprob = nprob; a.maxcover = p.maxcover; a.stages = p.stages; a.fill = p.fill;
   a.stage_bytes = p.stage_bytes; a.nxrows = p.nxrows; a.xwhole = p.xwhole; a.xw_stride = p.xw_stride;
   a.xw_bytes = p.xw_bytes;
   const long long need = (long long)nprob * p.T * p.maxcover * 16 * 8 * NT * 4;
