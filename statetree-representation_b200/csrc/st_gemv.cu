@@ -275,7 +275,7 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
     // block and the activation slices, all issued by one elected lane of the converged warp.  (A copy takes its operands
     // from uniform registers; issued by different lanes, or under a lane test, each costs ~500 cycles of serialising over the
     // lanes, which made the first ring fill 1.5 to 4 us long and the eight activation rows of a stage slower to ask for than
-    // to use: 4096 x 12288 at 8 rows 20.8 us, now DOWN8.)  Weights never depend on the previous kernel, so the first ring fill
+    // to use: 4096 x 12288 at 8 rows 20.8 us, now 14.7.)  Weights never depend on the previous kernel, so the first ring fill
     // is issued before griddepcontrol.wait; activations (and everything the reducer touches) after it.
     const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
     int lastp = -1;
@@ -771,7 +771,7 @@ static int tune(const char* name, int dflt) {
 
 // nx = activation rows staged per unit (the batch for a dense matrix, 1 per slot, 8 per block of slots).
 template <int NT>
-Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act = false, bool ar = false) {
+Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act = false, bool ar = false, bool norm = false) {
   Plan p;
   p.NG = (int)(N / 64);
   p.CPT = (p.NG + CW - 1) / CW;
@@ -779,9 +779,12 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
   p.nprob = nprob;
   p.U = (long long)nprob * p.T * p.CPT;
   p.nxrows = nx;
-  // Whole activation rows stay resident in shared memory when they fit in 66 KB (8 rows of 4096 columns), which leaves
-  // at least three ring stages; beyond that every stage carries the matching 512-column slice of each row.
-  static const int xw_kb = tune("STATETREE_GEMV_XWHOLE_KB", 66);
+  // Whole activation rows stay resident in shared memory when they fit in 34 KB (4 rows of 4096 columns), beside at least six
+  // ring stages; beyond that every stage carries the matching 512-column slice of each row (24576 x 4096 at 8 rows: whole
+  // rows beside three stages 31.2 us, slices 27.0; at 4 rows 25.6 / 25.9).  The pre-norm mode forms whole rows itself, so
+  // it takes up to 66 KB.
+  static const int xw_tune = tune("STATETREE_GEMV_XWHOLE_KB", 34);
+  const int xw_kb = norm ? 66 : xw_tune;
   p.xwhole = (dense && (long long)nx * (N * 2 + 16) <= (long long)xw_kb * 1024) ? 1 : 0;
   p.xw_stride = p.xwhole ? (int)(N * 2 + 16) : 0;
   p.xw_bytes = p.xwhole ? nx * p.xw_stride : 0;
@@ -792,7 +795,7 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
   // Two CTAs per SM, each with the deepest ring (at most 8 stages) that fits half of the SM's shared memory; one CTA
   // when even two stages do not fit twice (32 activation rows).
   static const int want_per_sm = tune("STATETREE_GEMV_CTAS_PER_SM", 2), max_stages = tune("STATETREE_GEMV_STAGES", 8),
-                   align = tune("STATETREE_GEMV_ALIGN", 1), min_units = tune("STATETREE_GEMV_MIN_UNITS", 2);
+                   align = tune("STATETREE_GEMV_ALIGN", 1), min_tune = tune("STATETREE_GEMV_MIN_UNITS", 3);
   int per_sm = want_per_sm < 1 ? 1 : (want_per_sm > 2 ? 2 : want_per_sm);
   int stages = 0;
   for (; per_sm >= 1; --per_sm) {
@@ -806,7 +809,10 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
   p.stages = stages;
   p.smem = (size_t)stages * p.stage_bytes + fixed;
   const long long slots = (long long)st::sm_count() * per_sm;
-  long long want = p.U / (min_units < 1 ? 1 : min_units);     // small matrices: no CTA with less than min_units units
+  // Small matrices: no CTA with less than three units, or a tile is cut into so many parts that their exchange is the tail
+  // (1024 x 4096, tiles of eight units: four parts 4.6 us at 1 row and 7.4 at 8, two parts 4.5 and 4.7)
+  const int min_units = act ? 2 : (min_tune < 1 ? 1 : min_tune);
+  long long want = p.U / min_units;
   if (want < 1) want = 1;
   p.C = (int)(want < slots ? want : slots);
   // Grid.  Cutting tiles at arbitrary unit boundaries fills every slot with the same amount of work, but the CTA that
@@ -846,7 +852,7 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
 
 template <int NT, int MODE>
 int launch(GemvArgs& a, int nprob, int nx, long long ws_bytes, cudaStream_t stream, const char* who) {
-  const Plan p = make_plan<NT>(a.M, a.N, nprob, nx, one_matrix(MODE), a.act != 0, MODE == MODE_AR);
+  const Plan p = make_plan<NT>(a.M, a.N, nprob, nx, one_matrix(MODE), a.act != 0, MODE == MODE_AR, MODE == MODE_NORM);
   a.NG = p.NG; a.CPT = p.CPT; a.T = p.T; a.U = p.U; a.uq = (int)(p.U / p.C); a.ur = (int)(p.U % p.C); a.nprob = nprob; a.maxcover = p.maxcover; a.stages = p.stages; a.fill = p.fill;
   a.stage_bytes = p.stage_bytes; a.nxrows = p.nxrows; a.xwhole = p.xwhole; a.xw_stride = p.xw_stride;
   a.xw_bytes = p.xw_bytes;
@@ -971,7 +977,7 @@ extern "C" int st_gemv_list(int64_t n, const void* const* trees, const int32_t* 
 extern "C" int st_gemv_prenorm_supported(int64_t M, int64_t N, int64_t B, int act) {
   if (M <= 0 || N <= 0 || M % 16 || N % 64 || N % 8 || B < 1 || B > 8) return 0;
   if (act && !st_gemv_swiglu_supported(M, N, B)) return 0;
-  const Plan p = make_plan<1>(M, N, 1, (int)B, true, act != 0);
+  const Plan p = make_plan<1>(M, N, 1, (int)B, true, act != 0, false, true);
   return (p.xwhole && p.stages >= 2) ? 1 : 0;
 }
 

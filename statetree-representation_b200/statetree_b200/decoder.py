@@ -207,9 +207,9 @@ class TreeDecoder:
         """(delta, summed): the output of a row-parallel projection (o, down) on this rank's activation slice.  A tree
         layer at GEMV batch sizes sums over the ranks inside its own kernel (summed = True); otherwise the partial
         output comes back and _add_norm adds the ranks."""
-        from .linear import GEMV_MAX, _state
+        from .linear import GEMV_AR_MAX, GEMV_MAX, _state
         B = xin.shape[0]
-        if (self.world > 1 and self.comm is not None and self.compressed and B <= min(GEMV_MAX, 32)
+        if (self.world > 1 and self.comm is not None and self.compressed and B <= min(GEMV_MAX, GEMV_AR_MAX)
                 and layer.bias is None and self.comm.gemv_allreduce_fits(layer.out_features, B)):
             eo, el, eb = layer.tables()
             y = torch.empty(B, layer.out_features, dtype=torch.bfloat16, device=self.dev)

@@ -12,10 +12,10 @@ from .linear import TreeLinear, _state
 from .ops import ext
 
 SLOT_MAX = 32                       # (token, expert) pairs up to which the ungrouped kernel runs
-GEMM_PAIRS_PER_EXPERT = 0.5         # average pairs per expert from which the grouped tcgen05 GEMM takes over: the
+GEMM_PAIRS_PER_EXPERT = 1.25        # average pairs per expert from which the grouped tcgen05 GEMM takes over: the
 #                                     grouped GEMV re-reads an expert's records for every 8 of its pairs, the GEMM
 #                                     reads them once per 64 or 128.  Block of 128 experts of 2048 x 768, us with the GEMV /
-#                                     the GEMM: 48 pairs 84 / 89, 64 pairs 106 / 104, 96 pairs 131 / 123, 1024 pairs 362 / 208
+#                                     the GEMM: 64 pairs 93 / 103, 128 pairs 140 / 147, 192 pairs 186 / 165, 1024 pairs 344 / 205
 GEMM_WIDE_PAIRS_PER_EXPERT = 48     # average from which its blocks hold 128 pairs (us with 64 / 128: 32 pairs per expert
 #                                     237 / 247, 62 per expert 317 / 294): an expert then rarely needs a second block
 

@@ -17,7 +17,10 @@ import torch.nn as nn
 from . import format as F
 from .ops import ext
 
-GEMV_MAX = int(os.environ.get("STATETREE_GEMV_MAX", "12"))     # activation rows up to which the GEMV kernel runs (<= 32)
+# activation rows up to which the GEMV kernel runs (<= 32).  The four projections of a 4096 / 12288 layer in a graph, us with
+# the GEMV / the tcgen05 GEMM: 8 rows 57 / 72, 16 rows 68 / 72, 20 rows 125 / 72 (beyond 16 the GEMV holds one CTA per SM)
+GEMV_MAX = int(os.environ.get("STATETREE_GEMV_MAX", "16"))
+GEMV_AR_MAX = 12                    # rows up to which the GEMV that sums over the ranks itself is used (tensor parallelism)
 # more activation rows than this (prefill): the tree is decoded once into a BF16 scratch matrix and cuBLAS multiplies by
 # it, the reference's path above 1024 rows (statetree/linear.py:37, 879-886), here from the size at which it overtakes the
 # tcgen05 kernel; 0 turns it off

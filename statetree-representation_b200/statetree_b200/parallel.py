@@ -170,11 +170,11 @@ class RowParallelTreeLinear(nn.Module):
         self.group = group
 
     def forward(self, x_local):
-        from .linear import GEMV_MAX, _rows_2d, _state
+        from .linear import GEMV_AR_MAX, GEMV_MAX, _rows_2d, _state
         tl = self.inner
         comm = peer_comm(self.group) if tl.tree.is_cuda else None
         rows = x_local.numel() // tl.in_features
-        if comm is None or tl.bias is not None or not (1 <= rows <= min(GEMV_MAX, 32)) \
+        if comm is None or tl.bias is not None or not (1 <= rows <= min(GEMV_MAX, GEMV_AR_MAX)) \
                 or not comm.gemv_allreduce_fits(tl.out_features, rows):
             return reduce_partials(tl(x_local), self.group)
         from . import ops
