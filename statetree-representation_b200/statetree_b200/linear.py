@@ -15,7 +15,7 @@ import torch
 import torch.nn as nn
 
 from . import format as F
-from .ops import ext
+from .ops import _raw_stream, ext, on_device
 
 # activation rows up to which the GEMV kernel runs (<= 32).  The four projections of a 4096 / 12288 layer in a graph, us with
 # the GEMV / the tcgen05 GEMM: 8 rows 57 / 72, 16 rows 68 / 72, 20 rows 125 / 72 (beyond 16 the GEMV holds one CTA per SM)
@@ -43,6 +43,7 @@ class _DevState:
     def __init__(self, device):
         self.device = device
         self._retired = []
+        self._need = {}                                 # workspace bytes per call shape (a pure function of it)
         self.ws = self._new_ws(1 << 20)
         self.scratch = torch.empty(1 << 20, dtype=torch.float32, device=device)   # the GEMM's partial tiles (no contract)
         self.cnt = torch.zeros(1 << 16, dtype=torch.int32, device=device)
@@ -55,6 +56,16 @@ class _DevState:
             self._retired.append(self.ws)
             self.ws = self._new_ws((nbytes + 3) // 4)
         return self.ws
+
+    def gemv_ws(self, M, N, B):
+        """workspace for a GEMV of an M x N matrix (M a tuple: a list of matrices) with B rows"""
+        need = self._need.get((M, N, B))
+        if need is None:
+            E = ext()
+            need = E.gemv_list_workspace_bytes(M, N, B) if isinstance(M, tuple) else E.gemv_workspace_bytes(M, N, B)
+            if len(self._need) < 4096:
+                self._need[(M, N, B)] = need
+        return self.get_ws(need)
 
     def get_scratch(self, nbytes):
         if self.scratch.numel() * 4 < nbytes:
@@ -143,13 +154,15 @@ class _DenseStage:
 
 
 def _state(device):
-    device = torch.device(device)
-    if device.index is None:
-        device = torch.device("cuda", torch.cuda.current_device())
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
+    index = device.index
+    if index is None:
+        index = torch.cuda.current_device()
+    key = (index, _raw_stream(index))
     st = _STATES.get(key)
     if st is None:
-        st = _STATES[key] = _DevState(device)
+        st = _STATES[key] = _DevState(torch.device("cuda", index))
     return st
 
 
@@ -167,9 +180,7 @@ def _rows_2d(x, width):
 _BY_HANDLE = weakref.WeakValueDictionary()
 
 
-def _tracing():
-    comp = getattr(torch, "compiler", None)
-    return comp is not None and hasattr(comp, "is_compiling") and comp.is_compiling()
+_tracing = getattr(getattr(torch, "compiler", None), "is_compiling", None) or (lambda: False)
 
 
 class TreeLinear(nn.Module):
@@ -308,7 +319,7 @@ class TreeLinear(nn.Module):
         """(eo, el, eb) escape side tables, built on first use (outside any graph capture).  The kernels read them
         before they wait for the preceding kernel of the stream (programmatic dependent launch), so the tables must be
         complete before that kernel starts: the stream is synchronised once after building them."""
-        if self._tables is None or self._tables[0].device != self.tree.device:
+        if self._tables is None or self._tables[0].device != self._buffers["tree"].device:
             self._tables = F.escape_tables(self.out_features, self.in_features, self.esc_rows, self.esc_cols,
                                            self.esc_bits)
             if self.tree.is_cuda and not torch.cuda.is_current_stream_capturing():
@@ -341,8 +352,7 @@ class TreeLinear(nn.Module):
         eo, el, eb = self.tables()
         st = _state(x.device)
         if B <= min(GEMV_MAX, 32):
-            ws = st.get_ws(E.gemv_workspace_bytes(M, N, B))
-            E.gemv(self.tree, eo, eb, el, x, y, ws, st.get_cnt(M // 16), yf32)
+            E.gemv(self._buffers["tree"], eo, eb, el, x, y, st.gemv_ws(M, N, B), st.get_cnt(M // 16), yf32)
         elif 0 < PREFILL_MIN < B and yf32 is None and self.dense_ok() and not torch.cuda.is_current_stream_capturing():
             st.dense_stage().run(self, x, y)                # decode once + cuBLAS, the next layer decoded meanwhile
         elif M % 128 == 0:
@@ -363,18 +373,20 @@ class TreeLinear(nn.Module):
     def _forward(self, x, yf32=None):
         """any leading shape, any float dtype, any device: the product runs where the tree lives, in BF16, and comes
         back in the caller's dtype on the caller's device"""
-        home, asked_dtype, asked_device = self.tree.device, x.dtype, x.device
+        home, asked_dtype, asked_device = self._buffers["tree"].device, x.dtype, x.device
         if home.type != "cuda":
             raise RuntimeError("statetree_b200: the kernels take CUDA tensors only (no CPU path); move the layer to a GPU")
         lead = x.shape[:-1]
         acts = _rows_2d(x if asked_device == home else x.to(home), self.in_features)
         result = torch.empty(acts.shape[0], self.out_features, dtype=torch.bfloat16, device=home)
         if acts.shape[0] > 0:
-            with torch.cuda.device(home):
+            with on_device(home.index):
                 self._run(acts, result, yf32)
-        if self.bias is not None:
-            result += self.bias
-        result = result.view(*lead, self.out_features)
+        bias = self.bias
+        if bias is not None:
+            result += bias
+        if len(lead) != 1:
+            result = result.view(*lead, self.out_features)
         if asked_dtype != torch.bfloat16:
             result = result.to(asked_dtype)
         return result if asked_device == home else result.to(asked_device)
@@ -414,47 +426,47 @@ def swiglu(self, x):
 TreeLinear.swiglu = swiglu
 
 
-@torch.no_grad()
 def forward_list(layers, x):
     """[layer(x) for layer in layers] for TreeLinear layers that read the same input (q / k / v or gate / up of a
     checkpoint that keeps them as separate trees): up to four layers run as ONE launch over the concatenation of their
     tiles (the GEMV up to GEMV_MAX rows, the tcgen05 GEMM beyond, if every layer has a multiple of 128 rows); anything
     else falls back to one call per layer."""
     first = layers[0]
-    home = first.tree.device
-    same = all(l.in_features == first.in_features and l.tree.device == home for l in layers)
-    lead = x.shape[:-1]
-    acts = _rows_2d(x if x.device == home else x.to(home), first.in_features) if same and home.type == "cuda" else None
-    if acts is None or acts.shape[0] < 1 or not 2 <= len(layers) <= 4:
+    trees = [l._buffers["tree"] for l in layers]
+    home, width = trees[0].device, first.in_features
+    lead, B = x.shape[:-1], x.numel() // width
+    use_gemm = B > min(GEMV_MAX, 32)
+    if (home.type != "cuda" or B < 1 or not 2 <= len(layers) <= 4
+            or any(l.in_features != width or t.device != home for l, t in zip(layers, trees))
+            or (use_gemm and any(l.out_features % 128 for l in layers))):
         return [l(x) for l in layers]
-    use_gemm = acts.shape[0] > min(GEMV_MAX, 32)
-    if use_gemm and any(l.out_features % 128 for l in layers):
-        return [l(x) for l in layers]
-    E, B = ext(), acts.shape[0]
+    here = x.device == home
+    acts = _rows_2d(x if here else x.to(home), width)
     widths = [l.out_features for l in layers]
+    # one allocation, a contiguous [B, width] block per layer
     flat = torch.empty(B * sum(widths), dtype=torch.bfloat16, device=home)
-    outs, at = [], 0
-    for w in widths:
-        outs.append(flat[at:at + B * w].view(B, w))
-        at += B * w
+    parts = flat.split([B * w for w in widths])
     tabs = []
-    for l in layers:
+    for l, t in zip(layers, trees):
         eo, el, eb = l.tables()
-        tabs.append((l.tree, eo, eb, el))
-    with torch.cuda.device(home):
+        tabs.append((t, eo, eb, el))
+    E = ext()
+    with on_device(home.index):
+        st = _state(home)
+        args = E.gemv_list_args(tabs, parts)
         if use_gemm:
-            E.gemm_list(E.gemv_list_args(tabs, outs), acts, _state(home).get_cnt((sum(widths) // 128) * ((B + 255) // 256)))
+            E.gemm_list(args, acts, st.get_cnt((sum(widths) // 128) * ((B + 255) // 256)))
         else:
-            ws = _state(home).get_ws(E.gemv_list_workspace_bytes(widths, first.in_features, B))
-            E.gemv_list(E.gemv_list_args(tabs, outs), acts, ws)
+            E.gemv_list(args, acts, st.gemv_ws(tuple(widths), width, B))
     res = []
-    for l, y in zip(layers, outs):
-        if l.bias is not None:
-            y += l.bias
-        y = y.view(*lead, l.out_features)
+    for l, y, w in zip(layers, parts, widths):
+        y = y.view(*lead, w)
+        bias = l.bias
+        if bias is not None:
+            y += bias
         if x.dtype != torch.bfloat16:
             y = y.to(x.dtype)
-        res.append(y if x.device == home else y.to(x.device))
+        res.append(y if here else y.to(x.device))
     return res
 
 

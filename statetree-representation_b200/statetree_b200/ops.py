@@ -107,14 +107,34 @@ def _ptr(t):
     return t.data_ptr()
 
 
+class _Here:
+    """the context of a call on the device that is current already: nothing to switch (torch.cuda.device costs ~2 us)"""
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE_CTX = _Here()
+# handle of the current stream of a device, without building a torch.cuda.Stream object for it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+
+
+def on_device(index):
+    """context in which device `index` is current"""
+    return _HERE_CTX if torch.cuda.current_device() == index else torch.cuda.device(index)
+
+
 def _ctx(t):
     if not t.is_cuda:
         raise RuntimeError("statetree_b200: the kernels take CUDA tensors only (no CPU path)")
-    return torch.cuda.device(t.device)
+    return on_device(t.get_device())
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.get_device())
 
 
 def _check(rc):
@@ -125,6 +145,17 @@ def _check(rc):
 def device_status():
     """0 unless a kernel gave up on one of its bounded waits since the last call (synchronises)"""
     return int(lib().st_device_status())
+
+
+class _ArrayTypes(dict):
+    """(pointer array, int64 array) types of n entries"""
+
+    def __missing__(self, n):
+        self[n] = (ctypes.c_void_p * n, ctypes.c_int64 * n)
+        return self[n]
+
+
+_ARRAYS = _ArrayTypes()
 
 
 class _Weights:
@@ -197,7 +228,7 @@ class _Weights:
 
     @staticmethod
     def gemv_list_workspace_bytes(Ms, N, B):
-        arr = (ctypes.c_int64 * len(Ms))(*Ms)
+        arr = _ARRAYS[len(Ms)][1](*Ms)
         return int(lib().st_gemv_list_workspace_bytes(len(Ms), arr, N, B))
 
     @staticmethod
@@ -205,11 +236,11 @@ class _Weights:
         """host pointer arrays of a list call: tabs = [(T, EO, EB, EL), ...] (1 to 4 matrices that share their column
         count), Ys = their outputs [B, M_i].  Build once for fixed buffers, pass to gemv_list on every call."""
         n = len(tabs)
-        VP = ctypes.c_void_p * n
-        cols = [VP(*[_ptr(t[k]) for t in tabs]) for k in range(4)]
+        VP, I64 = _ARRAYS[n]
+        cols = [VP(*[_ptr(t) for t in col]) for col in zip(*tabs)]
         ys = VP(*[_ptr(y) for y in Ys])
         yf = VP(*[_ptr(y) for y in Yf32s]) if Yf32s is not None else None
-        Ms = (ctypes.c_int64 * n)(*[t[0].shape[0] * 16 for t in tabs])
+        Ms = I64(*[t[0].shape[0] * 16 for t in tabs])
         return (n, cols[0], cols[1], cols[2], cols[3], ys, yf, Ms, tabs[0][0].shape[1] * 64, tabs[0][0].device)
 
     @staticmethod
@@ -219,9 +250,9 @@ class _Weights:
         B = X.shape[0]
         if X.shape[1] != N or not X.is_contiguous():
             raise RuntimeError(f"gemv_list: X must be contiguous [B, {N}]")
-        with torch.cuda.device(dev):
+        with on_device(dev.index):
             _check(lib().st_gemv_list(n, t, eo, eb, el, _ptr(X), ys, yf, B, Ms, N, _ptr(WS),
-                                      WS.numel() * WS.element_size(), torch.cuda.current_stream(dev).cuda_stream))
+                                      WS.numel() * WS.element_size(), _raw_stream(dev.index)))
 
     @staticmethod
     def gemm_list(args, X, CNT):
@@ -230,9 +261,8 @@ class _Weights:
         B = X.shape[0]
         if X.shape[1] != N or not X.is_contiguous():
             raise RuntimeError(f"gemm_list: X must be contiguous [B, {N}]")
-        with torch.cuda.device(dev):
-            _check(lib().st_gemm_list(n, t, eo, el, _ptr(X), ys, yf, B, Ms, N, _ptr(CNT),
-                                      torch.cuda.current_stream(dev).cuda_stream))
+        with on_device(dev.index):
+            _check(lib().st_gemm_list(n, t, eo, el, _ptr(X), ys, yf, B, Ms, N, _ptr(CNT), _raw_stream(dev.index)))
 
     @staticmethod
     def gemv_prenorm_supported(M, N, B, act=False):
