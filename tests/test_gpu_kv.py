@@ -416,3 +416,36 @@ def test_attention_split_counts_and_both_cta_sizes(B, heads, splits):
         assert float((out[b].double() - ref).norm() / ref.norm()) < 2.0 ** -9 * 1.1, b
     from statetree_b200 import ops
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("H,N,pad,first", [(1, 16, 0, 0), (2, 1040, 0, 0), (8, 2000, 0, 5), (2, 1100, 8, 0), (2, 1100, 2, 0), (3, 1024, 24, 16)])
+def test_whole_page_append_equals_the_oracle(H, N, pad, first):
+    """whole pages of consecutive tokens (encoded four rows at a time) beside partial pages at both ends and a hole, token
+    strides of every alignment, few and many escapes (the pool chain), the pages written twice
+    with their chains kept: pages and the values read back equal the oracle's"""
+    from statetree_b200.kvcache import PageStore
+    nb = (first + N + 15) // 16 + 1
+    Kb, Vb = G.kv_tokens(N, H, seed=N + H, tiny=0.02)
+    Kb[N // 2:] = G.kv_tokens(N, H, seed=N, tiny=0.3)[0][N // 2:]                # crowded records: 11 slots overflow
+    slots = (np.arange(N) + first).astype(np.int64)
+    if N > 64:
+        slots[48 - first:64 - first] = -1                                        # a page that is not stored (one call writes one
+                                                                                 # run of rows per page: its warp owns the page)
+    wide = [torch.zeros(N, H * D + pad, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    for w, b in zip(wide, (Kb, Vb)):
+        w[:, :H * D] = bits_to_torch(b, DEV).view(N, H * D)
+    K, V = (w[:, :H * D].view(N, H, D) for w in wide)
+    store = PageStore(nb, H, DEV, pool_blocks=1 << 17)
+    o = (np.zeros((nb, H, 2, 2, 1600), np.uint8), np.zeros((1 << 17, 16), np.uint32), np.zeros(2, np.int32))
+    for reuse in (False, True):
+        store.append(K, V, torch.from_numpy(slots).to(DEV), reuse)
+        oracle.kv_append(Kb, Vb, slots, *o, reuse=reuse)
+        got = store.pages.cpu().numpy()
+        assert np.array_equal(got[..., :1552], o[0][..., :1552]), reuse
+        assert np.array_equal(got[..., 1552] & 31, o[0][..., 1552] & 31) and np.array_equal(got[..., 1556:], o[0][..., 1556:])
+        Kd, Vd = store.dense()
+        live = torch.from_numpy(slots[slots >= 0]).to(DEV)
+        keep = torch.from_numpy(slots >= 0).to(DEV)
+        for dense, src in ((Kd, K), (Vd, V)):
+            assert torch.equal(dense.view(-1, H, D)[live].view(torch.int16), src[keep].view(torch.int16)), reuse
+    store.check()                                                                # (the pool held everything)
