@@ -209,14 +209,30 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
     }
   }
 
-  if (tid == 0) {
-    for (int s = 0; s < SA; ++s) { mbar_init(aready + s, NDEC); mbar_init(aempty + s, 1); }
-    for (int s = 0; s < SX; ++s) { mbar_init(xfull + s, 1); mbar_init(xempty + s, 1); }
-    for (int r = 0; r < R; ++r) { mbar_init(rfull + r, 1); mbar_init(rempty + r, NDEC); }
-    mbar_init(accbar, 1);
+  // Set-up, spread over the role warps.  The record producer prepares the barriers (a lane each) and sends the first ring
+  // fill off before the block synchronises: weights depend on no earlier kernel.
+  auto load_records = [&](int i, int r) {
+    // one tiled TMA load per pair of k-tiles fetches sixteen records (row tiles rb * 8 .. + 7, column groups k0 + 2 i and
+    // + 1) through a 3-D view of the tree [row tile][column group][194 x u64]; separate bulk copies would cost far more
+    if (elect_one()) {
+      mbar_expect_tx(rfull + r, (uint32_t)RAW_SLOT);
+      tma_load_3d(rawring + (size_t)r * RAW_SLOT, wm, 0, k0 + PAIR * i, lrb * 8, rfull + r);
+    }
+    __syncwarp();
+  };
+  if (warp == W_RAW) {
+    if (!GROUPED && elect_one()) asm volatile("prefetch.tensormap [%0];" :: "l"(wm) : "memory");
+    for (int b = lane; b < 2 * (SA + SX + R) + 1; b += 32) {
+      int count = 1;                                             // aempty, xfull, xempty, rfull, accbar
+      if (b < SA || (b >= 2 * (SA + SX) + R && b < 2 * (SA + SX + R))) count = NDEC;   // aready, rempty: one arrival per decode warp
+      mbar_init(aready + b, count);
+    }
     fence_barrier_init();
-  }
-  if (warp == W_MMA) {
+    __syncwarp();
+    for (int i = 0; i < min(np, R); ++i) load_records(i, i);
+  } else if (warp == W_X) {
+    if (elect_one()) asm volatile("prefetch.tensormap [%0];" :: "l"(&xmap) : "memory");
+  } else if (warp == W_MMA) {
     tmem_alloc(tmem_slot, (uint32_t)a.tmem_cols);
     tmem_relinquish();
   }
@@ -233,16 +249,10 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   pdl_launch_dependents();
 
   if (warp == W_RAW) {
-    // ---------------------------------------------------------------- record producer: one tiled TMA load per pair of
-    // k-tiles fetches sixteen records (row tiles rb * 8 .. + 7, column groups k0 + 2 i and + 1) through a 3-D view of the
-    // tree [row tile][column group][194 x u64]; separate bulk copies would cost far more issue time
-    for (int i = 0, r = 0, k = 0; i < np; ++i, r = (r + 1 == R ? 0 : r + 1), k += (r == 0)) {
-      if (k > 0 && !GW(rempty + r, (uint32_t)(k - 1) & 1u)) { if (lane == 0) atomicExch(a.status, ERR_WAIT_EMPTY); break; }
-      if (elect_one()) {
-        mbar_expect_tx(rfull + r, (uint32_t)RAW_SLOT);
-        tma_load_3d(rawring + (size_t)r * RAW_SLOT, wm, 0, k0 + PAIR * i, lrb * 8, rfull + r);
-      }
-      __syncwarp();
+    // ---------------------------------------------------------------- record producer, behind the first ring fill
+    for (int i = R, r = 0, k = 1; i < np; ++i, r = (r + 1 == R ? 0 : r + 1), k += (r == 0)) {
+      if (!GW(rempty + r, (uint32_t)(k - 1) & 1u)) { if (lane == 0) atomicExch(a.status, ERR_WAIT_EMPTY); break; }
+      load_records(i, r);
     }
   } else if (warp == W_X) {
     // ---------------------------------------------------------------- activation producer.  The activations are the
@@ -602,6 +612,9 @@ GemmPlan gemm_plan(long long M, long long N, long long B) {
     int best = 1;
     t = 1e30;
     for (int ks = 1; ks <= ksmax; ++ks) {
+#ifdef ST_TUNE                                                   // development builds may force a split
+      if (const char* f = getenv("STATETREE_GEMM_KS")) if (atoi(f) > 0 && atoi(f) != ks) continue;
+#endif
       const double e = estimate(rows, ks);
       if (e < t - 1e-9) { t = e; best = ks; }
     }

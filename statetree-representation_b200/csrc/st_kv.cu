@@ -530,10 +530,11 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_attn_kernel(const AttnLau
     fence_barrier_init();
   }
   const uint64_t stream_policy = policy_evict_first();
-  pdl_launch_dependents();
   pdl_wait();                               // queries, lengths and this step's pages come from earlier kernels
+  pdl_launch_dependents();
 
-  // ---- Q^T as the B operand: lane (g, t) holds head g, dims 16 ks + 2t, +1 and 16 ks + 8 + 2t, +1 (requested first: the
+  const int len = a.seq_len[seq], start = a.seq_start ? a.seq_start[seq] : 0;
+  // ---- Q^T as the B operand: lane (g, t) holds head g, dims 16 ks + 2t, +1 and 16 ks + 8 + 2t, +1 (requested here: the
   // loads run beside the chain length -> block table -> page)
   uint32_t qf[8][2];
   {
@@ -545,7 +546,6 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_attn_kernel(const AttnLau
     }
   }
   // ---- this warp's pages
-  const int len = a.seq_len[seq], start = a.seq_start ? a.seq_start[seq] : 0;
   const int first_page = start / PAGE;
   const int end_page = len > start ? (int)min((long long)(len + PAGE - 1) / PAGE, a.table_stride) : 0;
   const int per_split = max(a.min_pages, (end_page - first_page + a.splits - 1) / a.splits);
@@ -705,20 +705,23 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_attn_kernel(const AttnLau
   }
 }
 
-// One CTA of four warps per (sequence, query head): weighs the split partials by exp2(m_j - max m) and normalises.  Latency
-// bounds it (a few KB per row), so nothing is loaded inside a dependent loop: lane j of every warp takes (m, l) of split j,
-// and warp w has the partials of its splits w, w + 4, ... (eight at a time) in flight together.  32 rows x 32 splits:
-// 2 us behind the attention kernel; one warp per row walking the splits one after the other took 9 us.
+// Weighs the split partials of a (sequence, query head) by exp2(m_j - max m) and normalises.  Latency bounds it (a few KB per
+// row), so nothing is loaded inside a dependent loop: lane j takes (m, l) of split j, and the partials are requested four
+// or eight at a time.  WPR warps share a row: four when there are more than four splits (32 rows x 32 splits: 2 us behind the
+// attention kernel; one warp per row walking the splits one after the other took 9 us; 448 rows x 7 splits 1.8 us faster than
+// with one warp), one otherwise (64 sequences x 64 heads x 2 splits: four warps per row 1.6 us slower).
 constexpr int MERGE_WARPS = 4;
+template <int WPR>
 __global__ void __launch_bounds__(MERGE_WARPS * 32) kv_merge_kernel(const float* __restrict__ part_o,
                                                                     const float* __restrict__ part_ml,
                                                                     uint16_t* __restrict__ out, long long out_stride, int Hq,
-                                                                    int splits) {
+                                                                    int splits, long long rows) {
   __shared__ float4 s_num[MERGE_WARPS][32];
   pdl_wait();
   pdl_launch_dependents();
-  const long long row = blockIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % WPR;
+  const long long row = (long long)blockIdx.x * (MERGE_WARPS / WPR) + warp / WPR;
+  if (row >= rows) return;                         // (WPR = 4: one row per CTA, never beyond)
   const float* ml = part_ml + row * splits * 2;
   const float4* po = reinterpret_cast<const float4*>(part_o) + row * splits * (HD / 4) + lane;
   float top = -INFINITY;
@@ -732,27 +735,32 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) kv_merge_kernel(const float*
     if (c + lane < splits) { m = ml[2 * (c + lane)]; l = ml[2 * (c + lane) + 1]; }
     const float f = m == -INFINITY ? 0.f : exp2f(m - top);           // (a split without tokens weighs nothing)
     den += f * l;
-    float4 o[32 / MERGE_WARPS];
+    constexpr int U = WPR == 1 ? 4 : 8;
+    for (int k0 = 0; k0 < 32 && c + k0 < splits; k0 += U * WPR) {
+      float4 o[U];
 #pragma unroll
-    for (int k = 0; k < 32 / MERGE_WARPS; ++k) {
-      const int j = c + warp + MERGE_WARPS * k;
-      o[k] = j < splits ? po[(size_t)j * (HD / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+      for (int k = 0; k < U; ++k) {
+        const int j = c + k0 + sub + WPR * k;
+        o[k] = j < splits ? po[(size_t)j * (HD / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
 #pragma unroll
-    for (int k = 0; k < 32 / MERGE_WARPS; ++k) {
-      const float fj = __shfl_sync(FULL, f, warp + MERGE_WARPS * k);
-      num.x += fj * o[k].x; num.y += fj * o[k].y; num.z += fj * o[k].z; num.w += fj * o[k].w;
+      for (int k = 0; k < U; ++k) {
+        const float fj = __shfl_sync(FULL, f, k0 + sub + WPR * k);
+        num.x += fj * o[k].x; num.y += fj * o[k].y; num.z += fj * o[k].z; num.w += fj * o[k].w;
+      }
     }
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) den += __shfl_xor_sync(FULL, den, o);
-  s_num[warp][lane] = num;
-  __syncthreads();
-  if (warp != 0) return;
+  if (WPR > 1) {
+    s_num[warp][lane] = num;
+    __syncthreads();
+    if (sub != 0) return;
 #pragma unroll
-  for (int w = 1; w < MERGE_WARPS; ++w) {           // the warps in order: one fixed summation order
-    const float4 o = s_num[w][lane];
-    num.x += o.x; num.y += o.y; num.z += o.z; num.w += o.w;
+    for (int w = 1; w < WPR; ++w) {                 // the warps in order: one fixed summation order
+      const float4 o = s_num[warp + w][lane];
+      num.x += o.x; num.y += o.y; num.z += o.z; num.w += o.w;
+    }
   }
   const float inv = den > 0.f ? 1.f / den : 0.f;
   uint2 packed;
@@ -876,8 +884,12 @@ extern "C" int st_kv_attn(const void* q, int64_t qs, int64_t B, int64_t Hq, cons
   // 75 / 68, would gain, but the lengths are not known here).
   const int e = B * Hkv * S <= 2ll * st::sm_count() ? attn_launch<8, 2>(a, (int)B, st_) : attn_launch<4, 2>(a, (int)B, st_);
   if (e) return e;
-  if (S > 1)
-    return st::launch("st_kv_attn merge launch", kv_merge_kernel, dim3((unsigned)(B * Hq)), dim3(MERGE_WARPS * 32), 0, st_,
-                      (const float*)wo, (const float*)wml, (uint16_t*)out, (long long)os, (int)Hq, (int)S);
+  if (S > 1) {
+    const long long rows = B * Hq;
+    const int per_cta = S > 4 ? 1 : MERGE_WARPS;
+    return st::launch("st_kv_attn merge launch", S > 4 ? kv_merge_kernel<MERGE_WARPS> : kv_merge_kernel<1>,
+                      dim3((unsigned)((rows + per_cta - 1) / per_cta)), dim3(MERGE_WARPS * 32), 0, st_, (const float*)wo,
+                      (const float*)wml, (uint16_t*)out, (long long)os, (int)Hq, (int)S, rows);
+  }
   return 0;
 }

@@ -25,6 +25,11 @@ GEMV_AR_MAX = 12                    # rows up to which the GEMV that sums over t
 # it, the reference's path above 1024 rows (statetree/linear.py:37, 879-886), here from the size at which it overtakes the
 # tcgen05 kernel; 0 turns it off
 PREFILL_MIN = int(os.environ.get("STATETREE_PREFILL_MIN", "512"))
+# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel up to FUSED_ROWS rows: two layers of a
+# 4096 / 12288 model called in turn, us with the tcgen05 kernel / the scratch matrix: 700 rows 567 / 751, 1000 747 / 784,
+# 1500 1006 / 986, 2000 1351 / 1426, 3000 1906 / 1685, 4096 2544 / 2217.  (Smaller matrices take less time than their launches
+# on either path and keep the lower line.)
+FUSED_ROWS, FUSED_WEIGHTS = 2048, 1 << 22
 DENSE_MAX = 1 << 28                 # weights: larger matrices (vocabulary-sized tables) never get a dense scratch copy
 _STATES = {}
 _BUFFERS = ("tree", "esc_rows", "esc_cols", "esc_bits")
@@ -134,7 +139,7 @@ class _DenseStage:
         other = 1 - slot
         nxt = layer._next() if layer._next is not None else None
         fork = None
-        if (nxt is not None and nxt.dense_ok() and nxt.tree.device == layer.tree.device
+        if (nxt is not None and nxt.dense_for(x.shape[0]) and nxt.tree.device == layer.tree.device
                 and self.holds[other] != self._ident(nxt)):
             nxt.tables()                                     # built on the caller's stream, before the fork
             Wn = self._matrix(other, nxt)
@@ -301,6 +306,11 @@ class TreeLinear(nn.Module):
         """may this layer be decoded into a BF16 scratch matrix for prefill-size batches"""
         return self.allow_dec and self.tree.is_cuda and self.out_features * self.in_features <= DENSE_MAX
 
+    def dense_for(self, B):
+        """do B rows go through the scratch matrix"""
+        M, N = self.out_features, self.in_features
+        return 0 < PREFILL_MIN < B and not (B <= FUSED_ROWS and M * N >= FUSED_WEIGHTS and M % 128 == 0) and self.dense_ok()
+
     def extra_repr(self):
         return (f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}, "
                 f"escapes={self.esc_rows.numel()}, bits_per_weight={self.bits_per_weight:.3f}")
@@ -353,7 +363,7 @@ class TreeLinear(nn.Module):
         st = _state(x.device)
         if B <= min(GEMV_MAX, 32):
             E.gemv(self._buffers["tree"], eo, eb, el, x, y, st.gemv_ws(M, N, B), st.get_cnt(M // 16), yf32)
-        elif 0 < PREFILL_MIN < B and yf32 is None and self.dense_ok() and not torch.cuda.is_current_stream_capturing():
+        elif self.dense_for(B) and yf32 is None and not torch.cuda.is_current_stream_capturing():
             st.dense_stage().run(self, x, y)                # decode once + cuBLAS, the next layer decoded meanwhile
         elif M % 128 == 0:
             ws = st.get_scratch(E.gemm_workspace_bytes(M, N, B))

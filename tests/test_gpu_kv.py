@@ -382,7 +382,8 @@ def test_vllm_page_backend_data_path():
 
 
 @pytest.mark.parametrize("B,heads,splits", [(1, 2, 1), (1, 8, 2), (2, 2, 5), (3, 14, 31), (1, 16, 32), (2, 4, 33), (1, 2, 64),
-                                            (1, 6, 70), (40, 8, 4), (80, 2, 2)])
+                                            (1, 6, 70), (40, 8, 4), (80, 2, 2), (3, 2, 4),
+                                            (3, 2, 9)])
 def test_attention_split_counts_and_both_cta_sizes(B, heads, splits):
     """merge of 1 to 70 split partials (below, at and beyond the 32 of one pass; splits without tokens among them), grids of
     up to two CTAs per SM (eight warps each) and above it (four warps), an empty sequence, sequences that start late"""

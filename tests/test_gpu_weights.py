@@ -454,3 +454,35 @@ def test_encode_kernels_equal_the_torch_formulation(M, N, regime):
     bits[M - 1, N - 1] ^= 1
     layer = TreeLinear.from_weight(Wd)
     assert torch.equal(layer.dequantize().view(torch.int16), bits)
+
+
+@pytest.mark.parametrize("M,B", [(128 * 149, 20), (128 * 192, 64), (128 * 230, 17), (128 * 290, 33)])
+def test_gemm_row_blocks_beyond_one_per_sm(M, B):
+    """more row blocks than SMs, fewer than twice as many: the product goes out as two launches side by side; the activations
+    come from the kernel right before it in the stream and the result is read by the one right after it"""
+    from statetree_b200 import TreeLinear, ops
+    N = 1024
+    g = torch.Generator(DEV).manual_seed(M + B)
+    W = (torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+    W[:, 5] *= 4096                                                             # escapes
+    tl = TreeLinear.from_weight(W)
+    x = torch.randn(B, N, device=DEV, generator=g).to(torch.bfloat16)
+    want = x.double() @ W.double().t()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        tl(x)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            src = x * 1.0
+            for _ in range(3):
+                y = tl(src)
+                src = src + y[:, :N] * 0.0                                      # depends on the whole chain before it
+            out = y.float() * 1.0
+        for _ in range(3):
+            graph.replay()
+    side.synchronize()
+    assert torch.equal(out, tl(x).float())
+    assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1  # BF16 results: half an ulp each
+    assert ops.device_status() == 0
