@@ -192,6 +192,13 @@ int st_qk_norm_rope(const void* qkv, int64_t row_stride, const void* wq, const v
                     const float* sin_t, const int64_t* pos, int64_t max_pos, void* q_out, void* k_out, int64_t B,
                     int64_t hq, int64_t hkv, double eps, void* stream);
 
+/* Start of a decode step of B sequences that all hold cum[0] tokens: slots int64 [B] = table[b, page] * 16 + row of the new
+ * token (table int64 [B, max_pages]; -1 once max_len tokens are stored), lens int32 [B] = tokens with the new one. */
+int st_decode_slots(const int64_t* cum, const int64_t* table, int64_t max_pages, int64_t max_len, int64_t B, int64_t* slots,
+                    int32_t* lens, void* stream);
+/* out int64 [rows] = index of the largest value of each BF16 row [V], V % 8 == 0 (ties: the lower index; NaN is largest). */
+int st_argmax(const void* x, int64_t rows, int64_t V, int64_t* out, void* stream);
+
 /* ---- KV pages --------------------------------------------------------------------------------------------------- */
 /* 6400 * H.  Replaces `_kv.page_bytes` (statetree/csrc/kvcache.cu:295). */
 int64_t st_kv_page_bytes(int64_t H);

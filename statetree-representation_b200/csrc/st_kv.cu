@@ -387,11 +387,15 @@ __device__ __forceinline__ void apply_kv_escapes(uint32_t (&A)[4][4], const uint
   }
 }
 
-// listed pages (blocks != nullptr) or every page -> dense BF16 [n, 16, H, 128]; one warp per unit
+// listed pages (blocks != nullptr) or every page -> dense BF16 [n, 16, H, 128]; one warp per unit.  VEC: the fragments are
+// transposed through shared memory so that every row leaves as a full 128-byte line of 16-byte stores (outputs 16-byte
+// aligned); otherwise they are stored from registers, 4 bytes per lane (8192 tokens x 8 heads: 13.3 us, VEC 8.2).
+template <bool VEC>
 __global__ void __launch_bounds__(256) kv_dequant_kernel(const uint8_t* __restrict__ kv, long long nblocks, int H,
                                                          const uint32_t* __restrict__ pool, int P,
                                                          const int* __restrict__ blocks, long long n,
                                                          uint16_t* __restrict__ Kd, uint16_t* __restrict__ Vd) {
+  __shared__ __align__(16) uint8_t tile[VEC ? 8 : 1][16 * 144];  // row stride 144 B: conflict-free both ways
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (w >= n * H * 4) return;
@@ -412,6 +416,21 @@ __global__ void __launch_bounds__(256) kv_dequant_kernel(const uint8_t* __restri
       for (int q = 0; q < 4; ++q) A[s][q] = 0u;
   }
   uint16_t* out = (kvi ? Vd : Kd) + ((size_t)i * PAGE * H + h) * HD + half * 64;
+  if (VEC) {
+    uint8_t* const my = tile[threadIdx.x >> 5];
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint32_t*>(my + (g + 8 * (q & 1)) * 144 + (16 * s + 8 * (q >> 1) + 2 * t) * 2) = A[s][q];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = 4 * k + (lane >> 3), seg = lane & 7;
+      *reinterpret_cast<uint4*>(out + (size_t)row * H * HD + seg * 8) = *reinterpret_cast<const uint4*>(my + row * 144 + seg * 16);
+    }
+    return;
+  }
 #pragma unroll
   for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -842,7 +861,8 @@ extern "C" int st_kv_dequant_blocks(const void* kv, int64_t nblocks, int64_t H, 
   ST_REQUIRE(kv && pool && Kd && Vd, "st_kv_dequant_blocks: null pointer");
   ST_REQUIRE(st::aligned16(kv) && ((uintptr_t)Kd & 3u) == 0 && ((uintptr_t)Vd & 3u) == 0, "st_kv_dequant_blocks: alignment");
   const long long nw = n * H * 4;
-  kv_dequant_kernel<<<(unsigned)((nw + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
+  auto* kernel = st::aligned16(Kd) && st::aligned16(Vd) ? kv_dequant_kernel<true> : kv_dequant_kernel<false>;
+  kernel<<<(unsigned)((nw + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
       (const uint8_t*)kv, nblocks, (int)H, pool, (int)P, blocks, n, (uint16_t*)Kd, (uint16_t*)Vd);
   ST_LAUNCH_CHECK("st_kv_dequant launch");
   return 0;

@@ -301,6 +301,13 @@ class TreeDecoder:
         self.pos_buf += 1
         return logits
 
+    def _pick(self, logits):
+        """greedy: next_tok = argmax of every row"""
+        if self.compressed and logits.is_contiguous() and logits.shape[1] % 8 == 0 and logits.data_ptr() % 16 == 0:
+            ext().argmax(logits, self.next_tok)
+        else:
+            self.next_tok.copy_(logits.argmax(-1))
+
     def capture(self):
         from .kvcache import decode_splits
         self.splits = decode_splits(self.B, self.hkv, (self.max_len + 15) // 16) if self.compressed else 1
@@ -309,14 +316,14 @@ class TreeDecoder:
         side.wait_stream(torch.cuda.current_stream(self.dev))      # weights and buffers were written on that stream
         with torch.cuda.stream(side):
             for _ in range(2):                                   # warm-up steps (also sizes every workspace)
-                self.next_tok.copy_(self._step().argmax(-1))
+                self._pick(self._step())
         side.synchronize()
         self.reset()
         torch.cuda.synchronize(self.dev)
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=side):
             logits = self._step()
-            self.next_tok.copy_(logits.argmax(-1))
+            self._pick(logits)
         self.logits = logits
         self.reset()
         torch.cuda.synchronize(self.dev)

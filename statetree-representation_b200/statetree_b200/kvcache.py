@@ -117,6 +117,10 @@ class PagedKVCache:
     def begin_step(self, B):
         """decode step (one token per sequence): the slots every layer appends at, computed once; lens counts the new
         token.  Graph-safe (positions come from the GPU-side count)."""
+        if self.cum.is_cuda and B <= self.B:
+            slots = torch.empty(B, dtype=torch.long, device=self.cum.device)
+            kv_ext().decode_slots(self.cum, self.bt64[:B], self.max_len, slots, self.lens)
+            return slots
         page = (self.cum // PAGE).clamp(max=self.max_pages - 1)            # a full cache never indexes past the table:
         slots = self.bt64[:B].gather(1, page.expand(B, 1)).view(B) * PAGE + self.cum % PAGE
         slots = torch.where(self.cum < self.max_len, slots, torch.full_like(slots, -1))   # ... the token is dropped

@@ -269,7 +269,8 @@ class TreeLinear(nn.Module):
             if not same:
                 raise RuntimeError("TreeLinear: the tree does not decode to the weights it was built from")
         if on_gpu:                                      # (see tables(): complete before any later kernel may start)
-            torch.cuda.current_stream(W.device).synchronize()
+            if not verify:                              # (the check has synchronised)
+                torch.cuda.current_stream(W.device).synchronize()
             layer._tables = tables
         return layer
 

@@ -23,6 +23,8 @@ _SIGNATURES = {
     "st_device_status": (_int, []),
     "st_dec": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp]),
     "st_rows": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _i64, _vp, _vp]),
+    "st_decode_slots": (_int, [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp]),
+    "st_argmax": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "st_encode": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "st_encode_lists": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "st_dec_check": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
@@ -400,6 +402,12 @@ class _Weights:
                                          cos_t.shape[0], _ptr(q_out), _ptr(k_out), B, hq, hkv, float(eps), _stream(qkv)))
 
     @staticmethod
+    def argmax(x, out):
+        """out int64 [rows] = index of the largest value of each row of x [rows, V] BF16, V % 8 == 0"""
+        with _ctx(x):
+            _check(lib().st_argmax(_ptr(x), x.shape[0], x.shape[1], _ptr(out), _stream(x)))
+
+    @staticmethod
     def silu_mul(gu, act):
         S, I2 = gu.shape
         with _ctx(gu):
@@ -418,6 +426,13 @@ class _KV:
             _check(lib().st_rope_kv_append(_ptr(qkv), qkv.stride(0), _ptr(wq), _ptr(wk), _ptr(cos_t), _ptr(sin_t),
                                            _ptr(pos), cos_t.shape[0], _ptr(q_out), B, hq, hkv, float(eps), _ptr(slot),
                                            _ptr(kv), kv.size(0), _ptr(pool), pool.size(0), _ptr(pool_cnt), _stream(qkv)))
+
+    @staticmethod
+    def decode_slots(cum, table, max_len, slots, lens):
+        """slots [B] and lens [B] of a decode step from the device-side token count"""
+        with _ctx(cum):
+            _check(lib().st_decode_slots(_ptr(cum), _ptr(table), table.shape[1], max_len, slots.numel(), _ptr(slots),
+                                         _ptr(lens), _stream(cum)))
 
     @staticmethod
     def version():

@@ -450,3 +450,31 @@ def test_whole_page_append_equals_the_oracle(H, N, pad, first):
         for dense, src in ((Kd, K), (Vd, V)):
             assert torch.equal(dense.view(-1, H, D)[live].view(torch.int16), src[keep].view(torch.int16)), reuse
     store.check()                                                                # (the pool held everything)
+
+
+@pytest.mark.parametrize("rows,V", [(1, 8), (4, 32768), (3, 151936), (2, 4104), (70, 64)])
+def test_argmax_and_decode_slots_equal_torch(rows, V):
+    """argmax against torch on rows with ties, infinities, signed zeros and NaN; the slots of a step against the formula, up
+    to and beyond a full cache"""
+    from statetree_b200.kvcache import PagedKVCache
+    from statetree_b200.ops import ext
+    g = torch.Generator(DEV).manual_seed(V)
+    x = (torch.randn(rows, V, device=DEV, generator=g) * 2).round().to(torch.bfloat16)          # many ties
+    if rows > 1:
+        x[1] = torch.where(x[1] > 0, torch.zeros_like(x[1]), -torch.zeros_like(x[1]))           # +0 and -0 only
+        x[0, V // 2] = float("inf")
+        x[-1, V // 3] = float("nan")
+    out = torch.empty(rows, dtype=torch.long, device=DEV)
+    ext().argmax(x, out)
+    want = torch.stack([torch.nonzero(torch.isnan(r))[0, 0] if bool(torch.isnan(r).any())
+                        else torch.nonzero(r == r.max())[0, 0] for r in x.float()])
+    assert torch.equal(out, want)
+    cache = PagedKVCache(1, min(rows, 5), 50, 1, DEV, pool_blocks=8)
+    B = min(rows, 5)
+    for n in (0, 1, 15, 16, 47, 63, 64, 70):
+        cache.cum.fill_(n)
+        slots = cache.begin_step(B)
+        page = min(n // 16, cache.max_pages - 1)
+        full = n >= cache.max_len
+        assert slots.tolist() == [-1 if full else (b * cache.max_pages + page) * 16 + n % 16 for b in range(B)], n
+        assert cache.lens[:B].tolist() == [min(n + 1, cache.max_len)] * B
