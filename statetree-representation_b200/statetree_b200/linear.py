@@ -174,6 +174,8 @@ def _state(device):
 def _rows_2d(x, width):
     """x [..., width] of any float dtype / layout -> BF16 [rows, width], contiguous and 16-byte aligned"""
     flat = x.reshape(-1, width)
+    if x.shape[-1] != width and flat.shape[0] != x.shape[:-1].numel():    # (a multiple or a divisor of the width)
+        raise RuntimeError(f"statetree_b200: the layer takes inputs of {width} columns, got {tuple(x.shape)}")
     if flat.dtype != torch.bfloat16:
         flat = flat.to(torch.bfloat16)
     if flat.data_ptr() % 16 or not flat.is_contiguous():

@@ -486,3 +486,23 @@ def test_gemm_row_blocks_beyond_one_per_sm(M, B):
     assert torch.equal(out, tl(x).float())
     assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1  # BF16 results: half an ulp each
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,width", [(4, 512), (8, 128), (1, 512), (40, 512), (700, 512)])
+def test_inputs_of_another_width_are_refused(rows, width):
+    """a 2-D (3-D, 1-D) input whose last dimension is a multiple or a divisor of in_features: its values would make up whole
+    rows of in_features, but it is a mis-wired layer and not a batch"""
+    from statetree_b200.linear import forward_list
+    tls = [layer_from_oracle(G.weights(128, 256, seed, "mixed"))[0] for seed in (1, 2)]
+    x = torch.zeros(rows, width, dtype=torch.bfloat16, device=DEV)
+    for bad in (x, x[None], x.float(), x[0] if width > 256 else x.expand(2, rows, width)):
+        with pytest.raises(RuntimeError):
+            tls[0](bad)
+        with pytest.raises(RuntimeError):
+            forward_list(tls, bad)
+    for lead in ((rows,), (2, rows), (1, rows, 1), ()):                         # what fits is taken as before
+        good = torch.zeros(*lead, 256, dtype=torch.bfloat16, device=DEV)
+        assert tls[0](good).shape == (*lead, 128)
+        assert [t.shape for t in forward_list(tls, good)] == [(*lead, 128)] * 2
+    assert tls[0](x[:0]).shape == (0, 128)
+    _status_ok()
