@@ -90,6 +90,26 @@ class _DevState:
         return self.cnt
 
 
+class _Decoded:
+    """What a scratch matrix was decoded from: the tensor that holds the tree, as it was then, and the escape tables of that
+    time.  By weak reference: ids and addresses are given out again, and a matrix must never pass for that of the layer that took
+    the place of another."""
+
+    def __init__(self, layer):
+        tree = layer._buffers["tree"]
+        self.tree, self.eo = weakref.ref(tree), weakref.ref(layer.tables()[0])
+        self.version = None if tree.is_inference() else tree._version
+
+    def __eq__(self, other):
+        if not isinstance(other, _Decoded):
+            return False
+        tree, eo = self.tree(), self.eo()
+        return (tree is not None and tree is other.tree() and eo is not None and eo is other.eo()
+                and self.version == other.version)
+
+    __hash__ = None
+
+
 class _DenseStage:
     """Prefill-size batches: decode once, multiply with cuBLAS (statetree/linear.py:286-368 is the reference's form).
     Two BF16 scratch matrices per (device, stream).  While the GEMM reads one, a side stream decodes the layer linked
@@ -101,14 +121,12 @@ class _DenseStage:
         self.device = device
         self.side = torch.cuda.Stream(device)                # (a high-priority stream measured slower: 17.2 against 14.8 ms at 1024 rows)
         self.mat = [None, None]                              # flat BF16 scratch
-        self.holds = [None, None]                            # identity of the tree decoded into each
+        self.holds = [None, None]                            # _Decoded: what each holds
         self.decoded = [None, None]                          # event: that decode has finished
         self.read = [None, None]                             # event: the last GEMM that read it has finished
         self.turn = 0
 
-    @staticmethod
-    def _ident(layer):
-        return (id(layer), layer.tree.data_ptr(), layer.tree._version)
+    _ident = _Decoded
 
     def _matrix(self, slot, layer):
         need = layer.out_features * layer.in_features

@@ -506,3 +506,51 @@ def test_inputs_of_another_width_are_refused(rows, width):
         assert [t.shape for t in forward_list(tls, good)] == [(*lead, 128)] * 2
     assert tls[0](x[:0]).shape == (0, 128)
     _status_ok()
+
+
+@pytest.mark.parametrize("how", ["new_layers", "moved", "reloaded", "inference_mode"])
+def test_scratch_matrix_is_never_taken_for_another_layers(how):
+    """prefill batches while layers come and go: a layer made where another was freed (same id, same address), one that went
+    to the host and came back with other weights, one whose tree was loaded over, trees made in inference mode"""
+    from statetree_b200 import TreeLinear
+    B, g = 700, torch.Generator(DEV).manual_seed(5)
+    shapes = [(256, 512), (512, 256), (256, 512), (128, 1024)]
+
+    def weight(M, N):
+        W = (torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+        W[:, 5] *= 4096                                                         # escapes
+        return W
+
+    def check(tl, W):
+        x = torch.randn(B, W.shape[1], device=DEV, generator=g).to(torch.bfloat16)
+        want = x.double() @ W.double().t()
+        assert float((tl(x).double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1, how    # BF16 results: half an ulp each
+
+    seen, again = set(), 0
+    tl = TreeLinear.from_weight(weight(256, 512))
+    for i in range(24):
+        if how == "new_layers":
+            W = weight(*shapes[i % 4])
+            tl = None
+            tl = TreeLinear.from_weight(W)
+            again += (id(tl), tl.tree.data_ptr()) in seen
+            seen.add((id(tl), tl.tree.data_ptr()))
+        elif how == "moved":
+            W = weight(256, 512)
+            other = TreeLinear.from_weight(W.cpu())
+            tl.cpu()
+            tl.load_state_dict(other.state_dict())
+            tl.to(DEV)
+        elif how == "reloaded":
+            W = weight(256, 512)
+            tl.load_state_dict(TreeLinear.from_weight(W).state_dict())
+        else:
+            with torch.inference_mode():
+                W = weight(256, 512)
+                tl = TreeLinear.from_weight(W)
+                check(tl, W)
+                continue
+        check(tl, W)
+    if how == "new_layers":
+        assert again > 0                                                        # the case is met
+    _status_ok()
