@@ -9,6 +9,7 @@ semaphores) are kept per (device, stream) because callers may run layers on side
 given at statetree/linear.py:457-466); they are sized once per shape, so steady-state calls allocate only the output.
 """
 import os
+import threading
 import weakref
 
 import torch
@@ -125,6 +126,7 @@ class _DenseStage:
         self.decoded = [None, None]                          # event: that decode has finished
         self.read = [None, None]                             # event: the last GEMM that read it has finished
         self.turn = 0
+        self.lock = threading.Lock()                         # two threads may share a stream, and so this object
 
     _ident = _Decoded
 
@@ -139,6 +141,10 @@ class _DenseStage:
         return self.mat[slot][:need].view(layer.out_features, layer.in_features)
 
     def run(self, layer, x, y):
+        with self.lock:                                      # (the decode and the product that reads it go out together)
+            self._run(layer, x, y)
+
+    def _run(self, layer, x, y):
         cur = torch.cuda.current_stream(self.device)
         me = self._ident(layer)
         if me in self.holds:

@@ -554,3 +554,42 @@ def test_scratch_matrix_is_never_taken_for_another_layers(how):
     if how == "new_layers":
         assert again > 0                                                        # the case is met
     _status_ok()
+
+
+def test_prefill_batches_from_two_threads_on_one_stream():
+    """two threads that call different layers on the same stream share its scratch matrices: a layer's decode and the product that
+    reads it go out together"""
+    import sys
+    import threading
+    from statetree_b200 import TreeLinear
+    g = torch.Generator(DEV).manual_seed(9)
+    B, work = 600, []
+    for M, N in ((256, 512), (512, 256)):
+        tl = TreeLinear.from_weight((torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16))
+        x = torch.randn(B, N, device=DEV, generator=g).to(torch.bfloat16)
+        other = TreeLinear.from_weight((torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16))
+        work.append([(tl, x, tl(x)), (other, x, other(x))])
+    torch.cuda.synchronize()
+    wrong, failed = [], []
+
+    def run(items):
+        try:
+            for _ in range(300):
+                for tl, x, want in items:
+                    if not torch.equal(tl(x), want):
+                        wrong.append(1)
+        except Exception as e:                                                  # noqa: BLE001
+            failed.append(e)
+
+    was = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=run, args=(items,)) for items in work]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(was)
+    assert not failed and not wrong, (failed, len(wrong))
+    _status_ok()
