@@ -52,12 +52,16 @@ int st_rows(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, 
  *                    0, then the escapes of each record (its inclusive prefix sum is eo)
  *   st_encode_lists  given eo and roff int32 [M, N/64] (inclusive prefix sum of rowcnt, row-major): el and eb as above and the
  *                    format's lists rows / cols int32, bits int16 in (row, col) order; n = eo[last] entries each
- * st_dec_check decodes the tree and adds to *bad (int32, zeroed by the caller) for every record that differs from W. */
+ * st_dec_check decodes the tree through eo / el and adds to *bad (int32, zeroed by the caller) for every record that differs
+ * from W; st_lists_check adds to it unless the n stored entries rows / cols / bits are the escapes of W in (row, col) order and
+ * eo / el / eb the tables of those entries.  Both passed: the tree is lossless as it is read now and as it is stored. */
 int st_encode(const void* W, int64_t M, int64_t N, void* tree, uint8_t* rowcnt, int32_t* reccnt, void* stream);
 int st_encode_lists(const void* W, int64_t M, int64_t N, const uint8_t* rowcnt, const int32_t* roff, const int32_t* eo,
                     uint32_t* el, uint32_t* eb, int32_t* rows, int32_t* cols, int16_t* bits, void* stream);
 int st_dec_check(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, int64_t N, const void* W, int32_t* bad,
                  void* stream);
+int st_lists_check(const int32_t* rows, const int32_t* cols, const int16_t* bits, int64_t n, const int32_t* eo,
+                   const uint32_t* el, const uint32_t* eb, int64_t M, int64_t N, const void* W, int32_t* bad, void* stream);
 
 /* Small-batch fused decode + GEMV, 1 <= B <= 32.  Replaces the reference's mv / mvs / mvh / mvc / mvt entry points
  * (statetree/csrc/kernels.cu:243-254, 370-400, 548-599, 771-808; statetree/csrc/hop.cu:993-1019).

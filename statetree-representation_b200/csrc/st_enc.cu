@@ -3,8 +3,8 @@
 //
 // Bound: HBM.  st_encode reads the matrix once (2 B per weight) and writes the records once (1.52 B); the escape passes
 // touch only the records that have escapes.  4096 x 12288 on a B200: st_encode 39 us (177 MB, 4.5 TB/s), the two prefix
-// sums 15 us, st_encode_lists 23 us, st_dec_check 36 us (nothing dense is written back).  TreeLinear.from_weight of that
-// matrix with its check takes 0.22 ms; with the torch formulation (format._encode_chunk, still the CPU path: ~60 passes over
+// sums 15 us, st_encode_lists 23 us, st_dec_check 36 us (nothing dense is written back), st_lists_check 8 us (of the stored lists and the escape blocks).  TreeLinear.from_weight of that
+// matrix with its checks takes 0.24 ms; with the torch formulation (format._encode_chunk, still the CPU path: ~60 passes over
 // 32- and 64-bit copies, then a sort of the escapes and a dense decode to compare) it took 3.7 ms.
 #include "../../include/statetree_b200.h"
 #include "st_encode.cuh"
@@ -110,6 +110,62 @@ __global__ void __launch_bounds__(256) dec_check_kernel(const uint8_t* __restric
   if (__any_sync(FULL, diff != 0u) && lane == 0) atomicAdd(bad, 1);
 }
 
+// Are the lists a checkpoint stores (rows, cols, bits: n entries) the matrix's escapes, and are eo / el / eb the tables those
+// lists give?  dec_check_kernel has shown that the records and the entries that eo and el name decode to W; here every stored
+// entry must lie inside the matrix, follow its predecessor in (row, col) order, hold the matrix's bits and be found in its own
+// record's part of el.  eo partitions n entries, so stored and listed entries are then the same set, and a tree read back
+// from the stored lists decodes to W too.  eb: every word as the unit's part of eo and el gives it.
+// A thread takes one stored entry (a binary search over its record's few entries) and one word of eb.  Nothing is trusted:
+// offsets and positions are checked before they are followed.  4096 x 12288 with 8000 escapes: from_weight 236 -> 244 us.
+__global__ void __launch_bounds__(256) lists_check_kernel(const int* __restrict__ rows, const int* __restrict__ cols,
+                                                          const uint16_t* __restrict__ bits, int n, const int* __restrict__ eo,
+                                                          const uint32_t* __restrict__ el, const uint32_t* __restrict__ eb,
+                                                          long long M, long long N, int NG, int CPT, long long units,
+                                                          const uint16_t* __restrict__ W, int* __restrict__ bad) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  bool ok = true;
+  if (i < n) {
+    const int r = rows[i], c = cols[i];
+    ok = r >= 0 && r < M && c >= 0 && c < N;
+    if (ok && i > 0) ok = rows[i - 1] < r || (rows[i - 1] == r && cols[i - 1] < c);
+    if (ok) {
+      const long long rec = (long long)(r >> 4) * NG + (c >> 6);
+      const uint32_t want = (uint32_t)bits[i] << 16 | (uint32_t)((c >> 6) & 7) << 10 | (uint32_t)(r & 15) << 6 | (uint32_t)(c & 63);
+      int lo = eo[rec], hi = eo[rec + 1];
+      ok = bits[i] == W[(long long)r * N + c] && lo >= 0 && lo < hi && hi <= n;
+      if (ok) {
+        while (hi - lo > 1) {                                    // entries of a record are in (row, col) order: bits 0..9
+          const int mid = (lo + hi) >> 1;
+          if ((el[mid] & 0x3FFu) <= (want & 0x3FFu)) lo = mid;
+          else hi = mid;
+        }
+        ok = el[lo] == want;
+      }
+    }
+  }
+  if (i < units * 16) {
+    const long long u = i >> 4, tile = u / CPT;
+    const int word = (int)(i & 15), G0 = (int)(u % CPT) * 8, nrec = min(8, NG - G0);
+    const int* const off = eo + tile * NG + G0;
+    const int first = off[0], end = off[nrec];
+    bool sound = first >= 0 && first <= end && end <= n && (u > 0 || first == 0) && (u + 1 < units || end == n);
+    uint32_t want = 0u;
+    if (word == 0) {
+      want = (uint32_t)(end - first);
+      for (int k = 0; k < nrec; ++k) {
+        sound = sound && off[k] <= off[k + 1];
+        if (off[k] < off[k + 1]) want |= 1u << (16 + k);
+      }
+    } else if (word == 1) {
+      want = (uint32_t)first;
+    } else if (sound && word - 2 < end - first) {
+      want = el[first + word - 2];
+    }
+    ok = ok && sound && eb[i] == want;
+  }
+  if (__any_sync(FULL, !ok) && (threadIdx.x & 31) == 0) atomicAdd(bad, 1);
+}
+
 int shape_ok(const char* who, int64_t M, int64_t N) {
   ST_REQUIRE(M > 0 && N > 0 && M % 16 == 0 && N % 64 == 0, "%s: M %% 16 and N %% 64 must be 0 (got %lld x %lld)", who,
              (long long)M, (long long)N);
@@ -152,5 +208,19 @@ extern "C" int st_dec_check(const void* tree, const int32_t* eo, const uint32_t*
   dec_check_kernel<<<(unsigned)((nrec + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
       (const uint8_t*)tree, eo, el, nrec, (int)(N / 64), N, (const uint16_t*)W, bad);
   ST_LAUNCH_CHECK("st_dec_check launch");
+  return 0;
+}
+
+extern "C" int st_lists_check(const int32_t* rows, const int32_t* cols, const int16_t* bits, int64_t n, const int32_t* eo,
+                              const uint32_t* el, const uint32_t* eb, int64_t M, int64_t N, const void* W, int32_t* bad,
+                              void* stream) {
+  if (int e = shape_ok("st_lists_check", M, N)) return e;
+  ST_REQUIRE(n >= 0 && n < (1ll << 31), "st_lists_check: number of entries");
+  ST_REQUIRE(eo && el && eb && W && bad && (n == 0 || (rows && cols && bits)), "st_lists_check: null pointer");
+  const int NG = (int)(N / 64), CPT = (NG + 7) / 8;
+  const long long units = (M / 16) * CPT, threads = units * 16 > n ? units * 16 : n;
+  lists_check_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+      rows, cols, (const uint16_t*)bits, (int)n, eo, el, eb, M, N, NG, CPT, units, (const uint16_t*)W, bad);
+  ST_LAUNCH_CHECK("st_lists_check launch");
   return 0;
 }

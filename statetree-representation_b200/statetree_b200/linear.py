@@ -287,8 +287,10 @@ class TreeLinear(nn.Module):
         layer._reset_runtime()
         if verify:
             if on_gpu:
+                # (what is stored is checked, not only the tables of this process: a reload builds its tables from the lists)
                 same = ext().dec_check(enc["tree"], tables[0], tables[1],
-                                       W if W.data_ptr() % 16 == 0 and W.is_contiguous() else W.clone(memory_format=torch.contiguous_format))
+                                       W if W.data_ptr() % 16 == 0 and W.is_contiguous() else W.clone(memory_format=torch.contiguous_format),
+                                       (enc["esc_rows"], enc["esc_cols"], enc["esc_bits"], tables[2]))
             else:
                 back = F.decode_reference(*(layer._buffers[n] for n in _BUFFERS))
                 same = torch.equal(back.view(torch.int16), W.view(torch.int16))

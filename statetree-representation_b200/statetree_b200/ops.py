@@ -28,6 +28,7 @@ _SIGNATURES = {
     "st_encode": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "st_encode_lists": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "st_dec_check": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
+    "st_lists_check": (_int, [_vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
     "st_gemv_workspace_bytes": (_i64, [_i64, _i64, _i64]),
     "st_gemv": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp]),
     "st_gemv_static": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
@@ -194,12 +195,17 @@ class _Weights:
         return tree, rows, cols, bits, (eo, el, eb)
 
     @staticmethod
-    def dec_check(T, EO, EL, W):
-        """does the tree decode to W [M, N] BF16 exactly (synchronises)"""
+    def dec_check(T, EO, EL, W, stored=None):
+        """does the tree decode to W [M, N] BF16 exactly (synchronises).  stored = (rows, cols, bits, EB): the format's lists
+        and the GEMV's escape blocks are checked too"""
         M, N = W.shape
         bad = torch.zeros(1, dtype=torch.int32, device=W.device)
         with _ctx(T):
             _check(lib().st_dec_check(_ptr(T), _ptr(EO), _ptr(EL), M, N, _ptr(W), _ptr(bad), _stream(T)))
+            if stored is not None:
+                rows, cols, bits, EB = stored
+                _check(lib().st_lists_check(_ptr(rows), _ptr(cols), _ptr(bits), rows.numel(), _ptr(EO), _ptr(EL), _ptr(EB), M, N,
+                                            _ptr(W), _ptr(bad), _stream(T)))
             return int(bad) == 0
 
     @staticmethod

@@ -593,3 +593,69 @@ def test_prefill_batches_from_two_threads_on_one_stream():
         sys.setswitchinterval(was)
     assert not failed and not wrong, (failed, len(wrong))
     _status_ok()
+
+
+@pytest.mark.parametrize("regime", ["mixed", "heavy", "llm"])
+@pytest.mark.parametrize("fault", ["none", "bits", "cols", "rows", "row_range", "col_range", "twice", "swapped", "el", "el_record",
+                                   "eb_count", "eb_mask", "eb_offset", "eb_entry", "eb_tail", "eo"])
+def test_conversion_check_covers_what_is_saved_and_what_is_read(fault, regime, monkeypatch):
+    """from_weight(verify=True) on a GPU: one wrong entry in the saved lists (esc_rows / esc_cols / esc_bits, which a reload
+    builds its tables from) or in the tables that the kernels read meanwhile is found, and a sound conversion passes"""
+    from statetree_b200 import TreeLinear, ops
+    W = bits_to_torch(G.weights(320, 1088, 5, regime), DEV)
+    encode = ops._Weights.encode
+
+    def broken(Wd):
+        tree, rows, cols, bits, (eo, el, eb) = encode(Wd)
+        n = rows.numel()
+        assert n > 40
+        i = n // 2
+        unit = int((eb[:, 0] & 0xFFFF > 0).nonzero()[-1])                       # a unit with escapes
+        if fault == "bits":
+            bits[i] ^= 1
+        elif fault == "cols":
+            cols[i] ^= 1
+        elif fault == "rows":
+            rows[i] ^= 1
+        elif fault == "row_range":
+            rows[n - 1] = 320
+        elif fault == "col_range":
+            cols[i] = -1
+        elif fault == "twice":
+            rows[i], cols[i], bits[i] = rows[i - 1], cols[i - 1], bits[i - 1]
+        elif fault == "swapped":
+            for t in (rows, cols, bits):
+                t[i - 1:i + 1] = t[i - 1:i + 1].flip(0)
+        elif fault == "el":
+            el[i] ^= 1 << 16
+        elif fault == "el_record":
+            el[i] ^= 1 << 10
+        elif fault == "eb_count":
+            eb[unit, 0] -= 1
+        elif fault == "eb_mask":
+            eb[unit, 0] ^= 1 << 20
+        elif fault == "eb_offset":
+            eb[unit, 1] ^= 1
+        elif fault == "eb_entry":
+            eb[unit, 2] ^= 1 << 16
+        elif fault == "eb_tail":
+            eb[unit, 15] ^= -2 ** 31
+        elif fault == "eo":
+            eo[eo.numel() // 2] += 1
+        return tree, rows, cols, bits, (eo, el, eb)
+
+    monkeypatch.setattr(ops._Weights, "encode", staticmethod(broken))
+    if fault == "none":
+        tl = TreeLinear.from_weight(W)
+        assert torch.equal(tl.dequantize().view(torch.int16), W.view(torch.int16))
+        return
+    with pytest.raises(RuntimeError, match="does not decode"):
+        TreeLinear.from_weight(W)
+    TreeLinear.from_weight(W, verify=False)                                     # (the caller's choice)
+
+
+def test_conversion_check_without_escapes():
+    from statetree_b200 import TreeLinear
+    W = torch.ones(32, 640, dtype=torch.bfloat16, device=DEV)
+    tl = TreeLinear.from_weight(W)
+    assert tl.esc_rows.numel() == 0 and torch.equal(tl.dequantize(), W)
