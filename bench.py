@@ -1094,7 +1094,7 @@ def main():
             control["sweep"] = sweep
         # ---- prefill-size batches (512 / 1024 / 2048 / 4096 rows): the two ways the tree-stored layers can run them, the
         # tcgen05 kernel (every token tile decodes the records again) and decode once + cuBLAS with the next layer
-        # decoded on a side stream meanwhile (what TreeLinear does above PREFILL_MIN rows), against cuBLAS over the
+        # decoded on a side stream meanwhile, and the one that TreeLinear takes (per layer, dense_for), against cuBLAS over the
         # dense copies.  Eager launches: a launch takes tens of microseconds of device time here
         prefill = []
         if B == 1 and not args.no_sweep and main_mode == "fused":
@@ -1129,6 +1129,14 @@ def main():
                     for i, tl in enumerate(chain):
                         st.dense_stage().run(tl, xin4[i % 4], ys[i % 4])
 
+                def run_modules():
+                    for i, tl in enumerate(chain):
+                        if tl.dense_for(Bs):
+                            st.dense_stage().run(tl, xin4[i % 4], ys[i % 4])
+                        else:
+                            eo, el, eb = tl._tables
+                            E.gemm(tl.tree, eo, el, xin4[i % 4], ys[i % 4], ws_p, cnt_p)
+
                 def run_control():
                     for Wqkv, Wo, Wgu, Wd in dense_f:
                         torch.matmul(xs[0], Wqkv.t(), out=ys[0])
@@ -1142,10 +1150,12 @@ def main():
                     return timed(fn, 3)
 
                 fl = sum(2 * Bs * M * N for _, M, N, _ in SHAPES) * args.layers
-                t_k, t_d, t_c = eager_time(run_kernel), eager_time(run_dense_stage), eager_time(run_control)
-                prefill.append({"batch": Bs, "tcgen05_kernel_ms": t_k, "decode_plus_cublas_ms": t_d, "bf16_control_ms": t_c,
-                                "tflops_decode_plus_cublas": fl / (t_d * 1e-3) / 1e12,
-                                "speedup_vs_bf16": t_c / min(t_k, t_d)})
+                t_k, t_d, t_m, t_c = (eager_time(f) for f in (run_kernel, run_dense_stage, run_modules, run_control))
+                dense_layers = sum(tl.dense_for(Bs) for tl in chain[:4])
+                prefill.append({"batch": Bs, "tcgen05_kernel_ms": t_k, "decode_plus_cublas_ms": t_d, "modules_ms": t_m,
+                                "modules_path": {0: "tcgen05 kernel", 4: "decode + cuBLAS"}.get(dense_layers, "both"),
+                                "bf16_control_ms": t_c, "tflops_modules": fl / (t_m * 1e-3) / 1e12,
+                                "speedup_vs_bf16": t_c / t_m})
                 del xs, ys
             control["prefill"] = prefill
         del dense, dense_f

@@ -3,8 +3,9 @@ surface of the reference's statetree/linear.py (TreeLinear 595-1018, TreeSlice 1
 torch.compile custom ops 1070-1095).
 
 Dispatch is one kernel per regime (no tuner, no multi-kernel ladder): up to GEMV_MAX activation rows run the
-memory-order fused decode GEMV, more rows the fused decode + tcgen05 GEMM, more than PREFILL_MIN rows the decode kernel
-into a BF16 scratch matrix + cuBLAS (the reference's prefill path).  Workspaces (exchange slots and zeroed
+memory-order fused decode GEMV, more rows the fused decode + tcgen05 GEMM, and prefill batches (more than PREFILL_MIN rows;
+for larger matrices more than FUSED_ROWS or HOST_ROWS, see dense_for) the decode kernel into a BF16 scratch matrix + cuBLAS
+(the reference's prefill path).  Workspaces (exchange slots and zeroed
 semaphores) are kept per (device, stream) because callers may run layers on side streams concurrently (the reason
 given at statetree/linear.py:457-466); they are sized once per shape, so steady-state calls allocate only the output.
 """
@@ -26,11 +27,19 @@ GEMV_AR_MAX = 12                    # rows up to which the GEMV that sums over t
 # it, the reference's path above 1024 rows (statetree/linear.py:37, 879-886), here from the size at which it overtakes the
 # tcgen05 kernel; 0 turns it off
 PREFILL_MIN = int(os.environ.get("STATETREE_PREFILL_MIN", "512"))
-# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel up to FUSED_ROWS rows: two layers of a
-# 4096 / 12288 model called in turn, us with the tcgen05 kernel / the scratch matrix: 700 rows 567 / 751, 1000 747 / 784,
-# 1500 1006 / 986, 2000 1351 / 1426, 3000 1906 / 1685, 4096 2544 / 2217.  (Smaller matrices take less time than their launches
-# on either path and keep the lower line.)
-FUSED_ROWS, FUSED_WEIGHTS = 2048, 1 << 22
+# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel for up to FUSED_ROWS rows (three of its
+# token tiles: every tile decodes the records again), and for up to HOST_ROWS rows below DENSE_WEIGHTS weights, where the scratch
+# path, 75 us of Python, events and launches per call, waits for the host.  Whole models' projections called one layer after
+# the other, ms with the tcgen05 kernel, the scratch matrix, this rule:
+#                                   700 rows         960              1024             1500             2000
+#   4096 / 12288, 36 layers   12.6 13.4 12.7   14.3 14.8 14.2   16.5 15.0 15.7   21.5 22.5 20.7   28.6 25.2 25.8
+#   2560 /  9728, 36 layers    6.4 10.5  6.4    7.7 10.5  7.6   10.0 10.5  8.6   12.4 11.1 12.0   15.7 14.0 14.5
+#   2048 /  6144, 28 layers    2.8  7.9  2.8    3.1  7.9  3.1    3.5  7.9  3.3    5.2  7.9  4.7    6.6  8.0  5.7
+# (hidden / intermediate size; medians of nine, which spread by 10 % and more at 4096 under the power cap.  In three runs over its
+# 36 layers the kernel took 1 to 14 % longer at 1024 rows, a fourth token tile, and 13 to 27 % longer at 2000; from 1280 to 1600
+# the two change places within the spread.  Two layers alone can favour the kernel up to 1300: a prefill runs them all.)
+FUSED_ROWS, FUSED_WEIGHTS = 960, 1 << 22
+HOST_ROWS, DENSE_WEIGHTS = 2048, 1 << 24
 DENSE_MAX = 1 << 28                 # weights: larger matrices (vocabulary-sized tables) never get a dense scratch copy
 _STATES = {}
 _BUFFERS = ("tree", "esc_rows", "esc_cols", "esc_bits")
@@ -338,7 +347,8 @@ class TreeLinear(nn.Module):
     def dense_for(self, B):
         """do B rows go through the scratch matrix"""
         M, N = self.out_features, self.in_features
-        return 0 < PREFILL_MIN < B and not (B <= FUSED_ROWS and M * N >= FUSED_WEIGHTS and M % 128 == 0) and self.dense_ok()
+        fused = M % 128 == 0 and M * N >= FUSED_WEIGHTS and B <= (HOST_ROWS if M * N < DENSE_WEIGHTS else FUSED_ROWS)
+        return 0 < PREFILL_MIN < B and not fused and self.dense_ok()
 
     def extra_repr(self):
         return (f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}, "

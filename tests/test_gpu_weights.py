@@ -659,3 +659,25 @@ def test_conversion_check_without_escapes():
     W = torch.ones(32, 640, dtype=torch.bfloat16, device=DEV)
     tl = TreeLinear.from_weight(W)
     assert tl.esc_rows.numel() == 0 and torch.equal(tl.dequantize(), W)
+
+
+@pytest.mark.parametrize("M,N,line", [(2048, 1984, 512), (2048, 2048, 2048), (4096, 4032, 2048), (4096, 4096, 960), (12288, 4096, 960),
+                                      (4096 + 16, 4096, 512)])
+def test_path_of_a_prefill_batch(M, N, line, monkeypatch):
+    """which matrices go through the scratch matrix at which rows: below 4M weights (or rows that the tcgen05 kernel does not
+    take) above 512, below 16M above 2048, larger ones above 960; either path gives the product"""
+    from statetree_b200 import TreeLinear
+    import statetree_b200.linear as L
+    g = torch.Generator(DEV).manual_seed(M + N)
+    W = (torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+    tl = TreeLinear.from_weight(W, verify=False)
+    calls, run = [], L._DenseStage.run
+    monkeypatch.setattr(L._DenseStage, "run", lambda self, layer, x, y: (calls.append(x.shape[0]), run(self, layer, x, y))[1])
+    for rows in (512, line, line + 1, 3000):
+        x = torch.randn(rows, N, device=DEV, generator=g).to(torch.bfloat16)
+        calls.clear()
+        y = tl(x)
+        assert calls == ([rows] if rows > line else []), rows
+        want = x.double() @ W.double().t()
+        assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1   # half an ulp of BF16 each
+    _status_ok()
