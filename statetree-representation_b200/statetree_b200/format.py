@@ -8,8 +8,9 @@ go to a side list.  One 1552-byte record holds a 16-row x 64-column block in mma
 
 This implementation places bytes through three lookup tables (leaf / state / node position of element (r, c) of a
 record) instead of the reference's chain of reshapes; the tables are the closed form also used by the KV kernels
-(statetree/csrc/kvcache.cu:31-38).  It runs on the tensor's device (CPU works and is what the tests pin against the
-golden fixtures).  The side tables the kernels of this package read are built by escape_tables().
+(statetree/csrc/kvcache.cu:31-38).  It is torch code for any device (on the CPU the tests pin it against the golden
+fixtures); a matrix on a GPU is encoded by the library's kernels instead where the library has been built, to the same bytes.
+The side tables the kernels of this package read are built by escape_tables().
 """
 import torch
 
@@ -72,12 +73,15 @@ def _encode_chunk(W):
 @torch.no_grad()
 def encode(W, chunk_rows=4096):
     """W [M, N] bf16 (M % 16 == 0, N % 64 == 0) -> dict(tree uint8 [M/16, N/64, 1552], esc_rows / esc_cols int32,
-    esc_bits int16), escapes in (row, col) order.  Runs on W's device in row chunks."""
+    esc_bits int16), escapes in (row, col) order.  Runs on W's device: in row chunks, which bound the 32-bit copies, or by the
+    library's kernels, which make none."""
     assert W.dim() == 2 and W.dtype == torch.bfloat16, "encode expects a 2-D bf16 matrix"
     M, N = W.shape
     assert M % 16 == 0 and N % 64 == 0, f"shape {tuple(W.shape)}: rows must be a multiple of 16, cols of 64"
     if W.is_cuda and M > 0 and N > 0:
-        return encode_with_tables(W)[0]
+        from .ops import built
+        if built():
+            return encode_with_tables(W)[0]
     chunk_rows = max(16, chunk_rows // 16 * 16)
     tree = torch.empty(M // 16, N // 64, RECORD_BYTES, dtype=torch.uint8, device=W.device)
     rows, cols, bits = [], [], []

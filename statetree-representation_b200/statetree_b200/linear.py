@@ -17,7 +17,7 @@ import torch
 import torch.nn as nn
 
 from . import format as F
-from .ops import _raw_stream, ext, on_device
+from .ops import _raw_stream, built, ext, on_device
 
 # activation rows up to which the GEMV kernel runs (<= 32).  The four projections of a 4096 / 12288 layer in a graph, us with
 # the GEMV / the tcgen05 GEMM: 8 rows 57 / 72, 16 rows 68 / 72, 20 rows 125 / 72 (beyond 16 the GEMV holds one CTA per SM)
@@ -286,9 +286,9 @@ class TreeLinear(nn.Module):
             escapes = F.escape_count(W)
             if escapes > max_escape_fraction * W.numel():
                 raise EscapeHeavy(f"{escapes / W.numel():.2%} of the weights escape")
-        out_features, in_features = W.shape
-        on_gpu = W.is_cuda and W.dim() == 2 and W.numel() > 0 and out_features % 16 == 0 and in_features % 64 == 0
+        on_gpu = (W.is_cuda and W.dim() == 2 and W.numel() > 0 and W.shape[0] % 16 == 0 and W.shape[1] % 64 == 0 and built())
         enc, tables = F.encode_with_tables(W) if on_gpu else (F.encode(W), None)
+        out_features, in_features = W.shape
         layer = cls(in_features, out_features, bias=bias is not None, device="meta", n_esc=int(enc["esc_rows"].numel()))
         layer._buffers.update({name: enc[name] for name in _BUFFERS})
         if bias is not None:
@@ -301,7 +301,7 @@ class TreeLinear(nn.Module):
                                        W if W.data_ptr() % 16 == 0 and W.is_contiguous() else W.clone(memory_format=torch.contiguous_format),
                                        (enc["esc_rows"], enc["esc_cols"], enc["esc_bits"], tables[2]))
             else:
-                back = F.decode_reference(*(layer._buffers[n] for n in _BUFFERS))
+                back = layer.dequantize() if layer.tree.is_cuda else F.decode_reference(*(layer._buffers[n] for n in _BUFFERS))
                 same = torch.equal(back.view(torch.int16), W.view(torch.int16))
             if not same:
                 raise RuntimeError("TreeLinear: the tree does not decode to the weights it was built from")

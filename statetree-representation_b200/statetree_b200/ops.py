@@ -85,6 +85,11 @@ def exported_symbols():
     return sorted(_SIGNATURES)
 
 
+def built():
+    """is there a library to load"""
+    return _LIB is not None or os.path.exists(LIB_PATH)
+
+
 def lib():
     """the ctypes handle; raises when the library has not been built (python statetree-representation_b200/build.py)"""
     global _LIB

@@ -98,6 +98,13 @@ def test_shape_checks():
         F.encode(torch.zeros(16, 64))
 
 
+def test_shapes_a_layer_cannot_hold_are_refused_as_by_encode():
+    from statetree_b200 import TreeLinear
+    for shape in ((2, 16, 64), (16,), (8, 64), (16, 32)):
+        with pytest.raises(AssertionError):
+            TreeLinear.from_weight(torch.zeros(*shape, dtype=torch.bfloat16))
+
+
 def test_interleave_gate_up_layout():
     """tile 2j of the fused weight = rows 16j .. 16j + 15 of gate, tile 2j + 1 = the same rows of up"""
     import torch

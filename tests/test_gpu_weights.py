@@ -681,3 +681,20 @@ def test_path_of_a_prefill_batch(M, N, line, monkeypatch):
         want = x.double() @ W.double().t()
         assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1   # half an ulp of BF16 each
     _status_ok()
+
+
+def test_encode_of_a_gpu_tensor_without_the_library(monkeypatch):
+    """format.encode needs nothing but torch: where the kernel library has not been built, a matrix on a GPU is encoded by the
+    tensor code, in row chunks as asked, with the same result"""
+    from statetree_b200 import format as F, ops
+    W = bits_to_torch(G.weights(96, 320, 11, "mixed"), "cpu")
+    want = F.encode(W)
+    by_kernel = F.encode(W.to(DEV))
+    monkeypatch.setattr(ops, "LIB_PATH", "/nonexistent/libstatetree_b200.so")
+    monkeypatch.setattr(ops, "_LIB", None)
+    heights, chunk = [], F._encode_chunk
+    monkeypatch.setattr(F, "_encode_chunk", lambda w: (heights.append(w.shape[0]), chunk(w))[1])
+    got = F.encode(W.to(DEV), chunk_rows=32)
+    assert heights == [32, 32, 32]
+    for k in want:
+        assert torch.equal(got[k].cpu(), want[k]) and torch.equal(by_kernel[k].cpu(), want[k]), k
