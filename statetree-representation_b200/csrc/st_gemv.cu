@@ -782,9 +782,9 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
   // Whole activation rows stay resident in shared memory when they fit in 34 KB (4 rows of 4096 columns), beside at least six
   // ring stages; beyond that every stage carries the matching 512-column slice of each row (24576 x 4096 at 8 rows: whole
   // rows beside three stages 31.2 us, slices 27.0; at 4 rows 25.6 / 25.9).  The pre-norm mode forms whole rows itself, so
-  // it takes up to 66 KB.
+  // it takes up to 66 KB; the row-parallel mode, measured on several GPUs with that limit and not since, keeps it.
   static const int xw_tune = tune("STATETREE_GEMV_XWHOLE_KB", 34);
-  const int xw_kb = norm ? 66 : xw_tune;
+  const int xw_kb = norm || ar ? 66 : xw_tune;
   p.xwhole = (dense && (long long)nx * (N * 2 + 16) <= (long long)xw_kb * 1024) ? 1 : 0;
   p.xw_stride = p.xwhole ? (int)(N * 2 + 16) : 0;
   p.xw_bytes = p.xwhole ? nx * p.xw_stride : 0;
@@ -810,8 +810,10 @@ Plan make_plan(long long M, long long N, int nprob, int nx, bool dense, bool act
   p.smem = (size_t)stages * p.stage_bytes + fixed;
   const long long slots = (long long)st::sm_count() * per_sm;
   // Small matrices: no CTA with less than three units, or a tile is cut into so many parts that their exchange is the tail
-  // (1024 x 4096, tiles of eight units: four parts 4.6 us at 1 row and 7.4 at 8, two parts 4.5 and 4.7)
-  const int min_units = act ? 2 : (min_tune < 1 ? 1 : min_tune);
+  // (1024 x 4096, tiles of eight units: four parts 4.6 us at 1 row and 7.4 at 8, two parts 4.5 and 4.7).  Two in the
+  // row-parallel mode, whose tail is the other ranks' words (6.8 us against 4.7 for the plain shard of 4096 x 2048 on two
+  // GPUs, measured with two).
+  const int min_units = act || ar ? 2 : (min_tune < 1 ? 1 : min_tune);
   long long want = p.U / min_units;
   if (want < 1) want = 1;
   p.C = (int)(want < slots ? want : slots);
@@ -878,8 +880,8 @@ int launch(GemvArgs& a, int nprob, int nx, long long ws_bytes, cudaStream_t stre
 }
 
 template <int NT>
-long long ws_need(long long M, long long N, int nprob, int nx, bool dense = true) {
-  const Plan p = make_plan<NT>(M, N, nprob, nx, dense);
+long long ws_need(long long M, long long N, int nprob, int nx, bool dense = true, bool ar = false) {
+  const Plan p = make_plan<NT>(M, N, nprob, nx, dense, false, ar);
   return p.maxcover == 1 ? 0 : (long long)nprob * p.T * p.maxcover * 16 * 8 * NT * 4;
 }
 
@@ -911,7 +913,12 @@ int dense_gemv(const char* who, const void* tree, const int32_t* eo, const uint3
 
 extern "C" int64_t st_gemv_workspace_bytes(int64_t M, int64_t N, int64_t B) {
   if (M <= 0 || N <= 0 || M % 16 || N % 64 || B < 1 || B > 32) return -1;
-  return B <= 8 ? ws_need<1>(M, N, 1, (int)B) : (B <= 16 ? ws_need<2>(M, N, 1, (int)B) : ws_need<4>(M, N, 1, (int)B));
+  // the plain GEMV and the row-parallel one take the same workspace: the larger of their needs
+  long long need[2];
+  for (int ar = 0; ar < 2; ++ar)
+    need[ar] = B <= 8 ? ws_need<1>(M, N, 1, (int)B, true, ar) : (B <= 16 ? ws_need<2>(M, N, 1, (int)B, true, ar)
+                                                                         : ws_need<4>(M, N, 1, (int)B, true, ar));
+  return need[0] > need[1] ? need[0] : need[1];
 }
 
 extern "C" int st_gemv(const void* tree, const int32_t* eo, const uint32_t* eb, const uint32_t* el, const void* X,

@@ -56,6 +56,21 @@ def test_argument_errors_are_reported_without_a_gpu():
     assert b"block size" in L.st_last_error()
 
 
+@pytest.mark.parametrize("M,N,B,slots", [(1024, 4096, 1, 5), (1024, 4096, 8, 5), (512, 2048, 1, 3), (256, 8192, 4, 9)])
+def test_row_parallel_plan_cuts_tiles_down_to_two_units(M, N, B, slots):
+    """the row-parallel GEMV keeps the grid it was measured with on several GPUs (no CTA below two units): without a workspace
+    the call is refused before anything is launched, and names the exchange slots of that grid (slots per tile, of 16 x 8
+    words each); st_gemv_workspace_bytes covers them"""
+    import ctypes
+    ops = _built()
+    L = ops.lib()
+    p = ctypes.c_void_p(4096)
+    need = M // 16 * slots * 16 * 8 * 4
+    assert L.st_gemv_allreduce((ctypes.c_void_p * 2)(4096, 4096), 0, 2, p, p, p, p, p, p, None, B, M, N, None, 0, None) != 0
+    assert f"workspace of {need} bytes needed".encode() in L.st_last_error(), L.st_last_error()
+    assert L.st_gemv_workspace_bytes(M, N, B) >= need
+
+
 def test_cpu_tensors_are_rejected():
     import torch
     ops = _built()
