@@ -292,6 +292,10 @@ class TreeExperts(nn.Module):
         self._tabs = self._maps = None                      # the trees may have moved
         return out
 
+    def _load_from_state_dict(self, *args, **kwargs):
+        self._tabs = self._maps = None                      # the trees and their side tables are about to be replaced
+        super()._load_from_state_dict(*args, **kwargs)
+
     @classmethod
     @torch.no_grad()
     def from_weights(cls, gate_up, down, verify=True):

@@ -326,3 +326,31 @@ def test_silu_gather_equals_gate_then_gather(S, I, bs):
     want = torch.full_like(xg, 7.0)
     want[valid] = act[sorted_ids[valid].long()]
     assert torch.equal(xg.view(torch.int16), want.view(torch.int16))
+
+
+def test_experts_loaded_over_use_the_new_weights():
+    """load_state_dict into a block that has run (its address tables and tensor maps exist): every path computes with the weights
+    that were loaded, in place or by assignment"""
+    from statetree_b200.experts import TreeExperts
+    E, H, I = 4, 128, 64
+    g = torch.Generator(DEV).manual_seed(3)
+
+    def block():
+        up = torch.randn(E, 2 * I, H, device=DEV, generator=g) * 0.05
+        up[:, :, 7] *= 4096                                                     # escapes
+        return TreeExperts.from_weights(up.to(torch.bfloat16), (torch.randn(E, H, I, device=DEV, generator=g) * 0.05).to(torch.bfloat16))
+
+    for assign in (False, True):
+        a, b = block(), block()
+        for T in (2, 40):                                                       # slot kernel, grouped GEMM
+            x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+            ids = torch.randint(0, E, (T, 2), device=DEV, generator=g)
+            w = torch.full((T, 2), 0.5, device=DEV)
+            want = b(x, ids, w)
+            assert not torch.equal(a(x, ids, w), want)
+        a.load_state_dict(b.state_dict(), assign=assign)
+        for T in (2, 40):
+            x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+            ids = torch.randint(0, E, (T, 2), device=DEV, generator=g)
+            w = torch.full((T, 2), 0.5, device=DEV)
+            assert torch.equal(a(x, ids, w), b(x, ids, w)), (assign, T)
