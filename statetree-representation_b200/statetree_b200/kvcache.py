@@ -34,7 +34,8 @@ class PageStore:
         self.pages = torch.zeros(num_blocks, num_kv_heads, 2, 2, RKV, dtype=torch.uint8, device=device)
         self.pool = torch.zeros(pool_blocks, 16, dtype=torch.int32, device=device)
         self.pcnt = torch.zeros(2, dtype=torch.int32, device=device)
-        self._wo = self._wml = None
+        self._wo = self._wml = None                        # split partials: grown, never freed (a captured graph may write
+        self._retired = []                                 # into the ones it was given)
 
     def append(self, K, V, slots, reuse=False):
         """K, V [N, H, 128] bf16 (heads contiguous), slots int64 [N] = block * 16 + row, -1 = padding token"""
@@ -48,6 +49,8 @@ class PageStore:
         if splits > 1:
             need = B * Hq * splits
             if self._wo is None or self._wo.numel() < need * 128:
+                if self._wo is not None:
+                    self._retired.append((self._wo, self._wml))
                 self._wo = torch.empty(need * 128, dtype=torch.float32, device=q.device)
                 self._wml = torch.empty(need * 2, dtype=torch.float32, device=q.device)
         else:

@@ -478,3 +478,27 @@ def test_argmax_and_decode_slots_equal_torch(rows, V):
         full = n >= cache.max_len
         assert slots.tolist() == [-1 if full else (b * cache.max_pages + page) * 16 + n % 16 for b in range(B)], n
         assert cache.lens[:B].tolist() == [min(n + 1, cache.max_len)] * B
+
+
+def test_attention_workspace_growth_keeps_captured_graphs_valid():
+    """a larger call after a capture takes a new workspace; the one that the graph writes into stays allocated"""
+    import weakref
+    from statetree_b200.kvcache import PageStore
+    g = torch.Generator(DEV).manual_seed(1)
+    store = PageStore(64, 2, DEV)
+    K, V = (torch.randn(1024, 2, D, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    store.append(K, V, torch.arange(1024, device=DEV))
+    table = torch.arange(64, dtype=torch.int32, device=DEV).view(1, 64)
+    lens = torch.full((8,), 1000, dtype=torch.int32, device=DEV)
+    q = torch.randn(8, 4, D, device=DEV, generator=g).to(torch.bfloat16)
+    scale = 1.0 / math.sqrt(D)
+    want = store.attention(q[:1], table, lens[:1], scale, 4)
+    graph, out = torch.cuda.CUDAGraph(), torch.empty(1, 4, D, dtype=torch.bfloat16, device=DEV)
+    with torch.cuda.graph(graph):
+        store.attention(q[:1], table, lens[:1], scale, 4, out=out)
+    used = weakref.ref(store._wo), weakref.ref(store._wml)
+    store.attention(q, table.expand(8, 64).contiguous(), lens, scale, 16)
+    assert store._wo is not used[0]() and all(r() is not None for r in used)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
