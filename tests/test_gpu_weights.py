@@ -458,34 +458,91 @@ def test_encode_kernels_equal_the_torch_formulation(M, N, regime):
 
 @pytest.mark.parametrize("M,B", [(128 * 149, 20), (128 * 192, 64), (128 * 230, 17), (128 * 290, 33)])
 def test_gemm_row_blocks_beyond_one_per_sm(M, B):
-    """more row blocks than SMs, fewer than twice as many: the product goes out as two launches side by side; the activations
-    come from the kernel right before it in the stream and the result is read by the one right after it"""
+    """more row blocks than SMs, fewer than twice as many, two CTAs per SM; the activations come from the kernel right before
+    the product in the stream and its result is read by the one right after it, each link of the chain from the values of the one
+    before, on other inputs in every replay"""
     from statetree_b200 import TreeLinear, ops
     N = 1024
     g = torch.Generator(DEV).manual_seed(M + B)
     W = (torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
     W[:, 5] *= 4096                                                             # escapes
     tl = TreeLinear.from_weight(W)
-    x = torch.randn(B, N, device=DEV, generator=g).to(torch.bfloat16)
-    want = x.double() @ W.double().t()
+    x = torch.empty(B, N, dtype=torch.bfloat16, device=DEV)
+
+    def chain():
+        src, ys = x * 1.0, []
+        for _ in range(3):
+            ys.append(tl(src))
+            src = (ys[-1][:, :N] * 0.001 + x).to(torch.bfloat16)
+        return ys
+
+    x.zero_()
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        tl(x)
+        chain()
         side.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=side):
-            src = x * 1.0
-            for _ in range(3):
-                y = tl(src)
-                src = src + y[:, :N] * 0.0                                      # depends on the whole chain before it
-            out = y.float() * 1.0
+            ys = chain()
         for _ in range(3):
+            x.copy_(torch.randn(B, N, device=DEV, generator=g).to(torch.bfloat16))
             graph.replay()
+            side.synchronize()
+            got = [y.clone() for y in ys]
+            side.synchronize()
+            src = x
+            for y in got:                                                       # every link from the values it was given
+                want = src.double() @ W.double().t()
+                assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1   # BF16 results: half an ulp each
+                src = (y[:, :N] * 0.001 + x).to(torch.bfloat16)
     side.synchronize()
-    assert torch.equal(out, tl(x).float())
-    assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1  # BF16 results: half an ulp each
     assert ops.device_status() == 0
+
+
+def _kernel_launches(fn, side):
+    """kernels that fn launches, counted in a captured graph"""
+    import ctypes
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=side):
+        out = fn()
+    n = ctypes.c_size_t(0)
+    assert ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(n)) == 0
+    graph.replay()
+    side.synchronize()
+    return n.value, [t.clone() for t in out]
+
+
+@pytest.mark.parametrize("Ms,B", [((128 * 149,), 129), ((128 * 192,), 129), ((128 * 149,), 300), ((128 * 192,), 300), ((128 * 149,), 321),
+                                  ((128 * 100, 128 * 92), 300), ((128 * 148, 128 * 44), 300), ((128 * 170, 128 * 22), 129),
+                                  ((128 * 147, 128, 128 * 2), 300)])
+def test_gemm_full_waves_and_remainder_go_out_as_two_launches(Ms, B):
+    """one CTA per SM (over 128 rows) and more row blocks than SMs: the full waves unsplit, the rest of the row blocks in a second
+    launch with a split of its own, for one matrix and for lists whose members end before, at and beyond the cut (148 row blocks)"""
+    from statetree_b200 import TreeLinear
+    from statetree_b200.linear import forward_list
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the shapes are chosen for 148 SMs")
+    N = 2048
+    g = torch.Generator(DEV).manual_seed(sum(Ms) + B)
+    Ws = [(torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16) for M in Ms]
+    for W in Ws:
+        W[:, 5] *= 4096                                                         # escapes
+    tls = [TreeLinear.from_weight(W) for W in Ws]
+    x = torch.randn(B, N, device=DEV, generator=g).to(torch.bfloat16)
+    fn = (lambda: [tls[0](x)]) if len(tls) == 1 else (lambda: forward_list(tls, x))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        eager = fn()
+        side.synchronize()
+        launches, got = _kernel_launches(fn, side)
+    assert launches == 2
+    for y, e, W in zip(got, eager, Ws):
+        want = x.double() @ W.double().t()
+        assert torch.equal(y, e)
+        assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -9 * 1.1
+    _status_ok()
 
 
 @pytest.mark.parametrize("rows,width", [(4, 512), (8, 128), (1, 512), (40, 512), (700, 512)])
