@@ -3,9 +3,10 @@
 //
 // Bound: HBM.  st_encode reads the matrix once (2 B per weight) and writes the records once (1.52 B); the escape passes
 // touch only the records that have escapes.  4096 x 12288 on a B200: st_encode 39 us (177 MB, 4.5 TB/s), the two prefix
-// sums 15 us, st_encode_lists 23 us, st_dec_check 36 us (nothing dense is written back), st_lists_check 8 us (of the stored lists and the escape blocks).  TreeLinear.from_weight of that
-// matrix with its checks takes 0.24 ms; with the torch formulation (format._encode_chunk, still the CPU path: ~60 passes over
-// 32- and 64-bit copies, then a sort of the escapes and a dense decode to compare) it took 3.7 ms.
+// sums 15 us, st_encode_lists 23 us, st_dec_check 36 us (nothing dense is written back), st_lists_check 8 us (the stored lists and
+// the escape blocks).  TreeLinear.from_weight of that matrix with its checks takes 0.24 ms; with the torch formulation
+// (format._encode_chunk, still the CPU path: ~60 passes over 32- and 64-bit copies, then a sort of the escapes and a dense
+// decode to compare) it took 3.7 ms.
 #include "../../include/statetree_b200.h"
 #include "st_encode.cuh"
 #include "st_host.h"

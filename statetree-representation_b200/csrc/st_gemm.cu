@@ -444,7 +444,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
       const uint32_t mine = smem_addr(smem);
       // CPP columns per pass, every partial tile's float4 requested before the first add: distributed-shared-memory
       // reads have a long latency, so the loads of a pass must all be in flight together
-      constexpr int CPP = DG;                                    // (DG = 1 has 80 registers per thread, DG = 2 twice the columns)
+      constexpr int CPP = DG;                                    // (DG = 2 has up to twice the columns; DG = 1 takes 63 registers of the 88 it may)
       for (int c = c_lo + warp; c < c_end; c += CPP * NDW) {
         float4 v[CPP][8];
 #pragma unroll

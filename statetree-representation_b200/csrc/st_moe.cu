@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) silu_mul_vec_kernel(const uint4* __restri
 }
 // silu_mul of the pair each used entry of sorted names, written in block order: Xg[i, :] = silu(gate) * up of gu[sorted[i]]
 // (the activation rows of the second grouped product; no act array and no gather of it in between).  One warp per row,
-// 16-byte vectors.  8000 pairs of 768 in 24 576 bytes of gu each: silu_mul 13 us + gather 5 us before, 10 us.
+// 16-byte vectors.  8000 pairs of 768 (3072 bytes of gu each, 24.6 MB): silu_mul 13 us + gather 5 us before, 10 us.
 __global__ void __launch_bounds__(256) moe_silu_gather_kernel(const uint4* __restrict__ gu, const int* __restrict__ sorted,
                                                               const int* __restrict__ npost, int S, int I8, long long rows,
                                                               uint4* __restrict__ Xg) {

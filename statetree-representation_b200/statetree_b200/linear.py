@@ -60,7 +60,7 @@ class _DevState:
         self._retired = []
         self._need = {}                                 # workspace bytes per call shape (a pure function of it)
         self.ws = self._new_ws(1 << 20)
-        self.scratch = torch.empty(1 << 20, dtype=torch.float32, device=device)   # the GEMM's partial tiles (no contract)
+        self.scratch = torch.empty(0, dtype=torch.float32, device=device)         # the GEMM's workspace (it asks for none)
         self.cnt = torch.zeros(1 << 16, dtype=torch.int32, device=device)
 
     def _new_ws(self, words):

@@ -421,7 +421,7 @@ def test_attention_split_counts_and_both_cta_sizes(B, heads, splits):
 
 @pytest.mark.parametrize("H,N,pad,first", [(1, 16, 0, 0), (2, 1040, 0, 0), (8, 2000, 0, 5), (2, 1100, 8, 0), (2, 1100, 2, 0), (3, 1024, 24, 16)])
 def test_whole_page_append_equals_the_oracle(H, N, pad, first):
-    """whole pages of consecutive tokens (encoded four rows at a time) beside partial pages at both ends and a hole, token
+    """whole pages of consecutive tokens (encoded at once, in fragment order) beside partial pages at both ends and a hole, token
     strides of every alignment, few and many escapes (the pool chain), the pages written twice
     with their chains kept: pages and the values read back equal the oracle's"""
     from statetree_b200.kvcache import PageStore
