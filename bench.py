@@ -1144,13 +1144,18 @@ def main():
                         torch.matmul(xs[0], Wgu.t(), out=ys[2])
                         torch.matmul(xs[2], Wd.t(), out=ys[3])
 
-                def eager_time(fn):
-                    fn()
-                    torch.cuda.synchronize()
-                    return timed(fn, 3)
+                def in_turn(fns, rounds=4):
+                    """mean ms of each, in turn (under the power cap a path's time depends on what ran before it)"""
+                    total = [0.0] * len(fns)
+                    for _ in range(rounds):
+                        for k, fn in enumerate(fns):
+                            fn()
+                            torch.cuda.synchronize()
+                            total[k] += timed(fn, 3) / rounds
+                    return total
 
                 fl = sum(2 * Bs * M * N for _, M, N, _ in SHAPES) * args.layers
-                t_k, t_d, t_m, t_c = (eager_time(f) for f in (run_kernel, run_dense_stage, run_modules, run_control))
+                t_k, t_d, t_m, t_c = in_turn((run_kernel, run_dense_stage, run_modules, run_control))
                 dense_layers = sum(tl.dense_for(Bs) for tl in chain[:4])
                 prefill.append({"batch": Bs, "tcgen05_kernel_ms": t_k, "decode_plus_cublas_ms": t_d, "modules_ms": t_m,
                                 "modules_path": {0: "tcgen05 kernel", 4: "decode + cuBLAS"}.get(dense_layers, "both"),

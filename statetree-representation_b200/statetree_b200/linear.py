@@ -27,18 +27,17 @@ GEMV_AR_MAX = 12                    # rows up to which the GEMV that sums over t
 # it, the reference's path above 1024 rows (statetree/linear.py:37, 879-886), here from the size at which it overtakes the
 # tcgen05 kernel; 0 turns it off
 PREFILL_MIN = int(os.environ.get("STATETREE_PREFILL_MIN", "512"))
-# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel for up to FUSED_ROWS rows (three of its
-# token tiles: every tile decodes the records again), and for up to HOST_ROWS rows below DENSE_WEIGHTS weights, where the scratch
-# path, 75 us of Python, events and launches per call, waits for the host.  Whole models' projections called one layer after
-# the other, ms with the tcgen05 kernel, the scratch matrix, this rule:
-#                                   700 rows         960              1024             1500             2000
-#   4096 / 12288, 36 layers   12.6 13.4 12.7   14.3 14.8 14.2   16.5 15.0 15.7   21.5 22.5 20.7   28.6 25.2 25.8
-#   2560 /  9728, 36 layers    6.4 10.5  6.4    7.7 10.5  7.6   10.0 10.5  8.6   12.4 11.1 12.0   15.7 14.0 14.5
-#   2048 /  6144, 28 layers    2.8  7.9  2.8    3.1  7.9  3.1    3.5  7.9  3.3    5.2  7.9  4.7    6.6  8.0  5.7
-# (hidden / intermediate size; medians of nine, which spread by 10 % and more at 4096 under the power cap.  In three runs over its
-# 36 layers the kernel took 1 to 14 % longer at 1024 rows, a fourth token tile, and 13 to 27 % longer at 2000; from 1280 to 1600
-# the two change places within the spread.  Two layers alone can favour the kernel up to 1300: a prefill runs them all.)
-FUSED_ROWS, FUSED_WEIGHTS = 960, 1 << 22
+# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel for up to FUSED_ROWS rows (six of its token
+# tiles: every tile decodes the records again), and for up to HOST_ROWS rows below DENSE_WEIGHTS weights, where the scratch path,
+# 75 us of Python, events and launches per call, waits for the host.  All projections of a model called one layer after the
+# other, ms with the kernel / the scratch matrix, mean of 50 passes, the paths in turn (they draw on one power budget):
+#   rows                       960          1024         1152         1281         1536         1792         1920         2000
+#   4096 / 12288, 36 layers    13.7 / 15.5  15.9 / 15.6  16.5 / 17.6  20.0 / 19.3  22.0 / 21.0  24.6 / 25.0  25.6 / 25.9  28.5 / 25.7
+# (hidden / intermediate size.)  From 961 to 1920 rows the two change places: the kernel is up to 5 % slower from 961 to 1030, at
+# 1540 and from 1601 to 1860, and up to 12 % faster from 1050 to 1280, where cuBLAS takes one of two times 40 % apart; at 1921 a
+# seventh tile sets it back by 11 %.  5120 / 17408, 20 layers: 14.9 / 14.6 at 1024, 19.6 / 23.0 at 1536, 25.1 / 25.0 at 2000.
+# 2048 / 6144, 28 layers: 3.5 / 7.9 at 1024, 6.6 / 8.0 at 2000 (5.7 with its 25M gate + up on the scratch path).
+FUSED_ROWS, FUSED_WEIGHTS = 1920, 1 << 22
 HOST_ROWS, DENSE_WEIGHTS = 2048, 1 << 24
 DENSE_MAX = 1 << 28                 # weights: larger matrices (vocabulary-sized tables) never get a dense scratch copy
 _STATES = {}

@@ -718,11 +718,11 @@ def test_conversion_check_without_escapes():
     assert tl.esc_rows.numel() == 0 and torch.equal(tl.dequantize(), W)
 
 
-@pytest.mark.parametrize("M,N,line", [(2048, 1984, 512), (2048, 2048, 2048), (4096, 4032, 2048), (4096, 4096, 960), (12288, 4096, 960),
+@pytest.mark.parametrize("M,N,line", [(2048, 1984, 512), (2048, 2048, 2048), (4096, 4032, 2048), (4096, 4096, 1920), (12288, 4096, 1920),
                                       (4096 + 16, 4096, 512)])
 def test_path_of_a_prefill_batch(M, N, line, monkeypatch):
     """which matrices go through the scratch matrix at which rows: below 4M weights (or rows that the tcgen05 kernel does not
-    take) above 512, below 16M above 2048, larger ones above 960; either path gives the product"""
+    take) above 512, below 16M above 2048, larger ones above 1920; either path gives the product"""
     from statetree_b200 import TreeLinear
     import statetree_b200.linear as L
     g = torch.Generator(DEV).manual_seed(M + N)
