@@ -1,7 +1,9 @@
-// Large-batch fused tree-decode + GEMM on the 5th-generation tensor cores (tcgen05 / TMEM) of sm_100a.
+// Fused tree-decode + GEMM on the 5th-generation tensor cores (tcgen05 / TMEM) of sm_100a: up to 320 tokens in one tile, and the
+// grouped (mixture-of-experts) form.  More tokens, and fewer where they are the faster ones, go to CTA pairs (st_gemm_pair.cu).
 //   Y[B, M] = X[B, N] W[M, N]^T,  W as state-tree records, fp32 accumulation in tensor memory, BF16 output.
 //
-// One CTA computes a 128-row block of W against one tile of NT tokens over a contiguous range of 64-column k-tiles.
+// One CTA computes a 128-row block of W against a tile of NT tokens (all of a dense call's) over a contiguous range of
+// 64-column k-tiles.
 // Warp roles:
 //   8 DG decode warps, in DG groups of eight (group g takes the k-tile pairs g, g + DG, ...): each warp turns the two
 //              records of its 16 rows into mma-fragment registers (five integer ops per four weights), patches escapes,
@@ -22,99 +24,21 @@
 // are scattered back to their pair indices.
 // Every mbarrier wait is bounded; a wait that runs out sets the device status word and the CTA leaves after
 // releasing its tensor memory.
-#include <cuda.h>
-
 #include <stdlib.h>
 #include <string.h>
 
 #include <mutex>
 
 #include "../../include/statetree_b200.h"
-#include "st_common.cuh"
-#include "st_host.h"
+#include "st_tc.cuh"
 
 namespace {
 using namespace st;
 
-constexpr int NDEC = 8;                      // decode warps of a group = records per k-tile
-constexpr int A_COLS = 32;                   // tensor-memory columns of a decoded weight tile: 128 rows x 64 BF16
-constexpr int PAIR = 2;                      // k-tiles per decode step
-
-constexpr int MAXL = 4;                       // matrices in one list launch
-
-struct GemmArgs {
-  const uint8_t* tree; const int* eo; const uint32_t* el;
-  uint16_t* Y; float* Yf; int* status;
-  // grouped (mixture of experts): per-expert weight tensor maps and escape tables, pairs in moe_align layout
-  const CUtensorMap* maps; const long long* eop; const long long* elp;
-  const int* sorted; const int* bexp; const int* npost; int E;
-  long long M, N;
-  int B, NG, NT, KS, RB, TT, astages, xstages, rstages, bar_off, tmem_cols, rb0;
-  // list of matrices that share the activations (q / k / v, gate / up as separate trees): member of each row block
-  int nlist; int rbend[MAXL];                 // first row block after each member in the concatenation
-  const int* leo[MAXL]; const uint32_t* lel[MAXL]; uint16_t* lY[MAXL]; float* lYf[MAXL]; long long lM[MAXL];
-};
-struct WMaps { CUtensorMap m[MAXL]; };        // weight tensor maps: one, or one per member of a list
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               :: "r"(smem_addr(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-               :: "r"(smem_addr(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(slot)), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(addr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(bar)) : "memory");
-}
-// D[128 x n] (+)= A B^T with A (128 rows x 16 BF16: eight 32-bit columns) in tensor memory, B in shared memory
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-               :: "r"(d_tmem), "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-// a decoded record (16 rows x 64 BF16 as four mma A fragments) -> 16 lanes x 32 columns of tensor memory.  16x128b: lane
-// (g, t) holds column t of rows g (even registers) and g + 8 (odd), each register pair four columns further: exactly
-// (A[s][0], A[s][1]) = k 16 s + 2t, (A[s][2], A[s][3]) = k 16 s + 8 + 2t
-__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const uint32_t (&A)[4][4]) {
-  asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-               :: "r"(taddr), "r"(A[0][0]), "r"(A[0][1]), "r"(A[0][2]), "r"(A[0][3]), "r"(A[1][0]), "r"(A[1][1]),
-                  "r"(A[1][2]), "r"(A[1][3]), "r"(A[2][0]), "r"(A[2][1]), "r"(A[2][2]), "r"(A[2][3]), "r"(A[3][0]),
-                  "r"(A[3][1]), "r"(A[3][2]), "r"(A[3][3]) : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                 "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-               : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-
+constexpr int MAXL = MAXL_GEMM;              // matrices in one list launch
 #define GW mbar_wait_look
-constexpr int RAW_SLOT = NDEC * PAIR * REC;  // 24832 B: the sixteen records of a pair of k-tiles
 constexpr int XBOX_GROUPED = 32;             // rows per activation load of the grouped variant
 template <int DG> constexpr int gemm_threads() { return (DG * NDEC + 3) * 32; }
-
-// instruction descriptor: D fp32, A and B bf16, both K-major, N = n, M = 128
-__host__ __device__ constexpr uint32_t mma_idesc(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
 
 // Three rings.  The RAW ring (R slots of sixteen records) faces HBM: its depth sets the bytes in flight.  The A ring (SA
 // slots of two decoded weight tiles in tensor memory) covers the decode -> MMA hand-over, the X ring (SX activation tiles
@@ -127,7 +51,7 @@ __host__ __device__ constexpr uint32_t mma_idesc(int n) {
 // DG = 1 (token tiles up to 128): eight decode warps, at most half of an SM's shared memory, registers and tensor memory,
 // so two CTAs share an SM: one CTA's start-up, drain and epilogue run under the other's main loop, and the next launch's
 // CTAs become resident (and start streaming weights) as soon as any CTA of this launch leaves.
-// DG = 2 (up to 320 tokens): one CTA per SM, sixteen decode warps; a whole batch of up to 320 rows decodes every record once.
+// DG = 2 (up to 320 tokens): one CTA per SM, sixteen decode warps.
 //
 // Measured, the four projections of a layer (6144, 4096, 24576 x 4096 and 4096 x 12288) in a graph, us per layer: 64 rows
 // 108 -> 85, 300 rows 251 -> 153 (was: A through shared memory by stmatrix, one record per step, 64 / 128 / 256-token
@@ -164,10 +88,9 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accbar + 1);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0);   // (a warp-uniform value to the compiler)
-  // unit of this CTA.  Dense: the token tiles of a row block run next to each other (its records then come from HBM once
-  // and from L2 for the other tiles); grouped: the row blocks of a pair block do (they share the gathered activations)
+  // unit of this CTA.  Grouped: the row blocks of a pair block run next to each other (they share the gathered activations)
   const int ks = blockIdx.x % a.KS, rt = blockIdx.x / a.KS;
-  const int rb = GROUPED ? rt % a.RB : a.rb0 + rt / a.TT, tt = GROUPED ? rt / a.RB : rt % a.TT;
+  const int rb = GROUPED ? rt % a.RB : a.rb0 + rt, tt = GROUPED ? rt / a.RB : 0;
   // whole pairs of k-tiles; an odd last tile is paired with one beyond the matrix, which both tensor maps fill with zeros
   const int pairs = (a.NG + PAIR - 1) / PAIR;
   const int p0 = (int)((long long)pairs * ks / a.KS), np = (int)((long long)pairs * (ks + 1) / a.KS) - p0;
@@ -233,8 +156,8 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   } else if (warp == W_X) {
     if (elect_one()) asm volatile("prefetch.tensormap [%0];" :: "l"(&xmap) : "memory");
   } else if (warp == W_MMA) {
-    tmem_alloc(tmem_slot, (uint32_t)a.tmem_cols);
-    tmem_relinquish();
+    tmem_alloc<1>(tmem_slot, (uint32_t)a.tmem_cols);
+    tmem_relinquish<1>();
   }
   tc_fence_before();
   __syncthreads();
@@ -278,7 +201,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
     // (measured: ~1000 cycles for the four MMAs and the commit of a k-tile instead of < 200).
     // beyond 256 tokens one MMA cannot cover the tile: two, of (up to 16 tokens) different width
     const int half = NT > 256 ? ((NT / 2 + 15) & ~15) : 0;
-    const uint32_t idesc = mma_idesc(half ? half : nmma), idesc2 = mma_idesc(half ? NT - half : 16);
+    const uint32_t idesc = mma_idesc(128, half ? half : nmma), idesc2 = mma_idesc(128, half ? NT - half : 16);
     int xs = 0, xk = 0;
     bool ok = true;
     for (int i = 0, s = 0, k = 0; ok && i < np; ++i, s = (s + 1 == SA ? 0 : s + 1), k += (s == 0)) {
@@ -293,9 +216,9 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
         if (elect_one()) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            tc_mma(tmem, ta + 8 * j, db + 2 * j, idesc, (i || h || j) ? 1u : 0u);
+            tc_mma<1>(tmem, ta + 8 * j, db + 2 * j, idesc, (i || h || j) ? 1u : 0u);
             if (half)
-              tc_mma(tmem + (uint32_t)half, ta + 8 * j, db + 2 * j + (uint64_t)(half * 8), idesc2, (i || h || j) ? 1u : 0u);
+              tc_mma<1>(tmem + (uint32_t)half, ta + 8 * j, db + 2 * j + (uint64_t)(half * 8), idesc2, (i || h || j) ? 1u : 0u);
           }
           tc_commit(xempty + xs);
           if (h == PAIR - 1) tc_commit(aempty + s);
@@ -451,8 +374,11 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
         for (int h = 0; h < CPP; ++h)
 #pragma unroll
           for (int p = 0; p < 8; ++p)
-            if (p < a.KS && c + h * NDW < c_end)
-              v[h][p] = ld_cluster_f4(map_to_cta(mine + (uint32_t)(((c + h * NDW) * 128 + 4 * lane) * 4), (uint32_t)p));
+            if (p < a.KS && c + h * NDW < c_end) {
+              const uint32_t at = (uint32_t)(((c + h * NDW) * 128 + 4 * lane) * 4);
+              v[h][p] = p == ks ? *reinterpret_cast<const float4*>(smem + at)        // (not through the cluster's network)
+                                : ld_cluster_f4(map_to_cta(mine + at, (uint32_t)p));
+            }
 #pragma unroll
         for (int h = 0; h < CPP; ++h) {
           const int cc = c + h * NDW;
@@ -475,7 +401,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   }
   if (warp == W_MMA) {
     __syncwarp();
-    tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
+    tmem_dealloc<1>(tmem, (uint32_t)a.tmem_cols);
   }
 }
 
@@ -580,33 +506,29 @@ void gemm_rings(GemmPlan& p) {
 
 constexpr int NT_MAX = 320;                                      // 320 accumulator columns + 4 weight tiles of 32 fill TMEM
 
-GemmPlan gemm_plan(long long M, long long N, long long B) {
+GemmPlan gemm_plan(long long M, int NG, long long B, double& us) {   // B <= NT_MAX
   GemmPlan p;
-  // the fewest token tiles (every tile decodes the records again), of equal width
-  p.TT = (int)((B + NT_MAX - 1) / NT_MAX);
-  const int per = (int)((B + p.TT - 1) / p.TT);
-  p.NT = (per + 15) & ~15;                                        // MMA widths: multiples of 16
+  p.TT = 1;
+  p.NT = (int)((B + 15) & ~15);                                   // MMA widths: multiples of 16
   p.RB = (int)(M / 128);
-  const int NG = (int)(N / 64), sms = st::sm_count();
+  const int sms = st::sm_count();
   gemm_rings(p);
   // Split of the k range = cluster size (<= 8): the least estimated time in us, fitted to launches of the four projection
-  // shapes of a 4096 / 12288 model in a graph (32 to 192 row blocks, 16 to 304 tokens, splits 1 to 8; within 10 %):
+  // shapes of a 4096 / 12288 model (and 12288, 3072, 2048 x 2048) in a graph (16 to 192 row blocks, 16 to 304 tokens, splits 1 to
+  // 8; within 15 %):
   //   start-up + drain, the epilogue (grows with the tiles to add through distributed shared memory), and per pair of
   //   k-tiles a time that grows with the CTAs that stream at once (two per SM) or with the token tile (one per SM).
   // A grid larger than the CTAs that are resident at once runs in waves.
   const int pairs = (NG + PAIR - 1) / PAIR, ksmax = pairs / 4 < 1 ? 1 : (pairs / 4 > 8 ? 8 : pairs / 4);
   auto estimate = [&](int rows, int ks) {
-    const double ctas = (double)rows * p.TT * ks;
+    const double ctas = (double)rows * ks;
     const double slots = (double)(p.DG == 1 ? resident_ctas<1>(ks, p.smem, sms) : resident_ctas<2>(ks, p.smem, sms));
     if (slots <= 0) return 1e30;
     const double waves = ctas <= slots ? 1.0 : (double)(long long)((ctas + slots - 1) / slots);
-    const double per_cta = (double)((pairs + ks - 1) / ks);
-    if (p.DG == 1) {
-      const double load = ctas < slots ? ctas : slots;
-      return waves * (per_cta * (0.45 + 0.0024 * load) * (1.0 + 0.0015 * (p.NT - 16)) + 3.0 + 0.3 * ks * p.NT / 64.0);
-    }
+    const double per_cta = (double)((pairs + ks - 1) / ks), load = ctas < slots ? ctas : slots;
+    if (p.DG == 1) return waves * (per_cta * (0.45 + 0.0024 * load) * (1.0 + 0.0015 * (p.NT - 16)) + 3.0 + 0.3 * ks * p.NT / 64.0);
     const double pair = 0.785 * p.NT / 304.0 > 0.5 ? 0.785 * p.NT / 304.0 : 0.5;
-    return waves * (per_cta * pair + 4.0 + 0.45 * ks * p.NT / 64.0);
+    return waves * (per_cta * (pair + 0.1 * load / sms) + 6.0 + 0.3 * ks * p.NT / 64.0);
   };
   auto best_split = [&](int rows, double& t) {
     int best = 1;
@@ -620,18 +542,18 @@ GemmPlan gemm_plan(long long M, long long N, long long B) {
     }
     return best;
   };
-  double whole;
-  p.KS = best_split(p.RB, whole);
+  p.KS = best_split(p.RB, us);
   p.RB1 = 0;
   p.KS1 = 1;
-  // One CTA per SM: a last wave that is nearly empty costs as much as a full one (192 row blocks at 300 tokens: 148 + 44).
+  // One CTA per SM: a last wave that is nearly empty costs as much as a full one (192 row blocks at 129 tokens: 148 + 44).
   // Then the full waves go out unsplit and the rest of the row blocks in a second launch with a split of its own.
-  if (p.DG == 2 && p.RB * p.TT > sms) {
-    const int rows1 = (int)((long long)p.RB * p.TT / sms * sms / p.TT);
+  if (p.DG == 2 && p.RB > sms) {
+    const int rows1 = p.RB / sms * sms;
     double rest;
-    if (rows1 > 0 && rows1 < p.RB) {
+    if (rows1 < p.RB) {
       const int ks2 = best_split(p.RB - rows1, rest);
-      if (estimate(rows1, 1) + rest + 1.0 < whole) { p.RB1 = rows1; p.KS1 = 1; p.KS = ks2; }
+      const double both = estimate(rows1, 1) + rest + 1.0;
+      if (both < us) { p.RB1 = rows1; p.KS1 = 1; p.KS = ks2; us = both; }
     }
   }
   return p;
@@ -662,7 +584,22 @@ void plan_args(GemmArgs& a, const GemmPlan& p) {
   a.astages = p.astages; a.xstages = p.xstages; a.rstages = p.rstages; a.bar_off = p.bar_off; a.tmem_cols = p.tmem_cols;
 }
 
-int dense_launch(const GemmPlan& plan, GemmArgs& a, const CUtensorMap& xmap, const WMaps& wmaps, cudaStream_t stream) {
+// one matrix or a list (a names them, B, the rows of all members as M, NG and the status word)
+int dense_gemm(GemmArgs& a, const WMaps& wmaps, const void* X, const char* who, cudaStream_t stream) {
+  ST_REQUIRE(a.M / 128 * 8 < (1ll << 31), "%s: grid too large", who);
+  double us = 1e30;
+  if (a.B > NT_MAX) return pair_gemm(a, wmaps, X, who, us, stream);
+  const GemmPlan plan = gemm_plan(a.M, a.NG, a.B, us);
+  // From 129 to 320 tokens both kernels fit.  CTA pairs where they are estimated to be clearly faster (the estimates are within
+  // 10 to 15 %; measured, us, this kernel / CTA pairs at 129 and 300 tokens: 2048 x 2048 10.2 / 7.9 and 13.5 / 10.1, 3072 x 2048
+  // 10.6 / 9.7 and 14.1 / 12.9; 4096 x 4096 13.6 / 16.7 and 17.6 / 19.6, 4096 x 12288 25.9 / 35 and 31.8 / 39: few row blocks and
+  // long k ranges, which split over up to eight CTAs here and up to four pairs there)
+  if (plan.DG == 2) {
+    const int done = pair_gemm(a, wmaps, X, who, 0.95 * us, stream);
+    if (done >= 0) return done;
+  }
+  CUtensorMap xmap;
+  if (int e = make_xmap(&xmap, X, a.B, (long long)a.NG * 64, plan.NT > 256 ? plan.NT / 2 : plan.NT, who)) return e;
   GemmPlan p = plan;
   auto go = [&] {
     plan_args(a, p);
@@ -678,21 +615,6 @@ int dense_launch(const GemmPlan& plan, GemmArgs& a, const CUtensorMap& xmap, con
     a.rb0 = plan.RB1;
   }
   return go();
-}
-
-// activations [rows, N] BF16 as boxes of 64 columns x `box_rows` rows with the 128-byte swizzle
-int make_xmap(CUtensorMap* map, const void* X, long long rows, long long N, int box_rows, const char* who) {
-  EncodeTiledFn enc = encode_fn();
-  ST_REQUIRE(enc != nullptr, "%s: cuTensorMapEncodeTiled is not available from the driver", who);
-  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)N * 2};
-  const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1u, 1u};
-  const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  ST_REQUIRE(cr == CUDA_SUCCESS, "%s: cuTensorMapEncodeTiled failed (%d)", who, (int)cr);
-  return 0;
 }
 
 // a tree [M/16][N/64][1552 B] as 194 x u64 rows, boxes of eight row tiles of two column groups
@@ -712,6 +634,21 @@ int make_wmap(CUtensorMap* map, const void* tree, long long M, long long N, cons
 
 }  // namespace
 
+// activations [rows, N] BF16 as boxes of 64 columns x `box_rows` rows with the 128-byte swizzle
+int st::make_xmap(CUtensorMap* map, const void* X, long long rows, long long N, int box_rows, const char* who) {
+  EncodeTiledFn enc = encode_fn();
+  ST_REQUIRE(enc != nullptr, "%s: cuTensorMapEncodeTiled is not available from the driver", who);
+  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)N * 2};
+  const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+  const cuuint32_t estr[2] = {1u, 1u};
+  const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  ST_REQUIRE(cr == CUDA_SUCCESS, "%s: cuTensorMapEncodeTiled failed (%d)", who, (int)cr);
+  return 0;
+}
+
 extern "C" int64_t st_gemm_workspace_bytes(int64_t M, int64_t N, int64_t B) {
   if (M <= 0 || N <= 0 || M % 128 || N % 64 || B < 1) return -1;
   return 0;                                                      // split partial sums stay in shared memory
@@ -724,21 +661,16 @@ extern "C" int st_gemm(const void* tree, const int32_t* eo, const uint32_t* el, 
   ST_REQUIRE(B >= 1 && B < (1ll << 24), "st_gemm: batch out of range");
   ST_REQUIRE(tree && eo && el && X && Y && cnt, "st_gemm: null pointer");
   ST_REQUIRE(st::aligned16(tree) && st::aligned16(X), "st_gemm: tree and X must be 16-byte aligned");
-  const GemmPlan p = gemm_plan(M, N, B);
   (void)ws; (void)ws_bytes;
-  ST_REQUIRE((long long)p.RB * p.TT * p.KS < (1ll << 31), "st_gemm: grid too large");
-  CUtensorMap xmap;
   WMaps wmaps;
   memset(&wmaps, 0, sizeof(wmaps));
-  if (int e = make_xmap(&xmap, X, B, N, p.NT > 256 ? p.NT / 2 : p.NT, "st_gemm")) return e;
   if (int e = make_wmap(&wmaps.m[0], tree, M, N, "st_gemm")) return e;
   GemmArgs a = {};
-  a.tree = (const uint8_t*)tree; a.eo = eo; a.el = el; a.Y = (uint16_t*)Y; a.Yf = Yf32;
+  a.eo = eo; a.el = el; a.Y = (uint16_t*)Y; a.Yf = Yf32;
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "st_gemm: no device status word");
-  a.M = M; a.N = N; a.B = (int)B; a.NG = (int)(N / 64);
-  plan_args(a, p);
-  return dense_launch(p, a, xmap, wmaps, (cudaStream_t)stream);
+  a.M = M; a.B = (int)B; a.NG = (int)(N / 64);
+  return dense_gemm(a, wmaps, X, "st_gemm", (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------------------------- list of matrices
@@ -765,16 +697,11 @@ extern "C" int st_gemm_list(int64_t n, const void* const* trees, const int32_t* 
     a.rbend[i] = (int)(total / 128);
   }
   a.nlist = (int)n;
-  const GemmPlan p = gemm_plan(total, N, B);
-  ST_REQUIRE((long long)p.RB * p.TT * p.KS < (1ll << 31), "%s: grid too large", who);
-  CUtensorMap xmap;
-  if (int e = make_xmap(&xmap, X, B, N, p.NT > 256 ? p.NT / 2 : p.NT, who)) return e;
   a.eo = eo[0]; a.el = el[0]; a.Y = (uint16_t*)Y[0];
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "%s: no device status word", who);
-  a.M = total; a.N = N; a.B = (int)B; a.NG = (int)(N / 64);
-  plan_args(a, p);
-  return dense_launch(p, a, xmap, wmaps, (cudaStream_t)stream);
+  a.M = total; a.B = (int)B; a.NG = (int)(N / 64);
+  return dense_gemm(a, wmaps, X, who, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------------------------- grouped (MoE)
@@ -822,7 +749,7 @@ extern "C" int st_moe_group_gemm(const void* maps, const int64_t* eop, const int
   a.sorted = sorted; a.bexp = bexp; a.npost = npost; a.E = (int)E;
   a.status = st::status_ptr();
   ST_REQUIRE(a.status != nullptr, "st_moe_group_gemm: no device status word");
-  a.M = M; a.N = N; a.B = (int)S; a.NG = (int)(N / 64);
+  a.M = M; a.B = (int)S; a.NG = (int)(N / 64);
   plan_args(a, p);
   return gemm_launch<1, true>(p, a, xmap, unused, (cudaStream_t)stream);
 }

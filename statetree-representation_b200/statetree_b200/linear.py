@@ -27,16 +27,15 @@ GEMV_AR_MAX = 12                    # rows up to which the GEMV that sums over t
 # it, the reference's path above 1024 rows (statetree/linear.py:37, 879-886), here from the size at which it overtakes the
 # tcgen05 kernel; 0 turns it off
 PREFILL_MIN = int(os.environ.get("STATETREE_PREFILL_MIN", "512"))
-# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel for up to FUSED_ROWS rows (six of its token
-# tiles: every tile decodes the records again), and for up to HOST_ROWS rows below DENSE_WEIGHTS weights, where the scratch path,
-# 75 us of Python, events and launches per call, waits for the host.  All projections of a model called one layer after the
-# other, ms with the kernel / the scratch matrix, mean of 50 passes, the paths in turn (they draw on one power budget):
-#   rows                       960          1024         1152         1281         1536         1792         1920         2000
-#   4096 / 12288, 36 layers    13.7 / 15.5  15.9 / 15.6  16.5 / 17.6  20.0 / 19.3  22.0 / 21.0  24.6 / 25.0  25.6 / 25.9  28.5 / 25.7
-# (hidden / intermediate size.)  From 961 to 1920 rows the two change places: the kernel is up to 5 % slower from 961 to 1030, at
-# 1540 and from 1601 to 1860, and up to 12 % faster from 1050 to 1280, where cuBLAS takes one of two times 40 % apart; at 1921 a
-# seventh tile sets it back by 11 %.  5120 / 17408, 20 layers: 14.9 / 14.6 at 1024, 19.6 / 23.0 at 1536, 25.1 / 25.0 at 2000.
-# 2048 / 6144, 28 layers: 3.5 / 7.9 at 1024, 6.6 / 8.0 at 2000 (5.7 with its 25M gate + up on the scratch path).
+# ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel for up to FUSED_ROWS rows, and for up to
+# HOST_ROWS rows below DENSE_WEIGHTS weights, where the scratch path, 75 us of Python, events and launches per call, waits for the
+# host.  These lines are where the two paths met when a tile was one CTA's (all projections of 36 layers of 4096 / 12288, ms with
+# the kernel / the scratch matrix: 960 rows 13.7 / 15.5, 1920 25.6 / 25.9, 2000 28.5 / 25.7).  On CTA pairs the kernel is ahead on
+# both sides of them (us per layer, median of 11 passes, the paths in turn):
+#   rows               513         960         1536        2000        4096         8192
+#   4096 / 12288       196 / 380   301 / 426   486 / 577   642 / 696   1233 / 1388  2587 / 2612
+#   2048 / 6144        86 / 312    100 / 316   133 / 315   164 / 318   348 / 365    682 / 663
+# The lines have stayed: which matrices go through the scratch matrix at which rows is a property that callers' tests rely on.
 FUSED_ROWS, FUSED_WEIGHTS = 1920, 1 << 22
 HOST_ROWS, DENSE_WEIGHTS = 2048, 1 << 24
 DENSE_MAX = 1 << 28                 # weights: larger matrices (vocabulary-sized tables) never get a dense scratch copy
