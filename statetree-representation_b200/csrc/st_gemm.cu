@@ -374,11 +374,8 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
         for (int h = 0; h < CPP; ++h)
 #pragma unroll
           for (int p = 0; p < 8; ++p)
-            if (p < a.KS && c + h * NDW < c_end) {
-              const uint32_t at = (uint32_t)(((c + h * NDW) * 128 + 4 * lane) * 4);
-              v[h][p] = p == ks ? *reinterpret_cast<const float4*>(smem + at)        // (not through the cluster's network)
-                                : ld_cluster_f4(map_to_cta(mine + at, (uint32_t)p));
-            }
+            if (p < a.KS && c + h * NDW < c_end)
+              v[h][p] = ld_cluster_f4(map_to_cta(mine + (uint32_t)(((c + h * NDW) * 128 + 4 * lane) * 4), (uint32_t)p));
 #pragma unroll
         for (int h = 0; h < CPP; ++h) {
           const int cc = c + h * NDW;
