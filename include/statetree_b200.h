@@ -46,8 +46,8 @@ int st_dec(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, i
 int st_rows(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, int64_t N, const int64_t* ids,
             int64_t n, void* out, void* stream);
 
-/* BF16 matrix W [M, N] -> state tree (statetree/format.py:43-83 does this with PyTorch operations), in two passes with the
- * caller's prefix sums between them:
+/* BF16 matrix W [M, N] -> state tree (statetree/format.py:43-83 does this with PyTorch operations), in two passes with
+ * prefix sums between them (the caller's, or st_encode_offsets with a ws of st_encode_offsets_workspace_bytes() bytes):
  *   st_encode        the records; rowcnt uint8 [M, N/64] = escapes of each row's 64 values; reccnt int32 [M/16 * N/64 + 1] =
  *                    0, then the escapes of each record (its inclusive prefix sum is eo)
  *   st_encode_lists  given eo and roff int32 [M, N/64] (inclusive prefix sum of rowcnt, row-major): el and eb as above and the
@@ -56,6 +56,9 @@ int st_rows(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, 
  * from W; st_lists_check adds to it unless the n stored entries rows / cols / bits are the escapes of W in (row, col) order and
  * eo / el / eb the tables of those entries.  Both passed: the tree is lossless as it is read now and as it is stored. */
 int st_encode(const void* W, int64_t M, int64_t N, void* tree, uint8_t* rowcnt, int32_t* reccnt, void* stream);
+int64_t st_encode_offsets_workspace_bytes(int64_t M, int64_t N);
+int st_encode_offsets(const uint8_t* rowcnt, const int32_t* reccnt, int64_t M, int64_t N, int32_t* roff, int32_t* eo, void* ws,
+                      int64_t ws_bytes, void* stream);
 int st_encode_lists(const void* W, int64_t M, int64_t N, const uint8_t* rowcnt, const int32_t* roff, const int32_t* eo,
                     uint32_t* el, uint32_t* eb, int32_t* rows, int32_t* cols, int16_t* bits, void* stream);
 int st_dec_check(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, int64_t N, const void* W, int32_t* bad,

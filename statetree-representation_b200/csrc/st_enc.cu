@@ -2,11 +2,12 @@
 // matrix it was built from.
 //
 // Bound: HBM.  st_encode reads the matrix once (2 B per weight) and writes the records once (1.52 B); the escape passes
-// touch only the records that have escapes.  4096 x 12288 on a B200: st_encode 39 us (177 MB, 4.5 TB/s), the two prefix
-// sums 15 us, st_encode_lists 23 us, st_dec_check 36 us (nothing dense is written back), st_lists_check 8 us (the stored lists and
-// the escape blocks).  TreeLinear.from_weight of that matrix with its checks takes 0.24 ms; with the torch formulation
-// (format._encode_chunk, still the CPU path: ~60 passes over 32- and 64-bit copies, then a sort of the escapes and a dense
-// decode to compare) it took 3.7 ms.
+// touch only the records that have escapes.  4096 x 12288 on a B200, each launch by itself: st_encode 31 us (177 MB, 5.7 TB/s; 37
+// with 4-byte loads), st_encode_offsets 8.5 us (two torch.cumsum with their type conversion 25), st_encode_lists 28 us,
+// st_dec_check 28 us (33 with 4-byte loads; nothing dense is written back), st_lists_check 6 us (the stored lists and the escape
+// blocks).  TreeLinear.from_weight with its checks and one decode of that matrix take 0.21 ms (0.24 before these two); with the
+// torch formulation (format._encode_chunk, still the CPU path: ~60 passes over 32- and 64-bit copies, then a sort of the escapes
+// and a dense decode to compare) 3.7 ms.
 #include "../../include/statetree_b200.h"
 #include "st_encode.cuh"
 #include "st_host.h"
@@ -21,13 +22,14 @@ constexpr int ENC_WARPS = 8;
 __global__ void __launch_bounds__(ENC_WARPS * 32) encode_kernel(const uint16_t* __restrict__ W, long long N, int NG,
                                                                 long long nrec, uint8_t* __restrict__ tree,
                                                                 uint8_t* __restrict__ rowcnt, int* __restrict__ reccnt) {
+  __shared__ __align__(16) uint8_t s_stage[ENC_WARPS][ENC_STAGE];
   const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * ENC_WARPS + (threadIdx.x >> 5);
   if (r == 0 && lane == 0) reccnt[0] = 0;
   if (r >= nrec) return;
   const long long tile = r / NG;
   const int G = (int)(r % NG);
-  const EncFrag e = enc_block(W + tile * 16 * N + (long long)G * 64, N, lane);
+  const EncFrag e = enc_block<true>(W + tile * 16 * N + (long long)G * 64, N, s_stage[threadIdx.x >> 5], lane);
   enc_write(tree + r * REC, e, lane);
   int2 cnt = make_int2(0, 0);
   int total = 0;
@@ -53,6 +55,7 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, 4) encode_lists_kernel(
     const int* __restrict__ roff, const int* __restrict__ eo, uint32_t* __restrict__ el, uint32_t* __restrict__ eb,
     int* __restrict__ rows, int* __restrict__ cols, uint16_t* __restrict__ bits) {
   __shared__ uint32_t s_eb[ENC_WARPS][16];
+  __shared__ __align__(16) uint8_t s_stage[ENC_WARPS][ENC_STAGE];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long u = (long long)blockIdx.x * ENC_WARPS + warp;
   if (u >= units) return;
@@ -68,7 +71,7 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, 4) encode_lists_kernel(
   __syncwarp();
   for (unsigned m = mask; m; m &= m - 1) {
     const int k = __ffs(m) - 1, G = G0 + k;
-    const EncFrag e = enc_block(W + tile * 16 * N + (long long)G * 64, N, lane);
+    const EncFrag e = enc_block<true>(W + tile * 16 * N + (long long)G * 64, N, s_stage[warp], lane);
     const int at = __shfl_sync(FULL, mine, k);                   // first entry of this record
     enc_escapes(e, lane, [&](int before, int in_row, int row, int col, uint32_t val) {
       const uint32_t entry = val << 16 | (uint32_t)(G & 7) << 10 | (uint32_t)row << 6 | (uint32_t)col;
@@ -86,16 +89,95 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, 4) encode_lists_kernel(
   if (lane < 16) eb[u * 16 + lane] = blk[lane];
 }
 
+// Inclusive prefix sums of the two count arrays (rowcnt: n8 bytes -> roff; reccnt: n32 ints -> eo), in two launches without a CTA
+// that waits for another: the sums of chunks of SCAN_CHUNK values, then every CTA adds up the sums before its chunk and scans it.
+// The chunks of rowcnt come first, those of reccnt after them.
+constexpr int SCAN_CHUNK = 4096;                 // 16 values a thread
+struct ScanArgs {
+  const uint8_t* c8; const int* c32; long long n8, n32; int chunks8;
+  int* sums; int* out8; int* out32;
+};
+// this thread's sixteen values of the CTA's chunk (zeros behind the array's end)
+__device__ __forceinline__ void scan_values(const ScanArgs& a, int (&v)[16], long long& at, bool& bytes) {
+  bytes = (int)blockIdx.x < a.chunks8;
+  at = (long long)(bytes ? blockIdx.x : blockIdx.x - a.chunks8) * SCAN_CHUNK + threadIdx.x * 16;
+  if (bytes && at + 16 <= a.n8) {                // (rowcnt is 16-byte aligned, chunks are multiples of 16)
+    const uint4 w = *reinterpret_cast<const uint4*>(a.c8 + at);
+    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = (int)(ws[i >> 2] >> (8 * (i & 3)) & 0xFFu);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    v[i] = bytes ? (at + i < a.n8 ? (int)a.c8[at + i] : 0) : (at + i < a.n32 ? a.c32[at + i] : 0);
+}
+__global__ void __launch_bounds__(256) scan_sums_kernel(const ScanArgs a) {
+  __shared__ int s_sum[8];
+  int v[16], sum = 0;
+  long long at;
+  bool bytes;
+  scan_values(a, v, at, bytes);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) sum += v[i];
+  sum = __reduce_add_sync(FULL, sum);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) sum += s_sum[w];
+    a.sums[blockIdx.x] = sum;
+  }
+}
+__global__ void __launch_bounds__(256) scan_kernel(const ScanArgs a) {
+  __shared__ int s_before[8], s_warp[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int v[16];
+  long long at;
+  bool bytes;
+  scan_values(a, v, at, bytes);
+  int before = 0;                                // the chunks of the same array before this one
+  for (int b = (bytes ? 0 : a.chunks8) + threadIdx.x; b < (int)blockIdx.x; b += 256) before += a.sums[b];
+  before = __reduce_add_sync(FULL, before);
+#pragma unroll
+  for (int i = 1; i < 16; ++i) v[i] += v[i - 1];
+  int upto = v[15];                              // inclusive over the warp's threads
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(FULL, upto, o);
+    if (lane >= o) upto += n;
+  }
+  if (lane == 31) s_warp[warp] = upto;
+  if (lane == 0) s_before[warp] = before;
+  __syncthreads();
+  int add = upto - v[15];
+#pragma unroll
+  for (int w = 0; w < 8; ++w) add += s_before[w] + (w < warp ? s_warp[w] : 0);
+  int* const out = (bytes ? a.out8 : a.out32) + at;
+  const long long left = (bytes ? a.n8 : a.n32) - at;
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) {
+    if (i + 4 <= left) {
+      *reinterpret_cast<int4*>(out + i) = make_int4(v[i] + add, v[i + 1] + add, v[i + 2] + add, v[i + 3] + add);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i + k < left) out[i + k] = v[i + k] + add;
+    }
+  }
+}
+
 // decodes every record and compares it with the matrix; *bad counts the warps that found a difference
 __global__ void __launch_bounds__(256) dec_check_kernel(const uint8_t* __restrict__ tree, const int* __restrict__ eo,
                                                         const uint32_t* __restrict__ el, long long nrec, int NG, long long N,
                                                         const uint16_t* __restrict__ W, int* __restrict__ bad) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  __shared__ __align__(16) uint8_t s_stage[8][ENC_STAGE];
+  const int lane = threadIdx.x & 31;
   const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= nrec) return;
-  uint32_t A[4][4];
-  decode_frag(load_rec_global(tree + r * REC, lane), A);
-  const uint16_t* const src = W + (r / NG) * 16 * N + (r % NG) * 64;
+  uint32_t A[4][4], want[4][4];
+  const RecRegs rec = load_rec_global(tree + r * REC, lane);
+  load_block<true>(want, W + (r / NG) * 16 * N + (r % NG) * 64, N, s_stage[threadIdx.x >> 5], lane);
+  decode_frag(rec, A);
   uint32_t diff = 0;
   const int lo = __ldg(eo + r), hi = __ldg(eo + r + 1);
   for (int base = lo; base < hi; base += 32) {
@@ -106,8 +188,7 @@ __global__ void __launch_bounds__(256) dec_check_kernel(const uint8_t* __restric
 #pragma unroll
   for (int s = 0; s < 4; ++s)
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      diff |= A[s][q] ^ __ldg(reinterpret_cast<const uint32_t*>(src + (g + 8 * (q & 1)) * N + 16 * s + 8 * (q >> 1) + 2 * t));
+    for (int q = 0; q < 4; ++q) diff |= A[s][q] ^ want[s][q];
   if (__any_sync(FULL, diff != 0u) && lane == 0) atomicAdd(bad, 1);
 }
 
@@ -223,5 +304,30 @@ extern "C" int st_lists_check(const int32_t* rows, const int32_t* cols, const in
   lists_check_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       rows, cols, (const uint16_t*)bits, (int)n, eo, el, eb, M, N, NG, CPT, units, (const uint16_t*)W, bad);
   ST_LAUNCH_CHECK("st_lists_check launch");
+  return 0;
+}
+
+extern "C" int64_t st_encode_offsets_workspace_bytes(int64_t M, int64_t N) {
+  if (M <= 0 || N <= 0 || M % 16 || N % 64) return -1;
+  const long long n8 = M * (N / 64), n32 = (M / 16) * (N / 64) + 1;
+  return ((n8 + SCAN_CHUNK - 1) / SCAN_CHUNK + (n32 + SCAN_CHUNK - 1) / SCAN_CHUNK) * 4;
+}
+
+extern "C" int st_encode_offsets(const uint8_t* rowcnt, const int32_t* reccnt, int64_t M, int64_t N, int32_t* roff, int32_t* eo,
+                                 void* ws, int64_t ws_bytes, void* stream) {
+  if (int e = shape_ok("st_encode_offsets", M, N)) return e;
+  ST_REQUIRE(rowcnt && reccnt && roff && eo && ws, "st_encode_offsets: null pointer");
+  ST_REQUIRE(st::aligned16(rowcnt) && st::aligned16(roff) && st::aligned16(eo), "st_encode_offsets: 16-byte alignment");
+  const int64_t need = st_encode_offsets_workspace_bytes(M, N);
+  ST_REQUIRE(ws_bytes >= need, "st_encode_offsets: workspace of %lld bytes needed", (long long)need);
+  ScanArgs a;
+  a.c8 = rowcnt; a.c32 = reccnt; a.n8 = M * (N / 64); a.n32 = (M / 16) * (N / 64) + 1;
+  a.chunks8 = (int)((a.n8 + SCAN_CHUNK - 1) / SCAN_CHUNK);
+  a.sums = (int*)ws; a.out8 = roff; a.out32 = eo;
+  const unsigned grid = (unsigned)(need / 4);
+  scan_sums_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+  ST_LAUNCH_CHECK("st_encode_offsets launch");
+  scan_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+  ST_LAUNCH_CHECK("st_encode_offsets launch");
   return 0;
 }

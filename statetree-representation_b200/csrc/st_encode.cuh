@@ -1,8 +1,8 @@
 // One warp turns a 16 x 64 BF16 block into a state-tree record: shared by the weight encoder and the KV append of whole
 // pages.  The inverse of decode_frag: lane (g, t) holds the block as mma.m16n8k16 A fragments, which is exactly the part of
 // the record it writes (16 + 16 leaf bytes, 16 state bytes), so nothing is exchanged but the row maxima, and the record
-// leaves as three 16-byte stores per lane without shared memory.  (Rows of eight values per lane, bytes placed through
-// shared memory: 57 us for 4096 x 12288, most of it two-byte stores with four-way bank conflicts; this: 39 us.)
+// leaves as three 16-byte stores per lane.  (Rows of eight values per lane, bytes placed through
+// shared memory: 57 us for 4096 x 12288, most of it two-byte stores with four-way bank conflicts; this: 31 us.)
 #pragma once
 #include "st_common.cuh"
 
@@ -15,16 +15,44 @@ struct EncFrag {
   uint32_t esc;          // bit 8 s + 4 r + j: value j (byte order above) of k-step s, row half r, escapes
 };
 
-// src = first value of the block's first row, rows `stride` values apart; 4-byte aligned
-__device__ __forceinline__ EncFrag enc_block(const uint16_t* src, long long stride, int lane) {
-  EncFrag e;
+constexpr int ENC_ROW = 144;                   // staged row: 128 bytes and a pad that keeps ldmatrix free of bank conflicts
+constexpr int ENC_STAGE = 16 * ENC_ROW;        // bytes of shared memory a warp stages a block in
+
+// A 16 x 64 block as mma A fragments.  src = first value of its first row, rows `stride` values apart; 4-byte aligned.
+// Rows that are 16-byte aligned (ALIGNED, or found out here) come as four 16-byte loads per lane and go through `stage`
+// (ENC_STAGE bytes, 16-byte aligned, the warp's own), where ldmatrix picks up the fragments; others as sixteen 4-byte loads of
+// half a sector each.
+template <bool ALIGNED>
+__device__ __forceinline__ void load_block(uint32_t (&A)[4][4], const uint16_t* src, long long stride, uint8_t* stage, int lane) {
+  if (ALIGNED || ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(stride * 2)) & 15u) == 0u) {
+    const uint16_t* const p = src + (lane >> 3) * stride + (lane & 7) * 8;
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const uint4*>(p + 4 * i * stride);
+    uint8_t* const to = stage + (lane >> 3) * ENC_ROW + (lane & 7) * 16;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(to + 4 * i * ENC_ROW) = v[i];
+    __syncwarp();
+    // lane l names row l % 16 of the two 8-column halves l / 16: matrices in the order of the fragment registers
+    const uint32_t from = smem_addr(stage) + (uint32_t)((lane & 15) * ENC_ROW + (lane >> 4) * 16);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) ldmatrix_x4(from + 32 * s, A[s][0], A[s][1], A[s][2], A[s][3]);
+    __syncwarp();                                                // (the stage is reused)
+    return;
+  }
   const uint16_t* const p0 = src + (lane >> 2) * stride + 2 * (lane & 3);
   const uint16_t* const p1 = p0 + 8 * stride;
 #pragma unroll
   for (int s = 0; s < 4; ++s)
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      e.A[s][q] = *reinterpret_cast<const uint32_t*>(((q & 1) ? p1 : p0) + 16 * s + 8 * (q >> 1));
+      A[s][q] = *reinterpret_cast<const uint32_t*>(((q & 1) ? p1 : p0) + 16 * s + 8 * (q >> 1));
+}
+
+template <bool ALIGNED>
+__device__ __forceinline__ EncFrag enc_block(const uint16_t* src, long long stride, uint8_t* stage, int lane) {
+  EncFrag e;
+  load_block<ALIGNED>(e.A, src, stride, stage, lane);
   e.esc = 0u;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {

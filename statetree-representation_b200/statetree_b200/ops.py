@@ -27,6 +27,8 @@ _SIGNATURES = {
     "st_argmax": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "st_encode": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "st_encode_lists": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "st_encode_offsets_workspace_bytes": (_i64, [_i64, _i64]),
+    "st_encode_offsets": (_int, [_vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _vp]),
     "st_dec_check": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
     "st_lists_check": (_int, [_vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
     "st_gemv_workspace_bytes": (_i64, [_i64, _i64, _i64]),
@@ -184,10 +186,14 @@ class _Weights:
         tree = torch.empty(M // 16, N // 64, 1552, dtype=torch.uint8, device=dev)
         rowcnt = torch.empty(M * (N // 64), dtype=torch.uint8, device=dev)
         reccnt = torch.empty(nrec + 1, dtype=torch.int32, device=dev)
+        eo = torch.empty(nrec + 1, dtype=torch.int32, device=dev)
+        roff = torch.empty(M * (N // 64), dtype=torch.int32, device=dev)
+        need = int(lib().st_encode_offsets_workspace_bytes(M, N))
+        ws = torch.empty(need, dtype=torch.uint8, device=dev)
         with _ctx(W):
-            _check(lib().st_encode(_ptr(W), M, N, _ptr(tree), _ptr(rowcnt), _ptr(reccnt), _stream(W)))
-            eo = reccnt.cumsum(0, dtype=torch.int32)
-            roff = rowcnt.cumsum(0, dtype=torch.int32)
+            stream = _stream(W)
+            _check(lib().st_encode(_ptr(W), M, N, _ptr(tree), _ptr(rowcnt), _ptr(reccnt), stream))
+            _check(lib().st_encode_offsets(_ptr(rowcnt), _ptr(reccnt), M, N, _ptr(roff), _ptr(eo), _ptr(ws), need, stream))
             n = int(eo[-1])                              # (synchronises: the lists' length depends on the data)
             rows, cols = (torch.empty(n, dtype=torch.int32, device=dev) for _ in range(2))
             bits = torch.empty(n, dtype=torch.int16, device=dev)
@@ -196,7 +202,7 @@ class _Weights:
             spare = el                                   # (no escapes: empty tensors have no address; nothing is written)
             _check(lib().st_encode_lists(_ptr(W), M, N, _ptr(rowcnt), _ptr(roff), _ptr(eo), _ptr(el), _ptr(eb),
                                          _ptr(rows if n else spare), _ptr(cols if n else spare), _ptr(bits if n else spare),
-                                         _stream(W)))
+                                         stream))
         return tree, rows, cols, bits, (eo, el, eb)
 
     @staticmethod
