@@ -588,36 +588,77 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
   bool xready = !a.xwhole;
   if (MODE == MODE_NORM) {
     // x + delta -> new residual stream (BF16), its RMSNorm times the norm weights -> this CTA's activation rows.  The
-    // eight consumer warps share the work: 16-byte vectors, thread t takes vectors t, t + 256, ...
+    // eight consumer warps share the work: 16-byte vectors, thread t takes vectors t, t + 256, ... of every row.  Every CTA does
+    // all of it, so what counts is the number of dependent trips to L2: the vectors of four (row, vector) steps are requested
+    // together, and the norm weights with the first of them.  (Each step's loads behind the step before, the norm weights in the
+    // second loop: 6144 x 4096 at 4 rows, by itself, 18.5 us and now 15.2 to 16.4, 24576 x 4096 37.3 / 34.2; a decode step of four
+    // layers 357 / 348.)
     pdl_wait();
-    const int ct = warp * 32 + lane, nvec = (int)(a.N / 8);
+    const int ct = warp * 32 + lane, nvec = (int)(a.N / 8), per_row = (nvec + CW * 32 - 1) / (CW * 32);
     float* part = red;                                         // [rows][CW] partial sums of squares (red is still idle)
-    for (int b = 0; b < a.B; ++b) {
-      float ss = 0.f;
-      for (int v = ct; v < nvec; v += CW * 32) {
-        uint4 xv = *reinterpret_cast<const uint4*>(a.X + (size_t)b * a.N + (size_t)v * 8);
-        if (a.delta != nullptr) {
-          const uint4 dv = *reinterpret_cast<const uint4*>(a.delta + (size_t)b * a.N + (size_t)v * 8);
-          const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, ds[4] = {dv.x, dv.y, dv.z, dv.w};
-          uint32_t so[4];
+    constexpr int NWK = 2;                                     // norm-weight vectors kept in registers (rows of up to 4096)
+    uint4 gv[NWK];
+    int b0 = 0, i0 = 0;                                        // row and vector step of the batch's first element
+    float ss = 0.f;
+    for (int left = a.B * per_row; left > 0; left -= 4) {
+      uint4 xv[4], dv[4];
+      int row = b0, step = i0;
 #pragma unroll
-          for (int q = 0; q < 4; ++q)                           // the residual stream stays BF16
-            so[q] = pack_bf16(__uint_as_float(xs[q] << 16) + __uint_as_float(ds[q] << 16),
-                              __uint_as_float(xs[q] & 0xFFFF0000u) + __uint_as_float(ds[q] & 0xFFFF0000u));
-          xv = make_uint4(so[0], so[1], so[2], so[3]);
+      for (int q = 0; q < 4; ++q) {
+        const int v = ct + step * (CW * 32);
+        xv[q] = dv[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (q < left && v < nvec) {
+          xv[q] = *reinterpret_cast<const uint4*>(a.X + (size_t)row * a.N + (size_t)v * 8);
+          if (a.delta != nullptr) dv[q] = *reinterpret_cast<const uint4*>(a.delta + (size_t)row * a.N + (size_t)v * 8);
         }
-        if (blockIdx.x == 0 && a.xout != nullptr) *reinterpret_cast<uint4*>(a.xout + (size_t)b * a.N + (size_t)v * 8) = xv;
-        *reinterpret_cast<uint4*>(xw + (size_t)b * a.xw_stride + (size_t)v * 16) = xv;
-        const uint32_t ws_[4] = {xv.x, xv.y, xv.z, xv.w};
+        if (++step == per_row) { step = 0; ++row; }
+      }
+      if (b0 == 0 && i0 == 0) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float lo = __uint_as_float(ws_[q] << 16), hi = __uint_as_float(ws_[q] & 0xFFFF0000u);
-          ss += lo * lo + hi * hi;
+        for (int k = 0; k < NWK; ++k)
+          if (ct + k * (CW * 32) < nvec) gv[k] = *reinterpret_cast<const uint4*>(a.nw + (size_t)(ct + k * (CW * 32)) * 8);
+      }
+      float done[4];                                           // a row's sum of this thread, where the row ends
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int v = ct + i0 * (CW * 32);
+        done[q] = 0.f;
+        if (q < left) {
+          if (a.delta != nullptr) {
+            const uint32_t xs[4] = {xv[q].x, xv[q].y, xv[q].z, xv[q].w}, ds[4] = {dv[q].x, dv[q].y, dv[q].z, dv[q].w};
+            uint32_t so[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)                         // the residual stream stays BF16
+              so[k] = pack_bf16(__uint_as_float(xs[k] << 16) + __uint_as_float(ds[k] << 16),
+                                __uint_as_float(xs[k] & 0xFFFF0000u) + __uint_as_float(ds[k] & 0xFFFF0000u));
+            xv[q] = make_uint4(so[0], so[1], so[2], so[3]);
+          }
+          if (v < nvec) {
+            if (blockIdx.x == 0 && a.xout != nullptr) *reinterpret_cast<uint4*>(a.xout + (size_t)b0 * a.N + (size_t)v * 8) = xv[q];
+            *reinterpret_cast<uint4*>(xw + (size_t)b0 * a.xw_stride + (size_t)v * 16) = xv[q];
+            const uint32_t ws_[4] = {xv[q].x, xv[q].y, xv[q].z, xv[q].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float lo = __uint_as_float(ws_[k] << 16), hi = __uint_as_float(ws_[k] & 0xFFFF0000u);
+              ss += lo * lo + hi * hi;
+            }
+          }
+          if (i0 + 1 == per_row) { done[q] = ss; ss = 0.f; }
+          if (++i0 == per_row) { i0 = 0; ++b0; }
         }
       }
 #pragma unroll
-      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(FULL, ss, o);
-      if (lane == 0) part[b * CW + warp] = ss;
+      for (int o = 16; o; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) done[q] += __shfl_xor_sync(FULL, done[q], o);
+      // rows that ended in this batch: b0 has moved past them
+      int end = b0, st = i0;
+#pragma unroll
+      for (int q = 3; q >= 0; --q)
+        if (q < left) {
+          if (st == 0) { st = per_row; --end; if (lane == 0) part[end * CW + warp] = done[q]; }
+          --st;
+        }
     }
     asm volatile("bar.sync 2, %0;" :: "n"(CW * 32) : "memory");
     for (int b = 0; b < a.B; ++b) {
@@ -625,11 +666,10 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
 #pragma unroll
       for (int i = 0; i < CW; ++i) tot += part[b * CW + i];
       const float r = rsqrtf(tot / (float)a.N + a.eps);
-      for (int v = ct; v < nvec; v += CW * 32) {
+      auto scale = [&](int v, const uint4 g) {
         uint4* slot = reinterpret_cast<uint4*>(xw + (size_t)b * a.xw_stride + (size_t)v * 16);
         const uint4 xv = *slot;
-        const uint4 gv = *reinterpret_cast<const uint4*>(a.nw + (size_t)v * 8);
-        const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, gs[4] = {gv.x, gv.y, gv.z, gv.w};
+        const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, gs[4] = {g.x, g.y, g.z, g.w};
         uint32_t o[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {                           // normalised value rounded, then scaled
@@ -638,7 +678,11 @@ __global__ void __launch_bounds__((CW + 2) * 32, NT <= 2 ? 2 : 1) gemv_kernel(co
                            __uint_as_float(n & 0xFFFF0000u) * __uint_as_float(gs[q] & 0xFFFF0000u));
         }
         *slot = make_uint4(o[0], o[1], o[2], o[3]);
-      }
+      };
+#pragma unroll
+      for (int k = 0; k < NWK; ++k)
+        if (ct + k * (CW * 32) < nvec) scale(ct + k * (CW * 32), gv[k]);
+      for (int v = ct + NWK * (CW * 32); v < nvec; v += CW * 32) scale(v, *reinterpret_cast<const uint4*>(a.nw + (size_t)v * 8));
     }
     asm volatile("bar.sync 2, %0;" :: "n"(CW * 32) : "memory");
     xready = true;
