@@ -3,17 +3,20 @@
     python statetree-representation_b200/build.py [--force]
 
 nvcc cross-compiles without a GPU.  Objects are compiled in parallel and linked into
-statetree_b200/libstatetree_b200.so next to the Python package (git-ignored; it travels with the working tree).
+statetree_b200/libstatetree_b200.so next to the Python package (git-ignored; it travels with the working tree).  Beside it
+statetree_b200/_calls.so, the host path of module calls (csrc/py_calls.cpp, C++ against this interpreter's torch).
 """
 import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "statetree_b200", "libstatetree_b200.so")
+CALLS = os.path.join(HERE, "statetree_b200", "_calls.so")
 OBJ = os.path.join(HERE, "build")
 NVCC_FLAGS = ["-Wno-deprecated-gpu-targets", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr"]
@@ -55,7 +58,25 @@ def build_library(force=False, verbose=False, defines=(), out=None):
     return out
 
 
+def build_calls(force=False):
+    """_calls.so from csrc/py_calls.cpp"""
+    src = os.path.join(CSRC, "py_calls.cpp")
+    if force or _stale(CALLS, [src]):
+        import torch
+        root = os.path.dirname(torch.__file__)
+        cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+        dirs = [f"{root}/include", f"{root}/include/torch/csrc/api/include", f"{cuda}/include", sysconfig.get_paths()["include"]]
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+        cmd += [a for d in dirs for a in ("-isystem", d)] + [src, "-o", CALLS, f"-L{root}/lib"]
+        r = subprocess.run(cmd + ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"{cmd[0]} failed on {src}:\n{r.stdout}\n{r.stderr}")
+    return CALLS
+
+
 if __name__ == "__main__":
     defs = [a[2:] for a in sys.argv[1:] if a.startswith("-D")]
     outs = [a[6:] for a in sys.argv[1:] if a.startswith("--out=")]
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv, defines=defs, out=outs[0] if outs else None))
+    print(build_calls(force="--force" in sys.argv))

@@ -5,8 +5,8 @@
 // touch only the records that have escapes.  4096 x 12288 on a B200, each launch by itself: st_encode 31 us (177 MB, 5.7 TB/s; 37
 // with 4-byte loads), st_encode_offsets 8.5 us (two torch.cumsum with their type conversion 25), st_encode_lists 28 us,
 // st_dec_check 28 us (33 with 4-byte loads; nothing dense is written back), st_lists_check 6 us (the stored lists and the escape
-// blocks).  TreeLinear.from_weight with its checks and one decode of that matrix take 0.21 ms (0.24 before these two); with the
-// torch formulation (format._encode_chunk, still the CPU path: ~60 passes over 32- and 64-bit copies, then a sort of the escapes
+// blocks).  TreeLinear.from_weight with its checks and one decode of that matrix take 0.18 ms; with the torch formulation
+// (format._encode_chunk, still the CPU path: ~60 passes over 32- and 64-bit copies, then a sort of the escapes
 // and a dense decode to compare) 3.7 ms.
 #include "../../include/statetree_b200.h"
 #include "st_encode.cuh"

@@ -17,7 +17,7 @@ import torch
 import torch.nn as nn
 
 from . import format as F
-from .ops import _raw_stream, built, ext, on_device
+from .ops import _raw_stream, built, calls, ext, on_device
 
 # activation rows up to which the GEMV kernel runs (<= 32).  The four projections of a 4096 / 12288 layer in a graph, us with
 # the GEMV / the tcgen05 GEMM: 8 rows 57 / 72, 16 rows 68 / 72, 20 rows 125 / 72 (beyond 16 the GEMV holds one CTA per SM)
@@ -286,7 +286,12 @@ class TreeLinear(nn.Module):
                 raise EscapeHeavy(f"{escapes / W.numel():.2%} of the weights escape")
         on_gpu = (W.is_cuda and W.dim() == 2 and W.numel() > 0 and W.shape[0] % 16 == 0 and W.shape[1] % 64 == 0 and built())
         enc, tables = F.encode_with_tables(W) if on_gpu else (F.encode(W), None)
-        out_features, in_features = W.shape
+        if verify and on_gpu:
+            # (what is stored is checked, not only the tables of this process: a reload builds its tables from the lists)
+            bad = ext().check_start(enc["tree"], tables[0], tables[1],
+                                    W if W.data_ptr() % 16 == 0 and W.is_contiguous() else W.clone(memory_format=torch.contiguous_format),
+                                    (enc["esc_rows"], enc["esc_cols"], enc["esc_bits"], tables[2]))
+        out_features, in_features = W.shape             # (the module is made while the check runs)
         layer = cls(in_features, out_features, bias=bias is not None, device="meta", n_esc=int(enc["esc_rows"].numel()))
         layer._buffers.update({name: enc[name] for name in _BUFFERS})
         if bias is not None:
@@ -294,10 +299,7 @@ class TreeLinear(nn.Module):
         layer._reset_runtime()
         if verify:
             if on_gpu:
-                # (what is stored is checked, not only the tables of this process: a reload builds its tables from the lists)
-                same = ext().dec_check(enc["tree"], tables[0], tables[1],
-                                       W if W.data_ptr() % 16 == 0 and W.is_contiguous() else W.clone(memory_format=torch.contiguous_format),
-                                       (enc["esc_rows"], enc["esc_cols"], enc["esc_bits"], tables[2]))
+                same = int(bad) == 0
             else:
                 back = layer.dequantize() if layer.tree.is_cuda else F.decode_reference(*(layer._buffers[n] for n in _BUFFERS))
                 same = torch.equal(back.view(torch.int16), W.view(torch.int16))
@@ -417,12 +419,35 @@ class TreeLinear(nn.Module):
             return torch.ops.statetree.linear(x, self.tree, self._handle)
         return self._forward(x)
 
+    def _plain(self, x, home):
+        """the product in one native call, for inputs that need no conversion (BF16 rows on the layer's device, see
+        csrc/py_calls.cpp) and no bias; None for the others and for batches that go through the scratch matrix"""
+        M, N = self.out_features, self.in_features
+        if self.bias is not None or x.dim() == 0 or x.shape[-1] != N:
+            return None
+        B = x.numel() // N
+        eo, el, eb = self.tables()
+        if B <= min(GEMV_MAX, 32):
+            use_gemm, st = False, _state(home)
+            ws, cnt = st.gemv_ws(M, N, max(B, 1)), st.get_cnt(M // 16)
+        elif M % 128 == 0 and not self.dense_for(B):
+            use_gemm, st = True, _state(home)
+            ws, cnt = st.scratch, st.get_cnt((M // 128) * ((B + 255) // 256))     # (the GEMM asks for no workspace)
+        else:
+            return None
+        native, library = calls()
+        return native.linear(library, use_gemm, self._buffers["tree"], eo, el, eb, x, ws, cnt)
+
     def _forward(self, x, yf32=None):
         """any leading shape, any float dtype, any device: the product runs where the tree lives, in BF16, and comes
         back in the caller's dtype on the caller's device"""
         home, asked_dtype, asked_device = self._buffers["tree"].device, x.dtype, x.device
         if home.type != "cuda":
             raise RuntimeError("statetree_b200: the kernels take CUDA tensors only (no CPU path); move the layer to a GPU")
+        if yf32 is None:
+            result = self._plain(x, home)
+            if result is not None:
+                return result
         lead = x.shape[:-1]
         acts = _rows_2d(x if asked_device == home else x.to(home), self.in_features)
         result = torch.empty(acts.shape[0], self.out_features, dtype=torch.bfloat16, device=home)
@@ -488,8 +513,15 @@ def forward_list(layers, x):
             or (use_gemm and any(l.out_features % 128 for l in layers))):
         return [l(x) for l in layers]
     here = x.device == home
-    acts = _rows_2d(x if here else x.to(home), width)
     widths = [l.out_features for l in layers]
+    if here and x.shape[-1] == width and all(l.bias is None for l in layers):
+        st = _state(home)                               # one native call for inputs that need no conversion
+        scratch = (st.get_cnt((sum(widths) // 128) * ((B + 255) // 256)) if use_gemm else st.gemv_ws(tuple(widths), width, B))
+        native, library = calls()
+        res = native.linear_list(library, use_gemm, trees, [l.tables() for l in layers], x, scratch)
+        if res is not None:
+            return res
+    acts = _rows_2d(x if here else x.to(home), width)
     # one allocation, a contiguous [B, width] block per layer
     flat = torch.empty(B * sum(widths), dtype=torch.bfloat16, device=home)
     parts = flat.split([B * w for w in widths])

@@ -4,6 +4,7 @@ reference's extension modules: ext() stands where `statetree._C` stood and kv_ex
 torch's current stream of the tensors' device.  There is no fallback: a missing library or a non-CUDA tensor raises.
 """
 import ctypes
+import importlib.util
 import os
 
 import torch
@@ -109,6 +110,27 @@ def lib():
     return _LIB
 
 
+_CALLS = None
+
+
+def calls():
+    """(the native module of csrc/py_calls.cpp, the entry points of the loaded library for it): the host path of plain module
+    calls.  Raises when it has not been built."""
+    global _CALLS
+    if _CALLS is None:
+        L = lib()
+        path = os.path.join(_HERE, "_calls.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"statetree_b200: {path} is missing; build it with `python statetree-representation_b200/build.py`")
+        spec = importlib.util.spec_from_file_location("_calls", path)
+        native = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(native)
+        names = ("st_gemv", "st_gemm", "st_gemv_list", "st_gemm_list", "st_last_error", "st_encode", "st_encode_lists",
+                 "st_encode_offsets", "st_encode_offsets_workspace_bytes", "st_dec_check", "st_lists_check")
+        _CALLS = native, native.library({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names})
+    return _CALLS
+
+
 def _ptr(t):
     if t is None:
         return None
@@ -181,43 +203,21 @@ class _Weights:
     @staticmethod
     def encode(W):
         """W [M, N] BF16 on a GPU -> (tree, rows, cols, bits, (eo, el, eb)): the format's parts and the kernels' side tables"""
-        M, N = W.shape
-        dev, nrec = W.device, (M // 16) * (N // 64)
-        tree = torch.empty(M // 16, N // 64, 1552, dtype=torch.uint8, device=dev)
-        rowcnt = torch.empty(M * (N // 64), dtype=torch.uint8, device=dev)
-        reccnt = torch.empty(nrec + 1, dtype=torch.int32, device=dev)
-        eo = torch.empty(nrec + 1, dtype=torch.int32, device=dev)
-        roff = torch.empty(M * (N // 64), dtype=torch.int32, device=dev)
-        need = int(lib().st_encode_offsets_workspace_bytes(M, N))
-        ws = torch.empty(need, dtype=torch.uint8, device=dev)
-        with _ctx(W):
-            stream = _stream(W)
-            _check(lib().st_encode(_ptr(W), M, N, _ptr(tree), _ptr(rowcnt), _ptr(reccnt), stream))
-            _check(lib().st_encode_offsets(_ptr(rowcnt), _ptr(reccnt), M, N, _ptr(roff), _ptr(eo), _ptr(ws), need, stream))
-            n = int(eo[-1])                              # (synchronises: the lists' length depends on the data)
-            rows, cols = (torch.empty(n, dtype=torch.int32, device=dev) for _ in range(2))
-            bits = torch.empty(n, dtype=torch.int16, device=dev)
-            el = torch.empty(n, dtype=torch.int32, device=dev) if n else torch.zeros(1, dtype=torch.int32, device=dev)
-            eb = torch.empty((M // 16) * ((N // 64 + 7) // 8), 16, dtype=torch.int32, device=dev)
-            spare = el                                   # (no escapes: empty tensors have no address; nothing is written)
-            _check(lib().st_encode_lists(_ptr(W), M, N, _ptr(rowcnt), _ptr(roff), _ptr(eo), _ptr(el), _ptr(eb),
-                                         _ptr(rows if n else spare), _ptr(cols if n else spare), _ptr(bits if n else spare),
-                                         stream))
+        native, library = calls()
+        tree, rows, cols, bits, eo, el, eb = native.encode(library, W)
         return tree, rows, cols, bits, (eo, el, eb)
 
     @staticmethod
     def dec_check(T, EO, EL, W, stored=None):
         """does the tree decode to W [M, N] BF16 exactly (synchronises).  stored = (rows, cols, bits, EB): the format's lists
         and the GEMV's escape blocks are checked too"""
-        M, N = W.shape
-        bad = torch.zeros(1, dtype=torch.int32, device=W.device)
-        with _ctx(T):
-            _check(lib().st_dec_check(_ptr(T), _ptr(EO), _ptr(EL), M, N, _ptr(W), _ptr(bad), _stream(T)))
-            if stored is not None:
-                rows, cols, bits, EB = stored
-                _check(lib().st_lists_check(_ptr(rows), _ptr(cols), _ptr(bits), rows.numel(), _ptr(EO), _ptr(EL), _ptr(EB), M, N,
-                                            _ptr(W), _ptr(bad), _stream(T)))
-            return int(bad) == 0
+        return int(_Weights.check_start(T, EO, EL, W, stored)) == 0
+
+    @staticmethod
+    def check_start(T, EO, EL, W, stored=None):
+        """launches that check: an int32 tensor that will hold zero if all is well"""
+        native, library = calls()
+        return native.check_start(library, T, EO, EL, W, [] if stored is None else list(stored))
 
     @staticmethod
     def rows(T, EO, EL, ids, out):

@@ -1,0 +1,98 @@
+"""The native host path of module calls (csrc/py_calls.cpp) against the general path of linear.py, over the forms an input can have:
+the same bits, shapes and types where both take it, the same errors where neither does."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+class _General:
+    """stands in for the native module: takes nothing, so every call goes the general way"""
+    linear = linear_list = staticmethod(lambda *a: None)
+
+
+def _layers(Ms, N, bias=False):
+    from statetree_b200 import TreeLinear
+    g = torch.Generator(DEV).manual_seed(sum(Ms) + N)
+    out = []
+    for M in Ms:
+        W = (torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+        b = torch.randn(M, device=DEV, generator=g).to(torch.bfloat16) if bias else None
+        out.append(TreeLinear.from_weight(W, b))
+    return out
+
+
+def _forms(N):
+    """name -> input of width N"""
+    g = torch.Generator(DEV).manual_seed(N)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)                                     # noqa: E731
+    bf = lambda *s: r(*s).to(torch.bfloat16)                                                    # noqa: E731
+    wide = bf(6, 2 * N)
+    flat = bf(5 * N + 8)
+    return {"one": bf(1, N), "vector": bf(N), "three": bf(3, N), "lead": bf(2, 1, 3, N), "gemv_last": bf(16, N), "gemm_first": bf(17, N),
+            "gemm": bf(2, 65, N), "pairs": bf(331, N), "scratch": bf(600, N), "no_rows": bf(0, N), "no_rows_lead": bf(2, 0, N),
+            "float": r(3, N), "half": r(3, N).half(), "strided": wide[:, :N], "columns": bf(N, 4).t(), "expanded": bf(1, N).expand(4, N),
+            "offset_2": flat[1:1 + 5 * N].view(5, N), "offset_16": flat[8:8 + 5 * N].view(5, N), "cpu": bf(3, N).cpu(),
+            "grad": bf(3, N).requires_grad_()}
+
+
+def _both(monkeypatch, call):
+    import statetree_b200.linear as L
+    got = call()
+    with monkeypatch.context() as m:
+        m.setattr(L, "calls", lambda: (_General, None))
+        want = call()
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and a.device == b.device and a.shape == b.shape and a.stride() == b.stride()
+        assert not a.requires_grad and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("Ms,N,bias", [((128,), 64, False), ((256,), 512, False), ((256,), 512, True), ((48,), 128, False)])
+def test_layer_calls(Ms, N, bias, monkeypatch):
+    from statetree_b200 import ops
+    tl, = _layers(Ms, N, bias)
+    for name, x in _forms(N).items():
+        _both(monkeypatch, lambda: [tl(x)])
+    for bad in (torch.zeros(4, 2 * N), torch.zeros(2 * N), torch.zeros(4, N // 2)):
+        with pytest.raises(RuntimeError):
+            tl(bad.to(DEV, torch.bfloat16))
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("Ms,N,bias", [((128, 128), 64, False), ((256, 128, 384), 512, False), ((256, 128), 512, True),
+                                       ((48, 16, 32, 64), 128, False)])
+def test_list_calls(Ms, N, bias, monkeypatch):
+    from statetree_b200 import ops
+    from statetree_b200.linear import forward_list
+    tls = _layers(Ms, N, bias)
+    for name, x in _forms(N).items():
+        if x.dim() > 1:
+            _both(monkeypatch, lambda: forward_list(tls, x))
+    with pytest.raises(RuntimeError):
+        forward_list(tls, torch.zeros(4, 2 * N, dtype=torch.bfloat16, device=DEV))
+    assert ops.device_status() == 0
+
+
+def test_calls_in_a_graph_and_on_another_stream(monkeypatch):
+    """outputs come from the capture's pool and the kernels go to the current stream"""
+    from statetree_b200.linear import forward_list
+    tls = _layers((256, 128), 512)
+    x = torch.empty(3, 512, dtype=torch.bfloat16, device=DEV)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call = lambda: forward_list(tls, x) + [tls[0](x)]                                       # noqa: E731
+        x.normal_()
+        call()
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = call()
+        for _ in range(3):
+            x.normal_()
+            graph.replay()
+            side.synchronize()
+            for a, b in zip(out, call()):
+                assert torch.equal(a, b)
+        side.synchronize()
