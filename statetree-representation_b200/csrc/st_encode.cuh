@@ -22,22 +22,33 @@ constexpr int ENC_STAGE = 16 * ENC_ROW;        // bytes of shared memory a warp 
 // Rows that are 16-byte aligned (ALIGNED, or found out here) come as four 16-byte loads per lane and go through `stage`
 // (ENC_STAGE bytes, 16-byte aligned, the warp's own), where ldmatrix picks up the fragments; others as sixteen 4-byte loads of
 // half a sector each.
+__device__ __forceinline__ bool block_aligned(const uint16_t* src, long long stride) {
+  return ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(stride * 2)) & 15u) == 0u;
+}
+// the two halves of the aligned form: the loads (a caller may have other look-ups in flight with them), then the fragments
+__device__ __forceinline__ void request_block(uint4 (&v)[4], const uint16_t* src, long long stride, int lane) {
+  const uint16_t* const p = src + (lane >> 3) * stride + (lane & 7) * 8;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const uint4*>(p + 4 * i * stride);
+}
+__device__ __forceinline__ void place_block(uint32_t (&A)[4][4], const uint4 (&v)[4], uint8_t* stage, int lane) {
+  uint8_t* const to = stage + (lane >> 3) * ENC_ROW + (lane & 7) * 16;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(to + 4 * i * ENC_ROW) = v[i];
+  __syncwarp();
+  // lane l names row l % 16 of the two 8-column halves l / 16: matrices in the order of the fragment registers
+  const uint32_t from = smem_addr(stage) + (uint32_t)((lane & 15) * ENC_ROW + (lane >> 4) * 16);
+#pragma unroll
+  for (int s = 0; s < 4; ++s) ldmatrix_x4(from + 32 * s, A[s][0], A[s][1], A[s][2], A[s][3]);
+  __syncwarp();                                                  // (the stage is reused)
+}
+
 template <bool ALIGNED>
 __device__ __forceinline__ void load_block(uint32_t (&A)[4][4], const uint16_t* src, long long stride, uint8_t* stage, int lane) {
-  if (ALIGNED || ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(stride * 2)) & 15u) == 0u) {
-    const uint16_t* const p = src + (lane >> 3) * stride + (lane & 7) * 8;
+  if (ALIGNED || block_aligned(src, stride)) {
     uint4 v[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const uint4*>(p + 4 * i * stride);
-    uint8_t* const to = stage + (lane >> 3) * ENC_ROW + (lane & 7) * 16;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(to + 4 * i * ENC_ROW) = v[i];
-    __syncwarp();
-    // lane l names row l % 16 of the two 8-column halves l / 16: matrices in the order of the fragment registers
-    const uint32_t from = smem_addr(stage) + (uint32_t)((lane & 15) * ENC_ROW + (lane >> 4) * 16);
-#pragma unroll
-    for (int s = 0; s < 4; ++s) ldmatrix_x4(from + 32 * s, A[s][0], A[s][1], A[s][2], A[s][3]);
-    __syncwarp();                                                // (the stage is reused)
+    request_block(v, src, stride, lane);
+    place_block(A, v, stage, lane);
     return;
   }
   const uint16_t* const p0 = src + (lane >> 2) * stride + 2 * (lane & 3);
@@ -49,10 +60,8 @@ __device__ __forceinline__ void load_block(uint32_t (&A)[4][4], const uint16_t* 
       A[s][q] = *reinterpret_cast<const uint32_t*>(((q & 1) ? p1 : p0) + 16 * s + 8 * (q >> 1));
 }
 
-template <bool ALIGNED>
-__device__ __forceinline__ EncFrag enc_block(const uint16_t* src, long long stride, uint8_t* stage, int lane) {
-  EncFrag e;
-  load_block<ALIGNED>(e.A, src, stride, stage, lane);
+// e.A -> the rest of the fragment
+__device__ __forceinline__ void enc_finish(EncFrag& e) {
   e.esc = 0u;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -80,6 +89,13 @@ __device__ __forceinline__ EncFrag enc_block(const uint16_t* src, long long stri
       e.state[s][r] = st;
     }
   }
+}
+
+template <bool ALIGNED>
+__device__ __forceinline__ EncFrag enc_block(const uint16_t* src, long long stride, uint8_t* stage, int lane) {
+  EncFrag e;
+  load_block<ALIGNED>(e.A, src, stride, stage, lane);
+  enc_finish(e);
   return e;
 }
 

@@ -103,12 +103,12 @@ struct ChainTail {
 
 // A page that starts over: the unit's old chain, if it has one and `reuse` asks to keep it, is emptied (its links stay);
 // returns its first block, -1 = none.  Whole warp.
-__device__ __forceinline__ int recycle_chain(const AppendArgs& a, const uint8_t* grec, int lane) {
+__device__ __forceinline__ uint32_t old_header(const AppendArgs& a, const uint8_t* grec) {
+  return a.reuse ? *reinterpret_cast<const volatile uint32_t*>(grec + REC) : 0u;
+}
+__device__ __forceinline__ int recycle_chain(const AppendArgs& a, const uint32_t was, int lane) {
   int chain = -1;
-  if (a.reuse) {
-    const uint32_t was = *reinterpret_cast<const volatile uint32_t*>(grec + REC);
-    if ((was & 16u) && (int)(was >> 8) < a.P) chain = (int)(was >> 8);
-  }
+  if ((was & 16u) && (int)(was >> 8) < a.P) chain = (int)(was >> 8);
   if (chain >= 0 && lane == 0) {
     int b = chain;
     for (int hops = 0; b >= 0 && b < a.P && hops < 4096; ++hops) {
@@ -149,11 +149,17 @@ __device__ __forceinline__ void place_entries(const AppendArgs& a, uint8_t* cons
 
 // A whole page of one unit at once: sixteen rows of 64 values, `stride` values apart, encoded like a weight record instead of
 // row by row.  The same bytes as append_rows: entries are queued in row-major, column order.
-// 8192 tokens x 8 KV heads: 53 us row by row, 27.7 us with 4-byte loads, 26.4 us.
-__device__ __forceinline__ void append_page(const AppendArgs& a, uint8_t* const grec, uint32_t* const queue,
-                                            const uint16_t* src, long long stride, int lane) {
-  const EncFrag e = enc_block<false>(src, stride, reinterpret_cast<uint8_t*>(queue), lane);   // (the queue is still empty)
-  int chain = recycle_chain(a, grec, lane);
+// `ahead`: the block's loads went out before the slots were known (v), else they go out here.  8192 tokens x 8 KV heads, append and
+// read back (10 us): row by row 67 us, with 4-byte loads 37.7, 16-byte loads 36.8, requested ahead 28.8.
+__device__ __forceinline__ void append_page(const AppendArgs& a, uint8_t* const grec, uint32_t* const queue, bool ahead,
+                                            const uint4 (&v)[4], const uint16_t* src, long long stride, int lane) {
+  const uint32_t was = old_header(a, grec);                       // (in flight while the block is encoded)
+  EncFrag e;
+  uint8_t* const stage = reinterpret_cast<uint8_t*>(queue);       // (the queue is still empty)
+  if (ahead) place_block(e.A, v, stage, lane);
+  else load_block<false>(e.A, src, stride, stage, lane);
+  enc_finish(e);
+  int chain = recycle_chain(a, was, lane);
   __syncwarp();
   enc_write(grec, e, lane);
   int queued = 0, in_unit = 0;
@@ -182,7 +188,7 @@ __device__ __forceinline__ void append_rows(const AppendArgs& a, uint8_t* const 
                                             const uint32_t (&pairs)[PAGE], const int lane) {
   int in_unit, chain;                                             // entries already in the unit; first chain block or -1
   if (r0 == 0) {                                                  // the page starts over: an all-zero unit
-    chain = recycle_chain(a, grec, lane);
+    chain = recycle_chain(a, old_header(a, grec), lane);
     for (int i = lane; i < RKV / 16; i += 32) reinterpret_cast<uint4*>(rec)[i] = make_uint4(0, 0, 0, 0);
     in_unit = 0;
   } else {
@@ -245,6 +251,22 @@ __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   if (grp * a.gsz >= a.N) return;
   const int u = (int)(w % units), h = u >> 2, kvi = (u >> 1) & 1, half = u & 1;
   const long long n_end = min((long long)a.N, (grp + 1) * a.gsz);
+  // Where the group's tokens come from does not depend on their slots: in a long call, whose groups are whole pages as a rule,
+  // the sixteen rows are requested before the slots are looked up, so a page costs two trips to memory one after the other
+  // (slots and rows, then the old header) and not four
+  const uint16_t* const rows = (kvi ? a.V : a.K) + h * HD + half * 64;
+  const long long stride = kvi ? a.vs : a.ks;
+  if (a.gsz == PAGE && (grp + 1) * PAGE <= a.N && block_aligned(rows, stride)) {
+    const long long n = grp * PAGE;
+    uint4 v[4];
+    request_block(v, rows + n * stride, stride, lane);
+    const long long mine = a.slot[n + (lane & 15)], s0 = __shfl_sync(FULL, mine, 0), blk = s0 / PAGE;
+    if (s0 >= 0 && s0 % PAGE == 0 && blk < a.nblocks && __all_sync(FULL, mine == s0 + (lane & 15))) {
+      append_page(a, a.kv + unit_off(blk, a.H, h, kvi, half), s_queue[threadIdx.x >> 5], true, v, rows, stride, lane);
+      return;
+    }
+  }
+  const uint4 none[4] = {};
   for (long long n = grp * a.gsz; n < n_end; ++n) {
   const long long s0 = a.slot[n];
   if (s0 < 0) continue;
@@ -263,8 +285,7 @@ __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   const long long seg = n;
   n += nrow - 1;                                                  // the segment's other tokens
   if (nrow == PAGE) {
-    append_page(a, grec, s_queue[threadIdx.x >> 5],
-                (kvi ? a.V + seg * a.vs : a.K + seg * a.ks) + h * HD + half * 64, kvi ? a.vs : a.ks, lane);
+    append_page(a, grec, s_queue[threadIdx.x >> 5], false, none, rows + seg * stride, stride, lane);
     continue;
   }
   // fetch every row's pair of values now (independent loads), encode afterwards

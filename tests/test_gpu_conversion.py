@@ -59,3 +59,35 @@ def test_offsets_are_the_prefix_sums(M, N):
     for out, counts in ((roff, rowcnt), (eo, reccnt)):
         n = counts.numel()
         assert torch.equal(out[:n], counts.to(torch.int64).cumsum(0).to(torch.int32)) and bool((out[n:] == -7).all())
+
+
+@pytest.mark.parametrize("how", ["whole", "shifted", "holes", "outside", "reversed_pages"])
+def test_long_appends_equal_short_ones(how):
+    """a call of 1024 tokens and more (a warp per sixteen tokens, rows requested before their slots are looked up) against the same
+    tokens one call each: groups that are whole pages, start inside one, have dropped or foreign tokens"""
+    from statetree_b200.kvcache import PageStore
+    H, n = 2, 1061
+    K, V = (bits_to_torch(t, DEV) for t in G.kv_tokens(n, H, seed=n, tiny=0.02))
+    slots, pages = torch.arange(n, device=DEV), n // 16 + 3
+    if how == "shifted":
+        slots = slots + 5
+    elif how == "holes":
+        slots[torch.arange(0, n, 37, device=DEV)] = -1
+    elif how == "outside":
+        slots[160:176] += pages * 16
+        slots[200:205] = -1
+    elif how == "reversed_pages":
+        slots = (n // 16 - slots // 16) * 16 + slots % 16
+    stores = []
+    for step in (n, 1):
+        st = PageStore(pages, H, DEV, pool_blocks=4096)
+        for reuse in (False, True):                             # (the second time over pages that have chains)
+            for a in range(0, n, step):
+                st.append(K[a:a + step], V[a:a + step], slots[a:a + step].contiguous(), reuse)
+        torch.cuda.synchronize()
+        st.check()
+        stores.append(st)
+    for x, y in zip(stores[0].dense(), stores[1].dense()):
+        assert torch.equal(x, y)
+    ok = (slots >= 0) & (slots < pages * 16)
+    assert torch.equal(stores[0].dense()[0].view(-1, H, 128)[slots[ok]], K[ok])
