@@ -421,9 +421,11 @@ class TreeLinear(nn.Module):
 
     def _plain(self, x, home):
         """the product in one native call, for inputs that need no conversion (BF16 rows on the layer's device, see
-        csrc/py_calls.cpp) and no bias; None for the others and for batches that go through the scratch matrix"""
+        csrc/py_calls.cpp) and no bias; None for the others, for batches that go through the scratch matrix and where that module
+        has not been built"""
         M, N = self.out_features, self.in_features
-        if self.bias is not None or x.dim() == 0 or x.shape[-1] != N:
+        host = calls()
+        if host is None or self.bias is not None or x.dim() == 0 or x.shape[-1] != N:
             return None
         B = x.numel() // N
         eo, el, eb = self.tables()
@@ -435,8 +437,7 @@ class TreeLinear(nn.Module):
             ws, cnt = st.scratch, st.get_cnt((M // 128) * ((B + 255) // 256))     # (the GEMM asks for no workspace)
         else:
             return None
-        native, library = calls()
-        return native.linear(library, use_gemm, self._buffers["tree"], eo, el, eb, x, ws, cnt)
+        return host[0].linear(host[1], use_gemm, self._buffers["tree"], eo, el, eb, x, ws, cnt)
 
     def _forward(self, x, yf32=None):
         """any leading shape, any float dtype, any device: the product runs where the tree lives, in BF16, and comes
@@ -514,11 +515,11 @@ def forward_list(layers, x):
         return [l(x) for l in layers]
     here = x.device == home
     widths = [l.out_features for l in layers]
-    if here and x.shape[-1] == width and all(l.bias is None for l in layers):
+    host = calls()
+    if host is not None and here and x.shape[-1] == width and all(l.bias is None for l in layers):
         st = _state(home)                               # one native call for inputs that need no conversion
         scratch = (st.get_cnt((sum(widths) // 128) * ((B + 255) // 256)) if use_gemm else st.gemv_ws(tuple(widths), width, B))
-        native, library = calls()
-        res = native.linear_list(library, use_gemm, trees, [l.tables() for l in layers], x, scratch)
+        res = host[0].linear_list(host[1], use_gemm, trees, [l.tables() for l in layers], x, scratch)
         if res is not None:
             return res
     acts = _rows_2d(x if here else x.to(home), width)

@@ -110,25 +110,26 @@ def lib():
     return _LIB
 
 
-_CALLS = None
+CALLS_PATH = os.path.join(_HERE, "_calls.so")
+_CALLS = None                                           # False: there is none
 
 
 def calls():
     """(the native module of csrc/py_calls.cpp, the entry points of the loaded library for it): the host path of plain module
-    calls.  Raises when it has not been built."""
+    calls and of conversions.  None where it has not been built: the same kernels are then launched from Python."""
     global _CALLS
     if _CALLS is None:
         L = lib()
-        path = os.path.join(_HERE, "_calls.so")
-        if not os.path.exists(path):
-            raise RuntimeError(f"statetree_b200: {path} is missing; build it with `python statetree-representation_b200/build.py`")
-        spec = importlib.util.spec_from_file_location("_calls", path)
+        if not os.path.exists(CALLS_PATH):
+            _CALLS = False                              # (looked for once)
+            return None
+        spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
         native = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(native)
         names = ("st_gemv", "st_gemm", "st_gemv_list", "st_gemm_list", "st_last_error", "st_encode", "st_encode_lists",
                  "st_encode_offsets", "st_encode_offsets_workspace_bytes", "st_dec_check", "st_lists_check")
         _CALLS = native, native.library({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names})
-    return _CALLS
+    return _CALLS or None
 
 
 def _ptr(t):
@@ -203,8 +204,26 @@ class _Weights:
     @staticmethod
     def encode(W):
         """W [M, N] BF16 on a GPU -> (tree, rows, cols, bits, (eo, el, eb)): the format's parts and the kernels' side tables"""
-        native, library = calls()
-        tree, rows, cols, bits, eo, el, eb = native.encode(library, W)
+        host = calls()
+        if host is not None:
+            tree, rows, cols, bits, eo, el, eb = host[0].encode(host[1], W)
+            return tree, rows, cols, bits, (eo, el, eb)
+        M, N = W.shape
+        nrec = (M // 16) * (N // 64)
+        u8 = lambda *shape: torch.empty(*shape, dtype=torch.uint8, device=W.device)             # noqa: E731
+        i32 = lambda *shape: torch.empty(*shape, dtype=torch.int32, device=W.device)            # noqa: E731
+        tree, rowcnt, reccnt, roff, eo = u8(M // 16, N // 64, 1552), u8(M * (N // 64)), i32(nrec + 1), i32(M * (N // 64)), i32(nrec + 1)
+        ws = u8(max(0, int(lib().st_encode_offsets_workspace_bytes(M, N))))
+        with _ctx(W):
+            _check(lib().st_encode(_ptr(W), M, N, _ptr(tree), _ptr(rowcnt), _ptr(reccnt), _stream(W)))
+            _check(lib().st_encode_offsets(_ptr(rowcnt), _ptr(reccnt), M, N, _ptr(roff), _ptr(eo), _ptr(ws), ws.numel(), _stream(W)))
+            n = int(eo[-1])                              # (synchronises: the lists' length depends on the data)
+            rows, cols, bits = i32(n), i32(n), torch.empty(n, dtype=torch.int16, device=W.device)
+            el, eb = i32(n) if n else torch.zeros(1, dtype=torch.int32, device=W.device), i32((M // 16) * ((N // 64 + 7) // 8), 16)
+            spare = el                                   # (no escapes: empty tensors have no address; nothing is written)
+            _check(lib().st_encode_lists(_ptr(W), M, N, _ptr(rowcnt), _ptr(roff), _ptr(eo), _ptr(el), _ptr(eb),
+                                         _ptr(rows if n else spare), _ptr(cols if n else spare), _ptr(bits if n else spare),
+                                         _stream(W)))
         return tree, rows, cols, bits, (eo, el, eb)
 
     @staticmethod
@@ -216,8 +235,18 @@ class _Weights:
     @staticmethod
     def check_start(T, EO, EL, W, stored=None):
         """launches that check: an int32 tensor that will hold zero if all is well"""
-        native, library = calls()
-        return native.check_start(library, T, EO, EL, W, [] if stored is None else list(stored))
+        host = calls()
+        if host is not None:
+            return host[0].check_start(host[1], T, EO, EL, W, [] if stored is None else list(stored))
+        M, N = W.shape
+        bad = torch.zeros(1, dtype=torch.int32, device=W.device)
+        with _ctx(T):
+            _check(lib().st_dec_check(_ptr(T), _ptr(EO), _ptr(EL), M, N, _ptr(W), _ptr(bad), _stream(T)))
+            if stored is not None:
+                rows, cols, bits, EB = stored
+                _check(lib().st_lists_check(_ptr(rows), _ptr(cols), _ptr(bits), rows.numel(), _ptr(EO), _ptr(EL), _ptr(EB), M, N,
+                                            _ptr(W), _ptr(bad), _stream(T)))
+        return bad
 
     @staticmethod
     def rows(T, EO, EL, ids, out):

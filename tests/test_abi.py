@@ -107,3 +107,12 @@ def test_install_as_makes_the_reference_imports_resolve_here():
     finally:
         for k in [k for k in sys.modules if k.startswith("statetree_alias_for_test") or k == "taken_name_for_test"]:
             del sys.modules[k]
+
+
+def test_library_alone_is_enough(monkeypatch):
+    """a tree with the kernel library and without the native host path of module calls: no error, the calls go out from Python"""
+    ops = _built()
+    monkeypatch.setattr(ops, "CALLS_PATH", "/nonexistent/_calls.so")
+    monkeypatch.setattr(ops, "_CALLS", None)
+    assert ops.calls() is None and ops.built()
+    assert ops.calls() is None                          # (and when asked again)

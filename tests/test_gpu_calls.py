@@ -96,3 +96,33 @@ def test_calls_in_a_graph_and_on_another_stream(monkeypatch):
             for a, b in zip(out, call()):
                 assert torch.equal(a, b)
         side.synchronize()
+
+
+@pytest.mark.parametrize("M,N", [(256, 512), (48, 640), (128, 64)])
+def test_library_alone(M, N, monkeypatch):
+    """without the native module: conversion with its check, products and lists by the same kernels, the same bits"""
+    from statetree_b200 import TreeLinear, format as F, ops
+    from statetree_b200.linear import forward_list
+    g = torch.Generator(DEV).manual_seed(M + N)
+    Ws = [(torch.randn(M, N, device=DEV, generator=g) * 0.05).to(torch.bfloat16), torch.ones(M, N, dtype=torch.bfloat16, device=DEV)]
+    Ws[0][:, 5] *= 4096                                         # escapes in one, none in the other
+    x = torch.randn(3, N, device=DEV, generator=g).to(torch.bfloat16)
+
+    def work():
+        tls = [TreeLinear.from_weight(W) for W in Ws]
+        out = [t for tl in tls for t in (tl(x), tl.dequantize(), *tl.tables(), *(tl._buffers[n] for n in ("tree", "esc_rows", "esc_cols", "esc_bits")))]
+        enc = F.encode(Ws[0])
+        other = Ws[0].clone()
+        other[M - 1, N - 1] += 1
+        eo, el, _ = tls[0].tables()
+        out += forward_list(tls, x) + [enc[k] for k in sorted(enc)]
+        return out + [torch.tensor(ops.ext().dec_check(tls[0].tree, eo, el, W)) for W in (Ws[0], other)]
+
+    want = work()
+    monkeypatch.setattr(ops, "CALLS_PATH", "/nonexistent/_calls.so")
+    monkeypatch.setattr(ops, "_CALLS", None)
+    got = work()
+    assert [bool(t) for t in got[-2:]] == [True, False]
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+    assert ops.device_status() == 0
