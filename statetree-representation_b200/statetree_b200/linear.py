@@ -420,23 +420,25 @@ class TreeLinear(nn.Module):
         return self._forward(x)
 
     def _plain(self, x, home):
-        """the product in one native call, for inputs that need no conversion (BF16 rows on the layer's device, see
-        csrc/py_calls.cpp) and no bias; None for the others, for batches that go through the scratch matrix and where that module
-        has not been built"""
-        M, N = self.out_features, self.in_features
-        host = calls()
-        if host is None or self.bias is not None or x.dim() == 0 or x.shape[-1] != N:
+        """the product in one native call (csrc/py_calls.cpp), for a layer without a bias and BF16 inputs that lie on its device
+        contiguous and 16-byte aligned; None for inputs of another width or without rows, for batches that go through the scratch
+        matrix and where that module has not been built"""
+        M, N, shape = self.out_features, self.in_features, x.shape
+        if not shape or shape[-1] != N:
             return None
-        B = x.numel() // N
-        eo, el, eb = self.tables()
-        if B <= min(GEMV_MAX, 32):
-            use_gemm, st = False, _state(home)
-            ws, cnt = st.gemv_ws(M, N, max(B, 1)), st.get_cnt(M // 16)
+        B, host = x.numel() // N, calls()
+        if B < 1 or host is None:
+            return None
+        use_gemm = B > GEMV_MAX or B > 32
+        if not use_gemm:
+            st = _state(home)
+            ws, cnt = st.gemv_ws(M, N, B), st.get_cnt(M // 16)
         elif M % 128 == 0 and not self.dense_for(B):
-            use_gemm, st = True, _state(home)
+            st = _state(home)
             ws, cnt = st.scratch, st.get_cnt((M // 128) * ((B + 255) // 256))     # (the GEMM asks for no workspace)
         else:
             return None
+        eo, el, eb = self._tables or self.tables()                # (tables left on another device: the native call takes none)
         return host[0].linear(host[1], use_gemm, self._buffers["tree"], eo, el, eb, x, ws, cnt)
 
     def _forward(self, x, yf32=None):
@@ -445,7 +447,10 @@ class TreeLinear(nn.Module):
         home, asked_dtype, asked_device = self._buffers["tree"].device, x.dtype, x.device
         if home.type != "cuda":
             raise RuntimeError("statetree_b200: the kernels take CUDA tensors only (no CPU path); move the layer to a GPU")
-        if yf32 is None:
+        bias = self.bias
+        # (what rules an input out for _plain is looked at before anything is fetched for it)
+        if (bias is None and yf32 is None and asked_dtype == torch.bfloat16 and asked_device == home and x.is_contiguous()
+                and x.data_ptr() % 16 == 0):
             result = self._plain(x, home)
             if result is not None:
                 return result
@@ -455,7 +460,6 @@ class TreeLinear(nn.Module):
         if acts.shape[0] > 0:
             with on_device(home.index):
                 self._run(acts, result, yf32)
-        bias = self.bias
         if bias is not None:
             result += bias
         if len(lead) != 1:
@@ -506,20 +510,21 @@ def forward_list(layers, x):
     else falls back to one call per layer."""
     first = layers[0]
     trees = [l._buffers["tree"] for l in layers]
-    home, width = trees[0].device, first.in_features
-    lead, B = x.shape[:-1], x.numel() // width
-    use_gemm = B > min(GEMV_MAX, 32)
+    home, width, shape = trees[0].device, first.in_features, x.shape
+    lead, B = shape[:-1], x.numel() // width
+    use_gemm = B > GEMV_MAX or B > 32
     if (home.type != "cuda" or B < 1 or not 2 <= len(layers) <= 4
             or any(l.in_features != width or t.device != home for l, t in zip(layers, trees))
             or (use_gemm and any(l.out_features % 128 for l in layers))):
         return [l(x) for l in layers]
-    here = x.device == home
-    widths = [l.out_features for l in layers]
-    host = calls()
-    if host is not None and here and x.shape[-1] == width and all(l.bias is None for l in layers):
+    here, bf16 = x.device == home, x.dtype == torch.bfloat16
+    widths, biases = [l.out_features for l in layers], [l.bias for l in layers]
+    host = calls() if (here and bf16 and x.is_contiguous() and shape[-1] == width and x.data_ptr() % 16 == 0
+                       and all(b is None for b in biases)) else None
+    if host is not None:
         st = _state(home)                               # one native call for inputs that need no conversion
         scratch = (st.get_cnt((sum(widths) // 128) * ((B + 255) // 256)) if use_gemm else st.gemv_ws(tuple(widths), width, B))
-        res = host[0].linear_list(host[1], use_gemm, trees, [l.tables() for l in layers], x, scratch)
+        res = host[0].linear_list(host[1], use_gemm, trees, [l._tables or l.tables() for l in layers], x, scratch)
         if res is not None:
             return res
     acts = _rows_2d(x if here else x.to(home), width)
@@ -539,12 +544,11 @@ def forward_list(layers, x):
         else:
             E.gemv_list(args, acts, st.gemv_ws(tuple(widths), width, B))
     res = []
-    for l, y, w in zip(layers, parts, widths):
+    for bias, y, w in zip(biases, parts, widths):
         y = y.view(*lead, w)
-        bias = l.bias
         if bias is not None:
             y += bias
-        if x.dtype != torch.bfloat16:
+        if not bf16:
             y = y.to(x.dtype)
         res.append(y if here else y.to(x.device))
     return res
