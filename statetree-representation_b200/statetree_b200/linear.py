@@ -75,7 +75,8 @@ class _DevState:
         need = self._need.get((M, N, B))
         if need is None:
             E = ext()
-            need = E.gemv_list_workspace_bytes(M, N, B) if isinstance(M, tuple) else E.gemv_workspace_bytes(M, N, B)
+            with on_device(self.device.index):          # (the size depends on the device's SMs; the caller may be on another one)
+                need = E.gemv_list_workspace_bytes(M, N, B) if isinstance(M, tuple) else E.gemv_workspace_bytes(M, N, B)
             if len(self._need) < 4096:
                 self._need[(M, N, B)] = need
         return self.get_ws(need)

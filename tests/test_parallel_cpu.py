@@ -116,3 +116,27 @@ def test_peer_comm_is_not_used_off_gpu():
     from statetree_b200 import parallel
     assert parallel.peer_comm(None) is None                      # no process group here
     assert parallel.PeerComm.MAX_VALUES == 524288
+
+
+@pytest.mark.parametrize("rows", [256, (256, 128)])
+def test_workspaces_are_sized_on_the_layers_device(rows, monkeypatch):
+    """a layer on another device than the current one: its workspace is sized for its own device's SMs"""
+    import contextlib
+    import statetree_b200.linear as L
+    current, asked = [0], []
+
+    @contextlib.contextmanager
+    def on_device(index):
+        before, current[0] = current[0], index
+        yield
+        current[0] = before
+
+    class Lib:
+        gemv_workspace_bytes = gemv_list_workspace_bytes = staticmethod(lambda M, N, B: (asked.append((current[0], M, N, B)), 64)[1])
+
+    monkeypatch.setattr(L, "on_device", on_device)
+    monkeypatch.setattr(L, "ext", lambda: Lib)
+    st = L._DevState.__new__(L._DevState)
+    st.device, st._need, st._retired, st.ws = torch.device("cuda", 1), {}, [], torch.zeros(64)
+    assert st.gemv_ws(rows, 512, 3) is st.ws and st.gemv_ws(rows, 512, 3) is st.ws
+    assert asked == [(1, rows, 512, 3)] and current == [0]
