@@ -18,6 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "statetree_b200", "libstatetree_b200.so")
 CALLS = os.path.join(HERE, "statetree_b200", "_calls.so")
 OBJ = os.path.join(HERE, "build")
+CALLS_FOR = os.path.join(OBJ, "_calls.txt")
 NVCC_FLAGS = ["-Wno-deprecated-gpu-targets", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr"]
 
@@ -59,10 +60,16 @@ def build_library(force=False, verbose=False, defines=(), out=None):
 
 
 def build_calls(force=False):
-    """_calls.so from csrc/py_calls.cpp"""
+    """_calls.so from csrc/py_calls.cpp: compiled again when that file or the C ABI's header is newer, and for another torch or
+    Python than it was compiled for (noted in CALLS_FOR)"""
+    import torch
     src = os.path.join(CSRC, "py_calls.cpp")
-    if force or _stale(CALLS, [src]):
-        import torch
+    made_for = f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+    was_for = None
+    if os.path.exists(CALLS_FOR):
+        with open(CALLS_FOR) as f:
+            was_for = f.read()
+    if force or was_for != made_for or _stale(CALLS, [src, os.path.join(HERE, "..", "include", "statetree_b200.h")]):
         root = os.path.dirname(torch.__file__)
         cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
         dirs = [f"{root}/include", f"{root}/include/torch/csrc/api/include", f"{cuda}/include", sysconfig.get_paths()["include"]]
@@ -72,6 +79,9 @@ def build_calls(force=False):
         r = subprocess.run(cmd + ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"{cmd[0]} failed on {src}:\n{r.stdout}\n{r.stderr}")
+        os.makedirs(OBJ, exist_ok=True)
+        with open(CALLS_FOR, "w") as f:
+            f.write(made_for)
     return CALLS
 
 

@@ -10,6 +10,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/utils/pybind.h>
+#include <torch/version.h>
 
 #include <cstdint>
 #include <map>
@@ -18,39 +19,24 @@
 #include <type_traits>
 #include <vector>
 
+#include "../../include/statetree_b200.h"
+
 namespace py = pybind11;
 
 namespace {
-using Gemv = int (*)(const void*, const int32_t*, const uint32_t*, const uint32_t*, const void*, void*, float*, int64_t, int64_t,
-                     int64_t, void*, int64_t, int32_t*, void*);
-using Gemm = int (*)(const void*, const int32_t*, const uint32_t*, const void*, void*, float*, int64_t, int64_t, int64_t, void*,
-                     int64_t, int32_t*, void*);
-using GemvList = int (*)(int64_t, const void* const*, const int32_t* const*, const uint32_t* const*, const uint32_t* const*,
-                         const void*, void* const*, float* const*, int64_t, const int64_t*, int64_t, void*, int64_t, void*);
-using GemmList = int (*)(int64_t, const void* const*, const int32_t* const*, const uint32_t* const*, const void*, void* const*,
-                         float* const*, int64_t, const int64_t*, int64_t, int32_t*, void*);
-using LastError = const char* (*)();
-using Encode = int (*)(const void*, int64_t, int64_t, void*, uint8_t*, int32_t*, void*);
-using OffsetsBytes = int64_t (*)(int64_t, int64_t);
-using Offsets = int (*)(const uint8_t*, const int32_t*, int64_t, int64_t, int32_t*, int32_t*, void*, int64_t, void*);
-using Lists = int (*)(const void*, int64_t, int64_t, const uint8_t*, const int32_t*, const int32_t*, uint32_t*, uint32_t*, int32_t*,
-                      int32_t*, int16_t*, void*);
-using DecCheck = int (*)(const void*, const int32_t*, const uint32_t*, int64_t, int64_t, const void*, int32_t*, void*);
-using ListsCheck = int (*)(const int32_t*, const int32_t*, const int16_t*, int64_t, const int32_t*, const uint32_t*, const uint32_t*,
-                           int64_t, int64_t, const void*, int32_t*, void*);
-
+// the entry points of the loaded kernel library, with the types of the header that this file was compiled with
 struct Library {
-  Gemv gemv;
-  Gemm gemm;
-  GemvList gemv_list;
-  GemmList gemm_list;
-  LastError last_error;
-  Encode encode;
-  OffsetsBytes offsets_bytes;
-  Offsets offsets;
-  Lists lists;
-  DecCheck dec_check;
-  ListsCheck lists_check;
+  decltype(&st_gemv) gemv;
+  decltype(&st_gemm) gemm;
+  decltype(&st_gemv_list) gemv_list;
+  decltype(&st_gemm_list) gemm_list;
+  decltype(&st_last_error) last_error;
+  decltype(&st_encode) encode;
+  decltype(&st_encode_offsets_workspace_bytes) offsets_bytes;
+  decltype(&st_encode_offsets) offsets;
+  decltype(&st_encode_lists) lists;
+  decltype(&st_dec_check) dec_check;
+  decltype(&st_lists_check) lists_check;
 };
 
 // rows of x if it can be read as it is: BF16 [..., N] on `device`, contiguous, 16-byte aligned, at least one row; else 0
@@ -75,7 +61,7 @@ std::vector<int64_t> out_sizes(const at::Tensor& x, int64_t M) {
   return s;
 }
 
-// the entry points of the loaded kernel library
+// binds the entry points: their addresses by name
 Library library(const std::map<std::string, uint64_t>& address) {
   Library lib;
   auto bind = [&](auto& entry, const char* name) {
@@ -238,6 +224,8 @@ at::Tensor check_start(const Library& lib, const at::Tensor& tree, const at::Ten
 }  // namespace
 
 PYBIND11_MODULE(_calls, m) {
+  m.attr("ABI") = ST_ABI_VERSION;                // what this file was compiled against (compared when it is loaded)
+  m.attr("TORCH") = TORCH_VERSION;
   py::class_<Library>(m, "Library");
   m.def("library", &library);
   m.def("linear", &linear);

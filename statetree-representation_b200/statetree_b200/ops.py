@@ -6,6 +6,7 @@ torch's current stream of the tensors' device.  There is no fallback: a missing 
 import ctypes
 import importlib.util
 import os
+import warnings
 
 import torch
 
@@ -112,23 +113,31 @@ def lib():
 
 CALLS_PATH = os.path.join(_HERE, "_calls.so")
 _CALLS = None                                           # False: there is none
+_NATIVE = ("st_gemv", "st_gemm", "st_gemv_list", "st_gemm_list", "st_last_error", "st_encode", "st_encode_lists", "st_encode_offsets",
+           "st_encode_offsets_workspace_bytes", "st_dec_check", "st_lists_check")
 
 
 def calls():
     """(the native module of csrc/py_calls.cpp, the entry points of the loaded library for it): the host path of plain module
-    calls and of conversions.  None where it has not been built: the same kernels are then launched from Python."""
+    calls and of conversions.  None where it has not been built, or (with a warning) was built against another C ABI or torch: the
+    same kernels are then launched from Python."""
     global _CALLS
     if _CALLS is None:
         L = lib()
-        if not os.path.exists(CALLS_PATH):
-            _CALLS = False                              # (looked for once)
-            return None
-        spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
-        native = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(native)
-        names = ("st_gemv", "st_gemm", "st_gemv_list", "st_gemm_list", "st_last_error", "st_encode", "st_encode_lists",
-                 "st_encode_offsets", "st_encode_offsets_workspace_bytes", "st_dec_check", "st_lists_check")
-        _CALLS = native, native.library({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in names})
+        _CALLS = False                                  # (looked for once)
+        if os.path.exists(CALLS_PATH):
+            spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
+            try:
+                native = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(native)
+                found = f"C ABI {native.ABI}, torch {native.TORCH}"
+                if native.ABI == ABI and native.TORCH == torch.__version__.split("+")[0]:
+                    _CALLS = native, native.library({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in _NATIVE})
+            except ImportError as e:                    # (another interpreter's, or symbols that this torch does not have)
+                found = str(e)
+            if not _CALLS:
+                warnings.warn(f"statetree_b200: {CALLS_PATH} was built against another torch or C ABI ({found}) and is not used; "
+                              "rebuild it with `python statetree-representation_b200/build.py`")
     return _CALLS or None
 
 

@@ -7,15 +7,18 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
+def _build_module():
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("st_build", os.path.join(ROOT, "statetree-representation_b200", "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
 def _built():
     from statetree_b200 import ops
     if not os.path.exists(ops.LIB_PATH):
-        import importlib.util
-        spec = importlib.util.spec_from_file_location("st_build", os.path.join(ROOT, "statetree-representation_b200",
-                                                                               "build.py"))
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        mod.build_library()
+        _build_module().build_library()
     return ops
 
 
@@ -116,3 +119,50 @@ def test_library_alone_is_enough(monkeypatch):
     monkeypatch.setattr(ops, "_CALLS", None)
     assert ops.calls() is None and ops.built()
     assert ops.calls() is None                          # (and when asked again)
+
+
+def test_native_calls_are_compiled_again(monkeypatch, tmp_path):
+    """_calls.so is up to date only for the sources, the C header, the torch and the Python that it was compiled with"""
+    import torch
+    mod, compiled = _build_module(), []
+    src, header = tmp_path / "pkg" / "csrc" / "py_calls.cpp", tmp_path / "include" / "statetree_b200.h"
+    for f in (src, header):
+        f.parent.mkdir(parents=True)
+        f.write_text("")
+        os.utime(f, (1000, 1000))
+    for name, path in (("HERE", tmp_path / "pkg"), ("CSRC", src.parent), ("OBJ", tmp_path), ("CALLS", tmp_path / "_calls.so"),
+                       ("CALLS_FOR", tmp_path / "_calls.txt")):
+        monkeypatch.setattr(mod, name, str(path), raising=False)
+
+    def run(cmd, **kw):
+        compiled.append(cmd)
+        (tmp_path / "_calls.so").write_bytes(b"")
+        os.utime(mod.CALLS, (2000 + len(compiled),) * 2)
+        return type("Result", (), {"returncode": 0})
+
+    monkeypatch.setattr(mod.subprocess, "run", run)
+
+    def builds():
+        before = len(compiled)
+        mod.build_calls()
+        return len(compiled) - before
+
+    assert (builds(), builds()) == (1, 0)
+    for i, f in enumerate((src, header)):
+        os.utime(f, (2001.5 + i,) * 2)
+        assert (builds(), builds()) == (1, 0), f
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert (builds(), builds()) == (1, 0)
+
+
+def test_native_calls_of_another_abi_are_not_used(monkeypatch):
+    ops = _built()
+    if not os.path.exists(os.path.join(os.path.dirname(ops.LIB_PATH), "_calls.so")):
+        _build_module().build_calls()
+    ops.lib()
+    monkeypatch.setattr(ops, "_CALLS", None)
+    assert ops.calls() is not None
+    monkeypatch.setattr(ops, "_CALLS", None)
+    monkeypatch.setattr(ops, "ABI", ops.ABI + 1)
+    with pytest.warns(UserWarning, match="another torch or C ABI"):
+        assert ops.calls() is None
