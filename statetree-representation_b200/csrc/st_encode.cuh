@@ -39,7 +39,7 @@ __device__ __forceinline__ void place_block(uint32_t (&A)[4][4], const uint4 (&v
   // lane l names row l % 16 of the two 8-column halves l / 16: matrices in the order of the fragment registers
   const uint32_t from = smem_addr(stage) + (uint32_t)((lane & 15) * ENC_ROW + (lane >> 4) * 16);
 #pragma unroll
-  for (int s = 0; s < 4; ++s) ldmatrix_x4(from + 32 * s, A[s][0], A[s][1], A[s][2], A[s][3]);
+  for (int s = 0; s < 4; ++s) ldmatrix_x4_stored(from + 32 * s, A[s][0], A[s][1], A[s][2], A[s][3]);
   __syncwarp();                                                  // (the stage is reused)
 }
 
