@@ -1,9 +1,8 @@
-// Fused tree-decode + GEMM on the 5th-generation tensor cores (tcgen05 / TMEM) of sm_100a: up to 320 tokens in one tile, and the
-// grouped (mixture-of-experts) form.  More tokens, and fewer where they are the faster ones, go to CTA pairs (st_gemm_pair.cu).
+// Fused tree-decode + GEMM on the 5th-generation tensor cores (tcgen05 / TMEM) of sm_100a, one CTA per tile of at most 320 tokens,
+// and its grouped (mixture-of-experts) form.  More than 128 tokens go to CTA pairs (st_gemm_pair.cu) where those are the faster ones.
 //   Y[B, M] = X[B, N] W[M, N]^T,  W as state-tree records, fp32 accumulation in tensor memory, BF16 output.
 //
-// One CTA computes a 128-row block of W against a tile of NT tokens (all of a dense call's) over a contiguous range of
-// 64-column k-tiles.
+// One CTA computes a 128-row block of W against one tile of NT tokens over a contiguous range of 64-column k-tiles.
 // Warp roles:
 //   8 DG decode warps, in DG groups of eight (group g takes the k-tile pairs g, g + DG, ...): each warp turns the two
 //              records of its 16 rows into mma-fragment registers (five integer ops per four weights), patches escapes,
@@ -51,7 +50,7 @@ template <int DG> constexpr int gemm_threads() { return (DG * NDEC + 3) * 32; }
 // DG = 1 (token tiles up to 128): eight decode warps, at most half of an SM's shared memory, registers and tensor memory,
 // so two CTAs share an SM: one CTA's start-up, drain and epilogue run under the other's main loop, and the next launch's
 // CTAs become resident (and start streaming weights) as soon as any CTA of this launch leaves.
-// DG = 2 (up to 320 tokens): one CTA per SM, sixteen decode warps.
+// DG = 2 (tiles of up to 320 tokens): one CTA per SM, sixteen decode warps.
 //
 // Measured, the four projections of a layer (6144, 4096, 24576 x 4096 and 4096 x 12288) in a graph, us per layer: 64 rows
 // 108 -> 85, 300 rows 251 -> 153 (was: A through shared memory by stmatrix, one record per step, 64 / 128 / 256-token
@@ -88,9 +87,10 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accbar + 1);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0);   // (a warp-uniform value to the compiler)
-  // unit of this CTA.  Grouped: the row blocks of a pair block run next to each other (they share the gathered activations)
+  // unit of this CTA.  Dense: the token tiles of a row block run next to each other (its records then come from HBM once
+  // and from L2 for the other tiles); grouped: the row blocks of a pair block do (they share the gathered activations)
   const int ks = blockIdx.x % a.KS, rt = blockIdx.x / a.KS;
-  const int rb = GROUPED ? rt % a.RB : a.rb0 + rt, tt = GROUPED ? rt / a.RB : 0;
+  const int rb = GROUPED ? rt % a.RB : a.rb0 + rt / a.TT, tt = GROUPED ? rt / a.RB : rt % a.TT;
   // whole pairs of k-tiles; an odd last tile is paired with one beyond the matrix, which both tensor maps fill with zeros
   const int pairs = (a.NG + PAIR - 1) / PAIR;
   const int p0 = (int)((long long)pairs * ks / a.KS), np = (int)((long long)pairs * (ks + 1) / a.KS) - p0;
@@ -503,10 +503,11 @@ void gemm_rings(GemmPlan& p) {
 
 constexpr int NT_MAX = 320;                                      // 320 accumulator columns + 4 weight tiles of 32 fill TMEM
 
-GemmPlan gemm_plan(long long M, int NG, long long B, double& us) {   // B <= NT_MAX
+GemmPlan gemm_plan(long long M, int NG, long long B, double& us) {
   GemmPlan p;
-  p.TT = 1;
-  p.NT = (int)((B + 15) & ~15);                                   // MMA widths: multiples of 16
+  // the fewest token tiles (every tile decodes the records again), of equal width
+  p.TT = (int)((B + NT_MAX - 1) / NT_MAX);
+  p.NT = (int)(((B + p.TT - 1) / p.TT + 15) & ~15);               // MMA widths: multiples of 16
   p.RB = (int)(M / 128);
   const int sms = st::sm_count();
   gemm_rings(p);
@@ -518,7 +519,7 @@ GemmPlan gemm_plan(long long M, int NG, long long B, double& us) {   // B <= NT_
   // A grid larger than the CTAs that are resident at once runs in waves.
   const int pairs = (NG + PAIR - 1) / PAIR, ksmax = pairs / 4 < 1 ? 1 : (pairs / 4 > 8 ? 8 : pairs / 4);
   auto estimate = [&](int rows, int ks) {
-    const double ctas = (double)rows * ks;
+    const double ctas = (double)rows * p.TT * ks;
     const double slots = (double)(p.DG == 1 ? resident_ctas<1>(ks, p.smem, sms) : resident_ctas<2>(ks, p.smem, sms));
     if (slots <= 0) return 1e30;
     const double waves = ctas <= slots ? 1.0 : (double)(long long)((ctas + slots - 1) / slots);
@@ -542,9 +543,10 @@ GemmPlan gemm_plan(long long M, int NG, long long B, double& us) {   // B <= NT_
   p.KS = best_split(p.RB, us);
   p.RB1 = 0;
   p.KS1 = 1;
-  // One CTA per SM: a last wave that is nearly empty costs as much as a full one (192 row blocks at 129 tokens: 148 + 44).
-  // Then the full waves go out unsplit and the rest of the row blocks in a second launch with a split of its own.
-  if (p.DG == 2 && p.RB > sms) {
+  // One CTA per SM: a last wave that is nearly empty costs as much as a full one (192 row blocks at 300 tokens: 148 + 44).
+  // Then the full waves go out unsplit and the rest of the row blocks in a second launch with a split of its own.  (One token tile:
+  // with several of them CTA pairs were ahead of such a form at 780 of 790 sizes.)
+  if (p.DG == 2 && p.TT == 1 && p.RB > sms) {
     const int rows1 = p.RB / sms * sms;
     double rest;
     if (rows1 < p.RB) {
@@ -552,6 +554,18 @@ GemmPlan gemm_plan(long long M, int NG, long long B, double& us) {   // B <= NT_
       const double both = estimate(rows1, 1) + rest + 1.0;
       if (both < us) { p.RB1 = rows1; p.KS1 = 1; p.KS = ks2; us = both; }
     }
+  }
+  // One CTA per SM: what the plan is expected to take next to CTA pairs.  The same terms, fitted so that the ratio of the two kernels'
+  // times is met at 3900 sizes (8 to 296 row blocks, 1024 to 12288 columns, 129 to 2000 tokens): within 4 %, standard deviation.
+  // Up to half of the SMs, the next launch's CTAs start beside this one's.
+  if (p.DG == 2) {
+    auto expected = [&](int rows, int ks) {
+      const double ctas = (double)rows * p.TT * ks, slots = (double)resident_ctas<2>(ks, p.smem, sms);
+      const double waves = (double)(long long)((ctas + slots - 1) / slots), part = (ctas < slots ? ctas : slots) / sms;
+      const double per_cta = (double)((pairs + ks - 1) / ks), split = ks > 1 ? 0.91 + 0.159 * ks * p.NT / 64.0 : 0.0;
+      return -3.25 + 2.2 * part + (part > 0.5 ? 0.77 : 0.0) + waves * (per_cta * (0.332 + 0.0019 * p.NT + 0.156 * part) + 5.97 + split);
+    };
+    us = expected(p.RB - p.RB1, p.KS) + (p.RB1 > 0 ? expected(p.RB1, p.KS1) + 4.4 : 0.0);
   }
   return p;
 }
@@ -583,16 +597,19 @@ void plan_args(GemmArgs& a, const GemmPlan& p) {
 
 // one matrix or a list (a names them, B, the rows of all members as M, NG and the status word)
 int dense_gemm(GemmArgs& a, const WMaps& wmaps, const void* X, const char* who, cudaStream_t stream) {
-  ST_REQUIRE(a.M / 128 * 8 < (1ll << 31), "%s: grid too large", who);
-  double us = 1e30;
-  if (a.B > NT_MAX) return pair_gemm(a, wmaps, X, who, us, stream);
+  ST_REQUIRE(a.M / 128 * 8 * ((a.B + NT_MAX - 1) / NT_MAX) < (1ll << 31), "%s: grid too large", who);
+  double us;
   const GemmPlan plan = gemm_plan(a.M, a.NG, a.B, us);
-  // From 129 to 320 tokens both kernels fit.  CTA pairs where they are estimated to be clearly faster (the estimates are within
-  // 10 to 15 %; measured, us, this kernel / CTA pairs at 129 and 300 tokens: 2048 x 2048 10.2 / 7.9 and 13.5 / 10.1, 3072 x 2048
-  // 10.6 / 9.7 and 14.1 / 12.9; 4096 x 4096 13.6 / 16.7 and 17.6 / 19.6, 4096 x 12288 25.9 / 35 and 31.8 / 39: few row blocks and
-  // long k ranges, which split over up to eight CTAs here and up to four pairs there)
+  // More than 128 tokens: CTA pairs where they are expected to be the faster ones.  Measured, us, this kernel / CTA pairs:
+  //   2048 x 2048   at 300 tokens 11.2 / 10.1, 321 11.1 / 12.7        4096 x 4096   at 300 17.5 / 20.2, 321 19.0 / 20.4
+  //   4608 x 3584   at 321 18.2 / 22.3, 900 32.4 / 29.7               4096 x 12288  at 300 32.3 / 42.1
+  //   6144 x 4096   at 321 28.2 / 24.8                                4608 x 12288  at 512 56.9 / 77.0
+  // Few row blocks split over up to eight CTAs here and over up to four pairs there, of which fifteen find room at once; with many
+  // tiles a pair halves the activations' part of the shared-memory traffic.  Two launches here (between full waves of one token tile)
+  // stay unless pairs are an eighth faster: tests/test_gpu_weights.py expects them of 192 row blocks of 2048 columns, where pairs in
+  // one launch take 27.1 us against 30.5 at 136 tokens.
   if (plan.DG == 2) {
-    const int done = pair_gemm(a, wmaps, X, who, 0.95 * us, stream);
+    const int done = pair_gemm(a, wmaps, X, who, (plan.RB1 > 0 ? 0.88 : 0.98) * us, stream);
     if (done >= 0) return done;
   }
   CUtensorMap xmap;

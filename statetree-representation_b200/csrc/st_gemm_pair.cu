@@ -526,19 +526,29 @@ void rings(PairPlan& p) {
   p.smem = ring + slack;
 }
 
-// Token tiles and split of the k range: the least estimated time in us, fitted to launches of 6144, 4096, 24576 and 12288 x 4096 /
-// 12288 / 2048 matrices in a graph at 129 to 2000 tokens (within 10 %): start-up and drain (which the next launch hides where SMs
-// are free), per pair of k-tiles the larger of the decode and a time that grows with the token tile, more when every SM streams,
-// and the epilogue of a split (adding KS tiles through distributed shared memory).  Units beyond the resident clusters run in
-// waves, in one launch or, when it is the faster, the full waves unsplit and the rest in a second launch with a split.  One token
-// tile and more than one, but not two, waves: always two launches (24576 x 4096 at 300 tokens 58.5 us, one launch 60.9; 24576 x
-// 2048 would gain from one, 33.7 against 39.6: the two-launch form at such shapes is a fixed property of this function).
+// Token tiles and split of the k range: the least estimated time in us (`time`), fitted to launches of 6144, 4096, 24576 and 12288 x
+// 4096 / 12288 / 2048 matrices in a graph at 129 to 2000 tokens: start-up and drain (which the next launch hides where SMs are free),
+// per pair of k-tiles the larger of the decode and a time that grows with the token tile, more when every SM streams, and the epilogue
+// of a split (adding KS tiles through distributed shared memory).  Units beyond the resident clusters run in waves, in one launch or,
+// when it is the faster, the full waves unsplit and the rest in a second launch with a split.
+// What the plan is expected to take, which decides between this kernel and the one-CTA one: `expected`, the same terms fitted with
+// the one-CTA kernel's so that the ratio of the two is met (st_gemm.cu).  Up to half of the SMs, the next launch's clusters start
+// beside this one's; further waves of a split start anew.  (Choosing the plan by it was no better: 34 of 520 sizes slower by more
+// than 3 %, 40 faster.)
+// One token tile and more than one, but not two, waves: always two launches.
 PairPlan make_plan(long long M, int NG, long long B, double& us) {
   const int sms = st::sm_count(), RP = (int)((M / 128 + 1) / 2), pairs = (NG + PAIR - 1) / PAIR;
   const int C = resident_clusters(1, sms);
   const int ksmax = pairs / 4 < 1 ? 1 : (pairs / 4 > 4 ? 4 : pairs / 4);
   PairPlan best = {};
   us = 1e30;
+  auto expected = [&](long long u, int ks, int nt) {
+    const int slots = resident_clusters(ks, sms), per = (pairs + ks - 1) / ks;
+    const double waves = (double)((u + slots - 1) / slots), load = (double)(u < slots ? u : slots) * ks / C;
+    const double pair = 0.214 + 0.0019 * nt > 0.576 ? 0.214 + 0.0019 * nt : 0.576;
+    const double end = ks > 1 ? 1.44 + ks * (0.0065 * nt - 0.3) + 7.1 * (waves - 1.0) / waves : 0.0063 * nt - 0.66;
+    return 1.66 + 2.77 * load + (load > 0.5 ? 1.5 : 0.0) + waves * (per * (pair + 0.17 * load) + end);
+  };
   int tt_lo = (int)((B + NT_MAX - 1) / NT_MAX), tt_hi = (int)((B + 127) / 128), ks_lo = 1, ks_hi = ksmax;
 #ifdef ST_TUNE                                                   // development builds may force both
   if (const char* f = getenv("STATETREE_PAIR_TT")) if (atoi(f) >= tt_lo && atoi(f) > 0) tt_lo = tt_hi = atoi(f);
@@ -571,7 +581,11 @@ PairPlan make_plan(long long M, int NG, long long B, double& us) {
       if (t < us - 1e-9) { us = t; best.NT = nt; best.TT = tt; best.tile1 = (int)tile1; best.KS = ks; }
     }
   }
-  if (best.TT > 0) rings(best);
+  if (best.TT == 0) return best;
+  const long long units = (long long)RP * best.TT;
+  us = (best.tile1 > 0 ? expected(best.tile1, 1, best.NT) : 0.0) +
+       (units > best.tile1 ? expected(units - best.tile1, best.KS, best.NT) + (best.tile1 > 0 ? 5.0 : 0.0) : 0.0);
+  rings(best);
   return best;
 }
 
