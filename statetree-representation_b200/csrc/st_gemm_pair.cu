@@ -535,7 +535,10 @@ void rings(PairPlan& p) {
 // the one-CTA kernel's so that the ratio of the two is met (st_gemm.cu).  Up to half of the SMs, the next launch's clusters start
 // beside this one's; further waves of a split start anew.  (Choosing the plan by it was no better: 34 of 520 sizes slower by more
 // than 3 %, 40 faster.)
-// One token tile and more than one, but not two, waves: always two launches.
+// One token tile and between one and two waves: all of it in one launch, or the full wave and a split rest, by `expected` too.  us in
+// two launches / in one: 24576 x 1024 at 200 tokens 25.4 / 18.6, 24576 x 2048 at 330 42.5 / 36.9, 28672 x 2048 at 300 42.8 / 37.0,
+// 28672 x 4096 73.8 / 67.1, 24576 x 4096 at 330 65.5 / 65.5, 20480 x 2048 at 384 41.9 / 41.9 (one launch was never the slower one at the
+// 81 sizes where it is estimated to be the faster).
 PairPlan make_plan(long long M, int NG, long long B, double& us) {
   const int sms = st::sm_count(), RP = (int)((M / 128 + 1) / 2), pairs = (NG + PAIR - 1) / PAIR;
   const int C = resident_clusters(1, sms);
@@ -585,6 +588,11 @@ PairPlan make_plan(long long M, int NG, long long B, double& us) {
   const long long units = (long long)RP * best.TT;
   us = (best.tile1 > 0 ? expected(best.tile1, 1, best.NT) : 0.0) +
        (units > best.tile1 ? expected(units - best.tile1, best.KS, best.NT) + (best.tile1 > 0 ? 5.0 : 0.0) : 0.0);
+  if (tt_lo == 1 && ks_lo == 1 && RP > C && RP < 2 * C) {
+    const int nt = (int)((B + 31) & ~31ll);
+    const double one = expected(RP, 1, nt);
+    if (one < 0.97 * us) { us = one; best.NT = nt; best.TT = 1; best.tile1 = RP; best.KS = 1; }
+  }
   rings(best);
   return best;
 }

@@ -164,3 +164,19 @@ def test_kernel_of_a_batch(M, N, B, kernel):
     assert {k for k, _ in kernels} == {kernel}
     _check(y, None, W, x)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,B", [(128 * 149, 1024, 321), (128 * 224, 2048, 330)])
+def test_one_launch_where_it_is_the_faster(M, N, B):
+    """between one and two waves of CTA pairs: one launch, whose clusters take a second unit, instead of a full wave and a rest with a
+    split of its own (measured, us, two launches / one: 28672 x 2048 at 330 rows 45.8 / 39.2)"""
+    from statetree_b200 import TreeLinear, ops
+    _on_148_sms()
+    W = _weight(M, N, M + B)
+    tl = TreeLinear.from_weight(W)
+    tl.allow_dec = False
+    x = torch.randn(B, N, device=DEV, generator=torch.Generator(DEV).manual_seed(B)).to(torch.bfloat16)
+    kernels, (y,) = _kernels(lambda: [tl(x)])
+    assert kernels == [("pair", 2)]
+    _check(y, None, W, x)
+    assert ops.device_status() == 0
