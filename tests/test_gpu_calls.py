@@ -163,3 +163,46 @@ def test_library_alone(M, N, monkeypatch):
     for a, b in zip(got, want):
         assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("same_stream", [False, True])
+def test_calls_from_two_threads(same_stream):
+    """the native call lets other threads run: layers and inputs shared by two threads, on one stream and on a stream each, give the
+    products of a single thread (which are checked against fp64: BF16 results, half an ulp each)"""
+    import threading
+    from statetree_b200 import ops
+    from statetree_b200.linear import forward_list
+    N = 1088
+    tls = _layers((256, 128, 384), N)
+    Ws = [tl.dequantize().double() for tl in tls]
+    xs = [torch.randn(B, N, device=DEV).to(torch.bfloat16) for B in (1, 3, 16, 70, 330)]
+    work = lambda x: forward_list(tls, x) + [tls[0](x)]                                         # noqa: E731
+    want = [work(x) for x in xs]
+    for x, ys in zip(xs, want):
+        for y, W in zip(ys, Ws + Ws[:1]):
+            exact = x.double() @ W.t()
+            assert float((y.double() - exact).norm() / exact.norm()) < 2.0 ** -9 * 1.1
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream()] * 2 if same_stream else [torch.cuda.Stream() for _ in range(2)]
+    start, got, failed = threading.Barrier(2), [None, None], []
+
+    def thread(i):
+        try:
+            with torch.cuda.stream(streams[i]), torch.no_grad():
+                start.wait()
+                got[i] = [[work(x) for x in xs[::1 - 2 * i]] for _ in range(20)]
+                streams[i].synchronize()
+        except Exception as e:                                  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=thread, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    for i in range(2):
+        for lap in got[i]:
+            for ys, right in zip(lap, want[::1 - 2 * i]):
+                assert all(torch.equal(a, b) for a, b in zip(ys, right))
+    assert ops.device_status() == 0
