@@ -38,7 +38,6 @@ struct AppendArgs {
   int* pool_cnt;
   long long nblocks;
   int N, H, P, reuse;
-  int gsz;                  // tokens of the call scanned per warp for segment starts (1: decode steps, 16: prefill)
 };
 
 // ---- escapes of a record.  A value whose exponent lies more than 14 below its row's largest cannot be held by the
@@ -149,15 +148,13 @@ __device__ __forceinline__ void place_entries(const AppendArgs& a, uint8_t* cons
 
 // A whole page of one unit at once: sixteen rows of 64 values, `stride` values apart, encoded like a weight record instead of
 // row by row.  The same bytes as append_rows: entries are queued in row-major, column order.
-// `ahead`: the block's loads went out before the slots were known (v), else they go out here.  8192 tokens x 8 KV heads, append and
-// read back (10 us): row by row 67 us, with 4-byte loads 37.7, 16-byte loads 36.8, requested ahead 28.8.
-__device__ __forceinline__ void append_page(const AppendArgs& a, uint8_t* const grec, uint32_t* const queue, bool ahead,
-                                            const uint4 (&v)[4], const uint16_t* src, long long stride, int lane) {
+// load(A, stage): the block's fragments, from loads that went out before the slots were known or that go out there.  8192 tokens x 8
+// KV heads, append and read back (10 us): row by row 67 us, with 4-byte loads 37.7, 16-byte loads 36.8, requested ahead 28.8.
+template <class Load>
+__device__ __forceinline__ void append_page(const AppendArgs& a, uint8_t* const grec, uint32_t* const queue, const Load load, int lane) {
   const uint32_t was = old_header(a, grec);                       // (in flight while the block is encoded)
   EncFrag e;
-  uint8_t* const stage = reinterpret_cast<uint8_t*>(queue);       // (the queue is still empty)
-  if (ahead) place_block(e.A, v, stage, lane);
-  else load_block<false>(e.A, src, stride, stage, lane);
+  load(e.A, reinterpret_cast<uint8_t*>(queue));                   // (the queue is still empty)
   enc_finish(e);
   int chain = recycle_chain(a, was, lane);
   __syncwarp();
@@ -239,6 +236,10 @@ __device__ __forceinline__ void append_rows(const AppendArgs& a, uint8_t* const 
 // bytes, and the header is read-modify-write).  Semantics of statetree/csrc/kvcache.cu:62-192.
 // The warp edits the 1600-byte unit in shared memory: the segment's rows are fetched up front (independent loads),
 // encoded row by row with shared-memory byte stores, and the unit goes back to the page as 100 16-byte stores.
+// LONG (calls of many tokens): a warp takes sixteen of them, else one.  Two kernels, so that the requests ahead of the long one cost
+// the short one and the rows outside whole pages no registers: one token in each of 8192 pages (8 KV heads) 315 us in one kernel, 306
+// so, 1023 tokens in order (2 KV heads) 9.0 and 8.3.
+template <bool LONG>
 __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   __shared__ __align__(16) uint8_t s_unit[8][RKV];
   __shared__ __align__(16) uint32_t s_queue[8][PAGE * 64];        // a segment's escape entries, worst case all of them
@@ -247,27 +248,28 @@ __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int units = a.H * 4;
-  const long long grp = w / units;                                // a.gsz consecutive tokens of the call per warp
-  if (grp * a.gsz >= a.N) return;
+  const long long grp = w / units;
+  constexpr int GSZ = LONG ? PAGE : 1;                            // tokens of the call scanned per warp for segment starts
+  if (grp * GSZ >= a.N) return;
   const int u = (int)(w % units), h = u >> 2, kvi = (u >> 1) & 1, half = u & 1;
-  const long long n_end = min((long long)a.N, (grp + 1) * a.gsz);
+  const long long n_end = min((long long)a.N, (grp + 1) * GSZ);
   // Where the group's tokens come from does not depend on their slots: in a long call, whose groups are whole pages as a rule,
   // the sixteen rows are requested before the slots are looked up, so a page costs two trips to memory one after the other
   // (slots and rows, then the old header) and not four
   const uint16_t* const rows = (kvi ? a.V : a.K) + h * HD + half * 64;
   const long long stride = kvi ? a.vs : a.ks;
-  if (a.gsz == PAGE && (grp + 1) * PAGE <= a.N && block_aligned(rows, stride)) {
+  if (LONG && (grp + 1) * PAGE <= a.N && block_aligned(rows, stride)) {
     const long long n = grp * PAGE;
     uint4 v[4];
     request_block(v, rows + n * stride, stride, lane);
     const long long mine = a.slot[n + (lane & 15)], s0 = __shfl_sync(FULL, mine, 0), blk = s0 / PAGE;
     if (s0 >= 0 && s0 % PAGE == 0 && blk < a.nblocks && __all_sync(FULL, mine == s0 + (lane & 15))) {
-      append_page(a, a.kv + unit_off(blk, a.H, h, kvi, half), s_queue[threadIdx.x >> 5], true, v, rows, stride, lane);
+      append_page(a, a.kv + unit_off(blk, a.H, h, kvi, half), s_queue[threadIdx.x >> 5],
+                  [&](uint32_t (&A)[4][4], uint8_t* stage) { place_block(A, v, stage, lane); }, lane);
       return;
     }
   }
-  const uint4 none[4] = {};
-  for (long long n = grp * a.gsz; n < n_end; ++n) {
+  for (long long n = grp * GSZ; n < n_end; ++n) {
   const long long s0 = a.slot[n];
   if (s0 < 0) continue;
   const long long blk = s0 / PAGE;
@@ -285,7 +287,8 @@ __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   const long long seg = n;
   n += nrow - 1;                                                  // the segment's other tokens
   if (nrow == PAGE) {
-    append_page(a, grec, s_queue[threadIdx.x >> 5], false, none, rows + seg * stride, stride, lane);
+    append_page(a, grec, s_queue[threadIdx.x >> 5],
+                [&](uint32_t (&A)[4][4], uint8_t* stage) { load_block<false>(A, rows + seg * stride, stride, stage, lane); }, lane);
     continue;
   }
   // fetch every row's pair of values now (independent loads), encode afterwards
@@ -844,10 +847,11 @@ extern "C" int st_kv_append(const void* K, const void* V, int64_t ks, int64_t vs
   a.nblocks = nblocks; a.N = (int)N; a.H = (int)H; a.P = (int)P; a.reuse = reuse ? 1 : 0;
   // long calls are mostly whole pages of consecutive tokens: one warp per 16 tokens finds (typically) one segment
   // and the grid shrinks 16-fold; short calls (decode steps) keep one warp per token
-  a.gsz = N >= 1024 ? 16 : 1;
-  const long long warps = ((N + a.gsz - 1) / a.gsz) * H * 4;
-  return st::launch("st_kv_append launch", kv_append_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0,
-                    (cudaStream_t)stream, a);
+  const bool many = N >= 1024;
+  const long long warps = (many ? (N + PAGE - 1) / PAGE : N) * H * 4;
+  const dim3 grid((unsigned)((warps + 7) / 8));
+  return many ? st::launch("st_kv_append launch", kv_append_kernel<true>, grid, dim3(256), 0, (cudaStream_t)stream, a)
+              : st::launch("st_kv_append launch", kv_append_kernel<false>, grid, dim3(256), 0, (cudaStream_t)stream, a);
 }
 
 extern "C" int st_rope_kv_append(const void* qkv, int64_t row_stride, const void* wq, const void* wk, const float* cos_t,
@@ -869,7 +873,7 @@ extern "C" int st_rope_kv_append(const void* qkv, int64_t row_stride, const void
   AppendArgs a;
   a.K = nullptr; a.V = nullptr; a.ks = 0; a.vs = 0;
   a.slot = (const long long*)slot; a.kv = (uint8_t*)kv; a.pool = pool; a.pool_cnt = pool_cnt;
-  a.nblocks = nblocks; a.N = (int)B; a.H = (int)hkv; a.P = (int)P; a.reuse = 0; a.gsz = 1;
+  a.nblocks = nblocks; a.N = (int)B; a.H = (int)hkv; a.P = (int)P; a.reuse = 0;
   const long long warps = B * (hq + hkv * 4);
   return st::launch("st_rope_kv_append launch", rope_append_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0,
                     (cudaStream_t)stream, r, a);
