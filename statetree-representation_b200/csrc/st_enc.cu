@@ -97,20 +97,19 @@ struct ScanArgs {
   const uint8_t* c8; const int* c32; long long n8, n32; int chunks8;
   int* sums; int* out8; int* out32;
 };
-// this thread's sixteen values of the CTA's chunk (zeros behind the array's end)
+// this thread's sixteen values of the CTA's chunk (zeros behind the array's end; n8 is a multiple of 16, as M is)
 __device__ __forceinline__ void scan_values(const ScanArgs& a, int (&v)[16], long long& at, bool& bytes) {
   bytes = (int)blockIdx.x < a.chunks8;
   at = (long long)(bytes ? blockIdx.x : blockIdx.x - a.chunks8) * SCAN_CHUNK + threadIdx.x * 16;
-  if (bytes && at + 16 <= a.n8) {                // (rowcnt is 16-byte aligned, chunks are multiples of 16)
-    const uint4 w = *reinterpret_cast<const uint4*>(a.c8 + at);
+  if (bytes) {                                   // (rowcnt is 16-byte aligned, chunks are multiples of 16)
+    const uint4 w = at < a.n8 ? *reinterpret_cast<const uint4*>(a.c8 + at) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = (int)(ws[i >> 2] >> (8 * (i & 3)) & 0xFFu);
     return;
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-    v[i] = bytes ? (at + i < a.n8 ? (int)a.c8[at + i] : 0) : (at + i < a.n32 ? a.c32[at + i] : 0);
+  for (int i = 0; i < 16; ++i) v[i] = at + i < a.n32 ? a.c32[at + i] : 0;
 }
 __global__ void __launch_bounds__(256) scan_sums_kernel(const ScanArgs a) {
   __shared__ int s_sum[8];
