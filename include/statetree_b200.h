@@ -47,7 +47,8 @@ int st_rows(const void* tree, const int32_t* eo, const uint32_t* el, int64_t M, 
             int64_t n, void* out, void* stream);
 
 /* BF16 matrix W [M, N] -> state tree (statetree/format.py:43-83 does this with PyTorch operations), in two passes with
- * prefix sums between them (the caller's, or st_encode_offsets with a ws of st_encode_offsets_workspace_bytes() bytes):
+ * prefix sums between them (the caller's, or st_encode_offsets with a ws of st_encode_offsets_workspace_bytes() bytes; rowcnt, roff
+ * and eo 16-byte aligned for it):
  *   st_encode        the records; rowcnt uint8 [M, N/64] = escapes of each row's 64 values; reccnt int32 [M/16 * N/64 + 1] =
  *                    0, then the escapes of each record (its inclusive prefix sum is eo)
  *   st_encode_lists  given eo and roff int32 [M, N/64] (inclusive prefix sum of rowcnt, row-major): el and eb as above and the
