@@ -192,8 +192,8 @@ __device__ __forceinline__ void append_rows(const AppendArgs& a, uint8_t* const 
     for (int i = lane; i < RKV / 16; i += 32) reinterpret_cast<uint4*>(rec)[i] = reinterpret_cast<const uint4*>(grec)[i];
     __syncwarp();
     const uint32_t was = *reinterpret_cast<const uint32_t*>(rec + REC);
-    in_unit = (int)(was & 15u);
-    chain = (was & 16u) ? (int)(was >> 8) : -1;
+    in_unit = min((int)(was & 15u), NSLOT);                       // (a page that was never written may hold anything)
+    chain = (was & 16u) && (int)(was >> 8) < a.P ? (int)(was >> 8) : -1;
   }
   __syncwarp();
   // ---- phase 1: rows
