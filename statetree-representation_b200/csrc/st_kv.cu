@@ -237,8 +237,8 @@ __device__ __forceinline__ void append_rows(const AppendArgs& a, uint8_t* const 
 // The warp edits the 1600-byte unit in shared memory: the segment's rows are fetched up front (independent loads),
 // encoded row by row with shared-memory byte stores, and the unit goes back to the page as 100 16-byte stores.
 // LONG (calls of many tokens): a warp takes sixteen of them, else one.  Two kernels, so that the requests ahead of the long one cost
-// the short one and the rows outside whole pages no registers: one token in each of 8192 pages (8 KV heads) 315 us in one kernel, 306
-// so, 1023 tokens in order (2 KV heads) 9.0 and 8.3.
+// the short one and the rows outside whole pages no registers: one token in each of 8192 pages (8 KV heads) 313 us in one kernel, 303
+// so, 1023 tokens in order (2 KV heads) 9.2 and 8.2.
 template <bool LONG>
 __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   __shared__ __align__(16) uint8_t s_unit[8][RKV];
@@ -256,10 +256,11 @@ __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   // Where the group's tokens come from does not depend on their slots: in a long call, whose groups are whole pages as a rule,
   // the sixteen rows are requested before the slots are looked up, so a page costs two trips to memory one after the other
   // (slots and rows, then the old header) and not four
-  const uint16_t* const rows = (kvi ? a.V : a.K) + h * HD + half * 64;
-  const long long stride = kvi ? a.vs : a.ks;
-  if (LONG && (grp + 1) * PAGE <= a.N && block_aligned(rows, stride)) {
-    const long long n = grp * PAGE;
+  auto first_row = [&] { return (kvi ? a.V : a.K) + h * HD + half * 64; };   // (formed where rows are loaded: no register holds it)
+  auto row_step = [&] { return kvi ? a.vs : a.ks; };
+  if (LONG && (grp + 1) * PAGE <= a.N && block_aligned(first_row(), row_step())) {
+    const uint16_t* const rows = first_row();
+    const long long n = grp * PAGE, stride = row_step();
     uint4 v[4];
     request_block(v, rows + n * stride, stride, lane);
     const long long mine = a.slot[n + (lane & 15)], s0 = __shfl_sync(FULL, mine, 0), blk = s0 / PAGE;
@@ -288,7 +289,9 @@ __global__ void __launch_bounds__(256, 4) kv_append_kernel(const AppendArgs a) {
   n += nrow - 1;                                                  // the segment's other tokens
   if (nrow == PAGE) {
     append_page(a, grec, s_queue[threadIdx.x >> 5],
-                [&](uint32_t (&A)[4][4], uint8_t* stage) { load_block<false>(A, rows + seg * stride, stride, stage, lane); }, lane);
+                [&](uint32_t (&A)[4][4], uint8_t* stage) {
+                  load_block<false>(A, first_row() + seg * row_step(), row_step(), stage, lane);
+                }, lane);
     continue;
   }
   // fetch every row's pair of values now (independent loads), encode afterwards
