@@ -90,7 +90,8 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __
   // unit of this CTA.  Dense: the token tiles of a row block run next to each other (its records then come from HBM once
   // and from L2 for the other tiles); grouped: the row blocks of a pair block do (they share the gathered activations)
   const int ks = blockIdx.x % a.KS, rt = blockIdx.x / a.KS;
-  const int rb = GROUPED ? rt % a.RB : a.rb0 + rt / a.TT, tt = GROUPED ? rt / a.RB : rt % a.TT;
+  const bool tiles = DG == 2 && !GROUPED && a.TT > 1;            // (up to 128 tokens are one tile)
+  const int rb = GROUPED ? rt % a.RB : a.rb0 + (tiles ? rt / a.TT : rt), tt = GROUPED ? rt / a.RB : (tiles ? rt % a.TT : 0);
   // whole pairs of k-tiles; an odd last tile is paired with one beyond the matrix, which both tensor maps fill with zeros
   const int pairs = (a.NG + PAIR - 1) / PAIR;
   const int p0 = (int)((long long)pairs * ks / a.KS), np = (int)((long long)pairs * (ks + 1) / a.KS) - p0;
