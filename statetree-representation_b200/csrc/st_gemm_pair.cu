@@ -13,7 +13,8 @@
 //
 // The clusters are persistent: cluster c takes the (row pair, token tile) units c, c + C, ... and its rings run on across them.
 // The decode warps fill the first weight tiles of the next unit BEFORE they empty the accumulator of the last one, so between two
-// units the tensor cores wait for the accumulator to be read (~1000 cycles), not for a pipeline to start.
+// units the tensor cores wait for the accumulator to be read, not for a pipeline to start: a unit costs 0.9 us beyond its pairs of
+// k-tiles (1.3 and 1.37 us each at 352 and 384 tokens; one to three units of 8 to 32 pairs on every cluster).
 // A k range may be split over 2 to 4 pairs of one cluster (KS): they park their fp32 tiles in shared memory and add them in rank
 // order through distributed shared memory; such a cluster has one unit.
 //

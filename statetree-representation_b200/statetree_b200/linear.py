@@ -30,12 +30,13 @@ PREFILL_MIN = int(os.environ.get("STATETREE_PREFILL_MIN", "512"))
 # ... except that matrices of at least FUSED_WEIGHTS weights stay on the tcgen05 kernel for up to FUSED_ROWS rows, and for up to
 # HOST_ROWS rows below DENSE_WEIGHTS weights, where the scratch path, 75 us of Python, events and launches per call, waits for the
 # host.  These lines are where the two paths met when a tile was one CTA's (all projections of 36 layers of 4096 / 12288, ms with
-# the kernel / the scratch matrix: 960 rows 13.7 / 15.5, 1920 25.6 / 25.9, 2000 28.5 / 25.7).  On CTA pairs the kernel is ahead on
+# the kernel / the scratch matrix: 960 rows 13.7 / 15.5, 1920 25.6 / 25.9, 2000 28.5 / 25.7).  With CTA pairs the kernel is ahead on
 # both sides of them (us per layer, median of 11 passes, the paths in turn):
 #   rows               513         960         1536        2000        4096         8192
-#   4096 / 12288       196 / 380   301 / 426   486 / 577   642 / 696   1233 / 1388  2587 / 2612
-#   2048 / 6144        86 / 312    100 / 316   133 / 315   164 / 318   348 / 365    682 / 663
-# The lines have stayed: which matrices go through the scratch matrix at which rows is a property that callers' tests rely on.
+#   4096 / 12288       201 / 377   313 / 428   488 / 609   657 / 703   1230 / 1395  2517 / 2629
+#   2048 / 6144        82 / 342    98 / 342    130 / 343   161 / 343   333 / 365    668 / 682
+# The lines have not been moved with it: test_path_of_a_prefill_batch (tests/test_gpu_weights.py) states them, and moving them is a
+# change of its own.
 FUSED_ROWS, FUSED_WEIGHTS = 1920, 1 << 22
 HOST_ROWS, DENSE_WEIGHTS = 2048, 1 << 24
 DENSE_MAX = 1 << 28                 # weights: larger matrices (vocabulary-sized tables) never get a dense scratch copy
